@@ -229,7 +229,8 @@ ZG_API zg_error_code zg_unresize_process(const zg_unresize *u, const void *src, 
  * 3: a ring too small for a group). Bits 8-15: the tcgen05 FP32 wide kernel,
  * 16 + cause (17: converter warps, tile or operand buffer; 18: producer,
  * stage never released; 19: MMA lane, operands, accumulator or completion;
- * 20: epilogue, accumulator never complete). -1 when the device words cannot
+ * 20: epilogue, accumulator never complete). Bit 16: the error diffusion's
+ * hand-off between the warps of a plane never came. -1 when the device words cannot
  * be read. Nonzero means a library fault, not a caller error; the outputs of
  * the launches involved are not valid. With reset != 0 the words are
  * cleared. No zimg counterpart (zimg has no asynchronous device work). */

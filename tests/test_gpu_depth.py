@@ -94,6 +94,21 @@ def test_error_diffusion_whole_planes(cuda, oracle, case):
     np.testing.assert_array_equal(got.view(np.uint8), want.view(np.uint8), err_msg=f"{h}x{w}")
 
 
+@pytest.mark.parametrize("h,w", [
+    (1, 300), (31, 1), (32, 2), (33, 15), (33, 16), (64, 17), (65, 92), (96, 93), (97, 94), (128, 109), (129, 110),
+    (256, 111), (1024, 40), (1056, 33), (1057, 33), (2100, 130), (300, 11800), (70, 12100)])
+def test_error_diffusion_hand_off_edges(cuda, oracle, h, w):
+    """Bands of 32 lines around the counts of warps in a block (4) and a
+    cluster (32), lines around the chunk (16 steps) and the run-in of a band
+    (93 steps), and the widest lines of the clustered form and beyond it."""
+    from oracle.oracle import PixelFormat as PF
+    rng = np.random.default_rng(h * 100003 + w)
+    for fin, fout in ((PF("word", 10), PF("byte", 8)), (PF("float"), PF("word", 12))):
+        src = make_src(rng, fin, h, w, special=False)
+        got, _ = convert(src, fin, fout, "error_diffusion", 0)
+        np.testing.assert_array_equal(got, oracle.depth_convert(src, fin, fout, "error_diffusion", 0))
+
+
 def test_error_diffusion_non_finite(cuda, oracle):
     """zimg's C path keeps a NaN through the clamp, stores 0 for it and
     carries its NaN error to the samples after and below it; infinities clamp

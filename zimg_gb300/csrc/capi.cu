@@ -1,5 +1,6 @@
 // C ABI: errors, filter tables, single passes and two-pass conversions.
 #include "capi_common.h"
+#include "depth.h"
 
 #include <algorithm>
 #include <climits>
@@ -250,9 +251,10 @@ int zg_pipeline_status(int reset)
 {
 	const int chain = chain_tma_pipeline_error(reset != 0);
 	const int wide = wide_umma_pipeline_error(reset != 0);
-	if (chain < 0 || wide < 0)
+	const int diffusion = ed_wait_error(reset != 0);
+	if (chain < 0 || wide < 0 || diffusion < 0)
 		return -1;
-	return (chain & 0xFF) | (wide ? (16 + wide) << 8 : 0);
+	return (chain & 0xFF) | (wide ? (16 + wide) << 8 : 0) | (diffusion ? 1 << 16 : 0);
 }
 
 int zg_debug_pipeline_fault(int drop_group, unsigned long long wait_ns)

@@ -66,6 +66,8 @@ int ed_choose_warps(int width, int height);
 // Dynamic shared memory of a launch.
 size_t ed_smem_bytes(int warps, int ring);
 cudaError_t launch_error_diffusion(const EdLaunch &L, cudaStream_t stream);
+// Nonzero when a hand-off wait of the clustered form ran out (optionally reset); -1 when unreadable.
+int ed_wait_error(bool reset);
 
 } // namespace zg
 

@@ -8,15 +8,15 @@
 // 32 lines to a warp ("band"), line r of a band at column c on band step
 // c + 3r. A lane needs the line above's error at column c + 1 two steps after
 // that lane made it, so the value crosses lanes by shuffle off the critical
-// path, which is the left neighbour's error (ten dependent float operations
-// a sample). Band b starts `spacing` steps after band b - 1; the last line of
-// a band hands its errors to the first line of the next through a ring in
-// shared memory, read at least one barrier after it was written.
+// path, which is the left neighbour's error (nine dependent float operations
+// a sample). The last line of a band hands its errors to the first line of
+// the next.
 //
-// Per warp, inputs and outputs go through two 32 x 16 staging tiles in shared
-// memory (pitch 17 words: the lanes of a step hit 32 distinct banks), filled
-// and drained with coalesced loads and stores once per 16 steps; the loads of
-// the next 16 steps are in flight while the current ones run.
+// ed_cluster_kernel runs a plane on a cluster of up to 8 SMs, four warps
+// each, one to a scheduler, so that nothing but the chain sets a step's time;
+// the warps run free of one another and hand errors on through distributed
+// shared memory. ed_kernel (one block a plane, a block barrier every 16 steps)
+// stays for planes whose lines do not fit the cluster's hand-off buffers.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -25,6 +25,7 @@
 
 #include "depth.h"
 #include "depth_device.cuh"
+#include "pipeline.cuh"
 
 namespace zg {
 
@@ -204,9 +205,487 @@ __global__ void __launch_bounds__(kMaxWarps * 32) ed_kernel(const __grid_constan
 	}
 }
 
+// ------------------------------------------------- one plane on a cluster --
+// Bound: the chain of a step (multiply, four adds, the clamp, the rounding add
+// and subtract, the error) times width + 93 steps of a band plus about 120
+// steps per band before it. Warp w of the cluster's computing warps takes
+// bands w, w + warps, ...; warps, not blocks, wait on each other.
+//
+// A computing warp does the steps alone; two more warps move its data
+// meanwhile. The loading one converts the next chunk's inputs into a staging
+// tile and waits for the errors of the band above, the storing one hands the
+// band's last errors on and stores the previous chunk's outputs (one named
+// barrier of the three per chunk of 16 steps, two tiles each way). In one warp
+// the transfers ran after the steps and not beside them, 4,600 cycles a chunk,
+// 860 of them the steps. A block has two computing warps on two of its
+// schedulers and the moving ones on the other two, or, for planes that need
+// more bands in flight, four with the moving ones beside them (cluster_warps).
+//
+// Hand-off: the errors of a band's last line go, by band step, into the
+// receive buffer of the next band's warp with st.async, 16 bytes a lane,
+// which completes on the mbarrier of that chunk beside the buffer (one a
+// chunk, so that the writer may run any number of chunks ahead; a phase a
+// band). Plain stores and a flag with release order instead cost the writer
+// 900 cycles a chunk. A buffer holds a whole line, so the writer never waits:
+// a warp's next band is written only by a band that depends on every sample
+// the warp's current band has read. Waits are bounded (kWaitNs): one that runs
+// out is recorded in g_ed_wait_error and the warp goes on without waiting, so
+// that the launch ends.
+//
+// Measured, a 1920x1080 4:2:0 frame, WORD 10 bits -> BYTE, its planes side by
+// side: 1,185 us in ed_kernel, 224 us here (about 1,250 cycles a chunk; the
+// steps alone, one warp on an idle SM, take 52 cycles, 47 without the
+// shuffle, of which the dependent operations are 40).
+constexpr int kMaxClusterWarps = 4;                   // computing warps per block: 2 or 4
+constexpr int kClusterThreads = 3 * kMaxClusterWarps * 32;
+constexpr int kMaxCluster = 8;                        // blocks per cluster (the portable limit)
+constexpr int kRowPitch = 20;                         // words of a line in a staging tile: conflict-free 16-byte rows
+constexpr int kStage = kBandLines * kRowPitch;        // words of a staging tile
+constexpr int kReadAhead = kTail + kEdLag;            // line 0's step s reads the writer's step s + 96
+constexpr int kWarpFloats = 4 * kStage + 2 * kEdChunk;
+constexpr int kAheadChunks = kReadAhead / kEdChunk + 1;  // so chunk k needs the writer's chunks below k + 7
+static_assert(kReadAhead % kEdChunk == 0, "receive reads start on chunk boundaries");
+
+__device__ int g_ed_wait_error;
+
+// floats of one warp's receive buffer for lines of `width` samples: a slot
+// per band step, and the zeros that the last chunks read past them
+__host__ __device__ constexpr int receive_floats(int chunks)
+{
+	return chunks * kEdChunk + kReadAhead + 2 * kEdChunk;
+}
+
+// its receive buffer and the mbarriers of its chunks, in floats
+__host__ __device__ constexpr int hand_off_floats(int chunks)
+{
+	return receive_floats(chunks) + (2 * chunks + 3) / 4 * 4;
+}
+
+__host__ __device__ constexpr int band_chunks(int width)
+{
+	return (width + kTail + kEdChunk - 1) / kEdChunk;
+}
+
+size_t cluster_smem_bytes(int warps, int hand_off)
+{
+	return static_cast<size_t>(warps) * (kWarpFloats + hand_off) * 4;
+}
+
+__device__ __forceinline__ uint32_t cluster_addr(const void *p, unsigned rank)
+{
+	uint32_t r;
+	asm("mapa.shared::cluster.u32 %0, %1, %2;\n"
+	    : "=r"(r)
+	    : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(p))), "r"(rank));
+	return r;
+}
+
+__device__ __forceinline__ void cluster_barrier()
+{
+	asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+
+// Clamps that keep a NaN (PTX max.NaN / min.NaN), as zimg's std::clamp does.
+__device__ __forceinline__ float clamp_nan(float x, float hi)
+{
+	asm("max.NaN.f32 %0, %0, 0f00000000;\n"
+	    "min.NaN.f32 %0, %0, %1;\n"
+	    : "+f"(x)
+	    : "f"(hi));
+	return x;
+}
+
+// The barrier of computing warp `warp` and the two that move its data.
+__device__ __forceinline__ void chunk_barrier(int warp)
+{
+	asm volatile("bar.sync %0, 96;\n" ::"r"(warp + 1) : "memory");
+}
+
+// An integer sample as float without a conversion instruction (a quarter of
+// the issue rate): its bits below 2^23, minus 2^23.
+template <class T>
+__device__ __forceinline__ float staged_sample(T v)
+{
+	if constexpr (std::is_same_v<T, uint8_t> || std::is_same_v<T, uint16_t>)
+		return __fsub_rn(__uint_as_float(0x4B000000u | v), 8388608.0f);
+	else
+		return sample_to_float(v);
+}
+
+// A store under a predicate, without a branch.
+__device__ __forceinline__ void store_if(bool on, uint8_t *p, uint8_t v)
+{
+	asm volatile("{\n.reg .pred q;\nsetp.ne.s32 q, %0, 0;\n@q st.global.u8 [%1], %2;\n}\n" ::"r"(static_cast<int>(on)),
+	             "l"(p), "r"(static_cast<unsigned>(v))
+	             : "memory");
+}
+
+__device__ __forceinline__ void store_if(bool on, uint16_t *p, uint16_t v)
+{
+	asm volatile("{\n.reg .pred q;\nsetp.ne.s32 q, %0, 0;\n@q st.global.u16 [%1], %2;\n}\n" ::"r"(static_cast<int>(on)),
+	             "l"(p), "h"(v)
+	             : "memory");
+}
+
+// One warp's shared memory: two input tiles, two output tiles, the last
+// line's errors of two chunks, the receive buffer and its mbarriers.
+struct EdShared {
+	float *tile_in;
+	uint32_t *tile_out;
+	float *last;
+	float *recv;
+	uint64_t *bars;
+};
+
+// Transfer j of a moving warp's lane covers line 2j + half of the band at step
+// t16 of the chunk: half a warp along 16 samples of a line.
+struct EdLane {
+	int half, t16, c16;
+	__device__ __forceinline__ EdLane()
+	{
+		const int lane = threadIdx.x & 31;
+		half = lane >> 4;
+		t16 = lane & 15;
+		c16 = t16 - kEdLag * half;
+	}
+};
+
+// Chunks whose 32 x 16 samples all exist need no compares.
+__device__ __forceinline__ bool whole_chunk(const EdPlane &p, int band, int k)
+{
+	return (band + 1) * kBandLines <= p.height && k * kEdChunk >= kTail && (k + 1) * kEdChunk <= p.width;
+}
+
+// The loading warp: inputs into tile_in, and the wait for the errors that the
+// computing warp reads next.
+template <class T>
+__device__ __forceinline__ void ed_load(const EdPlane &p, int first_band, int nw, int warp, const EdShared &m)
+{
+	const EdLane l;
+	const int lane = threadIdx.x & 31;
+	const int W = p.width, H = p.height, chunks = band_chunks(W);
+	const float scale = p.scale, offset = p.offset;
+	const ptrdiff_t step = 2 * p.src_stride - 2 * kEdLag * static_cast<ptrdiff_t>(sizeof(T));
+	unsigned phase = 0;
+	bool gave_up = false;
+	for (int band = first_band; band < p.bands; band += nw) {
+		const char *in0 = static_cast<const char *>(p.src) +
+		                  static_cast<ptrdiff_t>(band * kBandLines + l.half) * p.src_stride +
+		                  static_cast<ptrdiff_t>(l.c16) * static_cast<ptrdiff_t>(sizeof(T));
+		// inputs of two chunks in flight: one chunk's time does not cover the
+		// memory's latency
+		T even[kEdChunk], odd[kEdChunk];
+		auto fetch = [&](T (&pre)[kEdChunk], int k) {
+			if (whole_chunk(p, band, k)) {
+				const char *a = in0 + static_cast<ptrdiff_t>(k) * static_cast<ptrdiff_t>(kEdChunk * sizeof(T));
+#pragma unroll
+				for (int j = 0; j < kEdChunk; ++j)
+					pre[j] = *reinterpret_cast<const T *>(a + j * step);
+				return;
+			}
+			// lines below the plane are read from its last one, columns
+			// outside it from its ends: no branches here either, since a
+			// band's first chunks hold up the bands below
+#pragma unroll
+			for (int j = 0; j < kEdChunk; ++j) {
+				const int line = min(band * kBandLines + 2 * j + l.half, H - 1);
+				const int c = min(max(k * kEdChunk + l.c16 - 2 * kEdLag * j, 0), W - 1);
+				pre[j] = reinterpret_cast<const T *>(static_cast<const char *>(p.src) +
+				                                     static_cast<ptrdiff_t>(line) * p.src_stride)[c];
+			}
+		};
+		// x = sample * scale + offset, two roundings (dither.cpp:76)
+		auto convert = [&](const T (&pre)[kEdChunk], int k) {
+			float *t = m.tile_in + (k & 1) * kStage + l.half * kRowPitch + l.t16;
+#pragma unroll
+			for (int j = 0; j < kEdChunk; ++j)
+				t[2 * j * kRowPitch] = __fadd_rn(__fmul_rn(staged_sample(pre[j]), scale), offset);
+			if (whole_chunk(p, band, k))
+				return;
+			// columns outside the plane: a base so low that the sample clamps
+			// to 0 and its error is 0. (A NaN among the errors above makes it
+			// one, but then the same errors do that to the neighbour inside
+			// the plane that would read it.)
+#pragma unroll
+			for (int j = 0; j < kEdChunk; ++j)
+				if (static_cast<unsigned>(k * kEdChunk + l.c16 - 2 * kEdLag * j) >= static_cast<unsigned>(W))
+					t[2 * j * kRowPitch] = -1.0e9f;
+		};
+		// the errors that chunk k reads have arrived; their mbarriers are
+		// armed again for the warp's next band
+		int arrived = 0;
+		auto receive = [&](int k) {
+			if (band == 0)
+				return;
+			for (const int need = min(k + kAheadChunks, chunks); arrived < need && !gave_up; ++arrived) {
+				if (!__all_sync(0xffffffffu, mbar_wait(m.bars + arrived, phase))) {
+					gave_up = true;
+					atomicExch(&g_ed_wait_error, 1);
+				} else if (lane == 0) {
+					mbar_arrive_expect_tx(m.bars + arrived, kEdChunk * 4);
+				}
+			}
+		};
+		fetch(even, 0);
+		fetch(odd, 1);
+		convert(even, 0);
+		fetch(even, 2);
+		receive(0);
+		chunk_barrier(warp);  // chunk 0's inputs are there
+		auto chunk = [&](T (&pre)[kEdChunk], int k) {
+			convert(pre, k + 1);
+			fetch(pre, k + 3);
+			if (k + 1 < chunks)
+				receive(k + 1);
+			chunk_barrier(warp);  // chunk k is done, chunk k + 1's inputs are there
+		};
+		for (int k = 0; k < chunks; k += 2) {
+			chunk(odd, k);
+			if (k + 1 < chunks)
+				chunk(even, k + 1);
+		}
+		if (band > 0)
+			phase ^= 1;
+	}
+}
+
+// The storing warp: outputs from tile_out, the last line's errors from `last`
+// to the next band's warp (next_recv, next_bars: its buffer and mbarriers).
+template <class U>
+__device__ __forceinline__ void ed_store(const EdPlane &p, int first_band, int nw, int warp, const EdShared &m,
+                                         uint32_t next_recv, uint32_t next_bars)
+{
+	const EdLane l;
+	const int lane = threadIdx.x & 31;
+	const int W = p.width, H = p.height, chunks = band_chunks(W);
+	const ptrdiff_t step = 2 * p.dst_stride - 2 * kEdLag * static_cast<ptrdiff_t>(sizeof(U));
+	for (int band = first_band; band < p.bands; band += nw) {
+		const int rows_left = H - band * kBandLines - l.half;  // line 2j + half exists iff 2j < rows_left
+		char *out0 = static_cast<char *>(p.dst) + static_cast<ptrdiff_t>(band * kBandLines + l.half) * p.dst_stride +
+		             static_cast<ptrdiff_t>(l.c16) * static_cast<ptrdiff_t>(sizeof(U));
+		chunk_barrier(warp);
+		for (int k = 0; k < chunks; ++k) {
+			chunk_barrier(warp);  // chunk k is done
+			if (lane < kEdChunk / 4 && band + 1 < p.bands) {
+				const float4 v = *reinterpret_cast<const float4 *>(m.last + (k & 1) * kEdChunk + 4 * lane);
+				asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];\n" ::"r"(
+					             next_recv + static_cast<uint32_t>(k * kEdChunk + 4 * lane) * 4),
+				             "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"(next_bars + static_cast<uint32_t>(k) * 8)
+				             : "memory");
+			}
+			__syncwarp();
+			char *a = out0 + static_cast<ptrdiff_t>(k) * static_cast<ptrdiff_t>(kEdChunk * sizeof(U));
+			const U *t = reinterpret_cast<const U *>(m.tile_out + (k & 1) * kStage + l.half * kRowPitch) + l.t16;
+			constexpr int kLine2 = 2 * kRowPitch * (4 / static_cast<int>(sizeof(U)));
+			U v[kEdChunk];
+#pragma unroll
+			for (int j = 0; j < kEdChunk; ++j)
+				v[j] = t[j * kLine2];
+			if (whole_chunk(p, band, k)) {
+#pragma unroll
+				for (int j = 0; j < kEdChunk; ++j)
+					*reinterpret_cast<U *>(a + j * step) = v[j];
+			} else {
+				const int cb = k * kEdChunk + l.c16;
+#pragma unroll
+				for (int j = 0; j < kEdChunk; ++j)
+					store_if(2 * j < rows_left && static_cast<unsigned>(cb - 2 * kEdLag * j) < static_cast<unsigned>(W),
+					         reinterpret_cast<U *>(a + j * step), v[j]);
+			}
+		}
+	}
+}
+
+template <class T, class U>
+__global__ void __launch_bounds__(kClusterThreads, 1) ed_cluster_kernel(const __grid_constant__ EdLaunch L)
+{
+	extern __shared__ __align__(16) float ed_smem[];
+	// C computing warps in each of `cluster` blocks. C = 2: warps 0, 1 compute,
+	// 2, 3 load, 6, 7 store (4 and 5 would share the computing warps'
+	// schedulers and do nothing); C = 4: 0-3, 4-7, 8-11
+	const int C = blockDim.x == kClusterThreads ? 4 : 2;
+	const int cluster = L.warps / C;
+	const EdPlane &p = L.planes[blockIdx.x / cluster];
+	const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+	const int role = C == 4 ? wid >> 2 : (wid < 2 ? 0 : (wid < 4 ? 1 : (wid < 6 ? 3 : 2)));
+	const int warp = wid % C;
+	const int nw = L.warps, g = (blockIdx.x % cluster) * C + warp;
+	const int next = (g + 1) % nw;
+	const int W = p.width, chunks = band_chunks(W);
+	const int per_warp = kWarpFloats + L.ring;
+	EdShared m;
+	m.tile_in = ed_smem + warp * per_warp;
+	m.tile_out = reinterpret_cast<uint32_t *>(m.tile_in + 2 * kStage);
+	m.last = m.tile_in + 4 * kStage;
+	m.recv = m.tile_in + kWarpFloats;
+	m.bars = reinterpret_cast<uint64_t *>(m.recv + receive_floats(chunks));
+	if (role == 0) {
+		// the first band's reads find zeros, as the last chunks' past the line do
+		for (int i = (g == 0 ? 0 : chunks * kEdChunk) + lane; i < receive_floats(chunks); i += 32)
+			m.recv[i] = 0.0f;
+		for (int i = lane; i < chunks; i += 32) {
+			mbar_init(m.bars + i, 1);
+			mbar_arrive_expect_tx(m.bars + i, kEdChunk * 4);
+		}
+		asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+	}
+	cluster_barrier();
+
+	if (role == 1) {
+		ed_load<T>(p, g, nw, warp, m);
+		cluster_barrier();
+		return;
+	}
+	if (role >= 2) {
+		const float *next_recv = ed_smem + (next % C) * per_warp + kWarpFloats;
+		if (role == 2)
+			ed_store<U>(p, g, nw, warp, m, cluster_addr(next_recv, next / C),
+			            cluster_addr(next_recv + receive_floats(chunks), next / C));
+		cluster_barrier();
+		return;
+	}
+	const float vmax = p.vmax;
+	constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23: an ulp of 1 for 0 <= x < 2^22, so nearest even
+	for (int band = g; band < p.bands; band += nw) {
+		// errors: left neighbour; h2 / h3 / h4 the line above at columns
+		// c + 1, c, c - 1 for this step; down / above the one for the next
+		// step, chosen only then, so that no step waits for its own shuffle
+		float left = 0.0f, h2 = 0.0f, h3 = 0.0f, h4 = 0.0f, down = 0.0f, above = 0.0f;
+		chunk_barrier(warp);
+		for (int k = 0; k < chunks; ++k) {
+			const float *xin = m.tile_in + (k & 1) * kStage + lane * kRowPitch;
+			const float *uin = m.recv + k * kEdChunk + kReadAhead;
+			uint32_t *row = m.tile_out + (k & 1) * kStage + lane * kRowPitch;
+			float *last = m.last + (k & 1) * kEdChunk;
+			if (k == 0 && band > 0 && lane == 0) {
+				h3 = m.recv[kTail];
+				h2 = m.recv[kTail + 1];
+				above = m.recv[kTail + 2];
+			}
+			float u[kEdChunk], x0[kEdChunk], err[kEdChunk];
+			uint32_t out[kEdChunk];
+#pragma unroll
+			for (int q = 0; q < kEdChunk / 4; ++q) {
+				*reinterpret_cast<float4 *>(x0 + 4 * q) = *reinterpret_cast<const float4 *>(xin + 4 * q);
+				*reinterpret_cast<float4 *>(u + 4 * q) = *reinterpret_cast<const float4 *>(uin + 4 * q);
+			}
+#pragma unroll
+			for (int t = 0; t < kEdChunk; ++t) {
+				// left * 7/16 + top-right * 3/16 + top * 5/16 + top-left *
+				// 1/16, in that order (dither.cpp:78-83). zimg's sum starts
+				// from 0, which only turns a -0 into +0: the sample's base
+				// is never -0 (x * scale + offset with offset never -0), so
+				// a zero's sign cannot reach x and the start is left out.
+				float d = __fmul_rn(left, 0.4375f);
+				d = __fadd_rn(d, __fmul_rn(h2, 0.1875f));
+				d = __fadd_rn(d, __fmul_rn(h3, 0.3125f));
+				d = __fadd_rn(d, __fmul_rn(h4, 0.0625f));
+				// the clamp keeps a NaN as the error; it stores 0, as
+				// zimg's lrint does. Compares and a select instead of the
+				// clamp measured 63 cycles a step against 52: a predicate
+				// comes later than a clamped value.
+				const float x = clamp_nan(__fadd_rn(x0[t], d), vmax);
+				const float r = __fadd_rn(x, kMagic);
+				const float e = __fsub_rn(x, __fsub_rn(r, kMagic));
+				out[t] = __float_as_uint(fmaxf(r, kMagic));
+				err[t] = e;
+				left = e;
+				h4 = h3;
+				h3 = h2;
+				h2 = lane != 0 ? down : above;
+				down = __shfl_up_sync(0xffffffffu, e, 1);
+				above = u[t];
+			}
+#pragma unroll
+			for (int q = 0; q < kEdChunk / 4; ++q) {
+				if (lane == kBandLines - 1)
+					*reinterpret_cast<float4 *>(last + 4 * q) =
+						make_float4(err[4 * q], err[4 * q + 1], err[4 * q + 2], err[4 * q + 3]);
+				if constexpr (sizeof(U) == 2)
+					*reinterpret_cast<uint2 *>(row + 2 * q) = make_uint2(__byte_perm(out[4 * q], out[4 * q + 1], 0x5410),
+					                                                     __byte_perm(out[4 * q + 2], out[4 * q + 3], 0x5410));
+			}
+			if constexpr (sizeof(U) == 1) {
+				uint32_t w[4];
+#pragma unroll
+				for (int q = 0; q < 4; ++q)
+					w[q] = __byte_perm(__byte_perm(out[4 * q], out[4 * q + 1], 0x0040),
+					                   __byte_perm(out[4 * q + 2], out[4 * q + 3], 0x0040), 0x5410);
+				*reinterpret_cast<uint4 *>(row) = make_uint4(w[0], w[1], w[2], w[3]);
+			}
+			chunk_barrier(warp);
+		}
+	}
+	cluster_barrier();  // no block leaves while another may write to its shared memory
+}
+
+// Chunk times until a plane's last band ends, with nw warps: a band starts
+// about 8 chunks after the one above (7 by the skew, the rest the hand-off),
+// or when its warp is free.
+long long wavefront_chunks(const EdPlane &p, int nw)
+{
+	const long long chunks = band_chunks(p.width), b = (p.height + kBandLines - 1) / kBandLines - 1;
+	const long long lag = kAheadChunks + 1;
+	return lag * nw >= chunks ? b * lag + chunks : b / nw * chunks + b % nw * lag + chunks;
+}
+
+// Computing warps per block for these planes: 2 where 16 warps in a cluster
+// (2 x 8 blocks) are as fast, 4 otherwise; 0 when the hand-off buffers do not
+// fit. A chunk takes about 1,000 cycles with the moving warps on other
+// schedulers and 1,300 beside them. 2 admits lines of about 21,000 samples, 4
+// of 10,000.
+int cluster_warps(const EdLaunch &L)
+{
+	long long t2 = 0, t4 = 0;
+	int hand_off = 0;
+	for (int k = 0; k < L.num_planes; ++k) {
+		if (L.planes[k].width > (1 << 16))
+			return 0;
+		t2 = std::max(t2, wavefront_chunks(L.planes[k], 2 * kMaxCluster) * 10);
+		t4 = std::max(t4, wavefront_chunks(L.planes[k], 4 * kMaxCluster) * 13);
+		hand_off = std::max(hand_off, hand_off_floats(band_chunks(L.planes[k].width)));
+	}
+	if (t4 < t2 && cluster_smem_bytes(4, hand_off) <= kMaxSmem)
+		return 4;
+	return cluster_smem_bytes(2, hand_off) <= kMaxSmem ? 2 : 0;
+}
+
+template <class T, class U>
+cudaError_t launch_cluster(const EdLaunch &L, int warps, cudaStream_t st)
+{
+	// blocks per cluster: enough warps for the bands
+	EdLaunch C = L;
+	int cluster = 1;
+	C.ring = 0;
+	for (int k = 0; k < L.num_planes; ++k) {
+		while (cluster < kMaxCluster && cluster * warps < L.planes[k].bands)
+			cluster *= 2;
+		C.ring = std::max(C.ring, hand_off_floats(band_chunks(L.planes[k].width)));
+	}
+	C.warps = cluster * warps;
+	cudaError_t e = cudaFuncSetAttribute(ed_cluster_kernel<T, U>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+	                                     static_cast<int>(kMaxSmem));
+	if (e != cudaSuccess)
+		return e;
+	cudaLaunchConfig_t cfg{};
+	cfg.gridDim = dim3(static_cast<unsigned>(L.num_planes * cluster));
+	cfg.blockDim = dim3(warps == 4 ? kClusterThreads : 256);
+	cfg.dynamicSmemBytes = cluster_smem_bytes(warps, C.ring);
+	cfg.stream = st;
+	cudaLaunchAttribute attr{};
+	attr.id = cudaLaunchAttributeClusterDimension;
+	attr.val.clusterDim.x = static_cast<unsigned>(cluster);
+	attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+	cfg.attrs = &attr;
+	cfg.numAttrs = 1;
+	return cudaLaunchKernelEx(&cfg, ed_cluster_kernel<T, U>, C);
+}
+
 template <class T, class U>
 cudaError_t launch_tu(const EdLaunch &L, size_t smem, cudaStream_t st)
 {
+	if (const int warps = cluster_warps(L))
+		return launch_cluster<T, U>(L, warps, st);
 	static bool raised = false;
 	if (!raised) {
 		cudaError_t e = cudaFuncSetAttribute(ed_kernel<T, U>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -235,6 +714,18 @@ int round_up(int v, int m)
 }
 
 } // namespace
+
+int ed_wait_error(bool reset)
+{
+	int v = 0;
+	if (cudaMemcpyFromSymbol(&v, g_ed_wait_error, sizeof(v)) != cudaSuccess)
+		return -1;
+	if (reset && v) {
+		const int zero = 0;
+		cudaMemcpyToSymbol(g_ed_wait_error, &zero, sizeof(zero));
+	}
+	return v;
+}
 
 size_t ed_smem_bytes(int warps, int ring)
 {
