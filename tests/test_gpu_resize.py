@@ -104,6 +104,36 @@ def test_golden_planes_on_gpu(cuda, golden, oracle):
             _f32_check(oracle, src, got, p["dst_w"], p["dst_h"], p["kind"], p["a"], p["b"], exact=False, **kw)
 
 
+@pytest.mark.parametrize("sw,sh,dw,dh,kind,a", [
+    (256, 64, 128, 32, "spline36", math.nan),     # 2x down, one strip and its window's edge
+    (515, 131, 257, 65, "spline36", math.nan),    # odd lines: 2-byte u16 and 4-byte f32 alignment
+    (400, 90, 266, 60, "bicubic", math.nan),      # 1.5x down
+    (1030, 260, 129, 33, "bilinear", math.nan),   # 8x down: 16 taps, narrow strips, lines loaded late
+    (999, 100, 333, 33, "bicubic", math.nan),     # 3x down
+    (130, 7, 65, 3, "lanczos", 2.0),              # fewer rows than a step
+    (33, 17, 129, 67, "lanczos", 3.0),            # up, one column past a strip
+    (64, 64, 1000, 1001, "spline64", math.nan),   # strong upscale: windows shared by many steps
+    (250, 120, 252, 119, "spline16", math.nan)])  # about 1x
+@pytest.mark.parametrize("pad,offset", [(0, 0), (1, 1), (2, 2), (4, 4), (5, 0)])
+def test_streaming_kernel_edges(cuda, oracle, sw, sh, dw, dh, kind, a, pad, offset):
+    """The CUDA-core streaming kernel at the ends of its strips, steps and
+    windows, planes at every alignment its line copies tell apart: u16 at
+    depths 10 (engine "cuda") and 16 against the C path, samples over the
+    depth's range included, f32 against the FMA order; bit for bit."""
+    rng = np.random.default_rng(sw * 7919 + dw * 31 + pad)
+    for depth in (10, 16):
+        src = rng.integers(0, 1 << 16, size=(sh, sw), dtype=np.uint16)
+        got, r = run_conversion(src, dw, dh, kind, a, depth=depth, engine="cuda", pad=pad, offset=offset)
+        assert r.info["engine"] == "cuda"
+        want = oracle.resize_plane(src, dw, dh, kind, a, depth=depth, mode="c", nthreads=16)
+        np.testing.assert_array_equal(got, want, err_msg=f"depth {depth}")
+    src = rng.random((sh, sw), dtype=np.float32)
+    got, r = run_conversion(src, dw, dh, kind, a, engine="cuda", pad=pad, offset=offset)
+    assert r.info["engine"] == "cuda"
+    want = oracle.resize_plane(src, dw, dh, kind, a, mode="fma", nthreads=16)
+    np.testing.assert_array_equal(got.view(np.uint32), want.view(np.uint32))
+
+
 # ------------------------------------------------- headline configurations --
 
 def test_fhd_to_uhd_u16_lanczos3_bitexact(cuda, oracle):

@@ -9,32 +9,18 @@
 namespace zg {
 
 // per-(H_FIRST, kind) instantiation units (fused_inst_*.cu)
-cudaError_t launch_fused_v_f32(int, int, const FusedJob *, int, int, const SmemLayout &, int, const FusedJob &,
-                               const WorkChunks &, cudaStream_t);
-cudaError_t launch_fused_v_u16(int, int, const FusedJob *, int, int, const SmemLayout &, int, const FusedJob &,
-                               const WorkChunks &, cudaStream_t);
-cudaError_t launch_fused_h_f32(int, int, const FusedJob *, int, int, const SmemLayout &, int, const FusedJob &,
-                               const WorkChunks &, cudaStream_t);
-cudaError_t launch_fused_h_u16(int, int, const FusedJob *, int, int, const SmemLayout &, int, const FusedJob &,
-                               const WorkChunks &, cudaStream_t);
 const void *fused_kernel_ptr_v_f32(int hw, int vs);
-const void *fused_kernel_ptr_v_u16(int hw, int vs);
 const void *fused_kernel_ptr_h_f32(int hw, int vs);
-const void *fused_kernel_ptr_h_u16(int hw, int vs);
-cudaError_t launch_fused_v_i16(int, int, const FusedJob *, int, int, const SmemLayout &, int, const FusedJob &,
-                               const WorkChunks &, cudaStream_t);
-cudaError_t launch_fused_h_i16(int, int, const FusedJob *, int, int, const SmemLayout &, int, const FusedJob &,
-                               const WorkChunks &, cudaStream_t);
 const void *fused_kernel_ptr_v_i16(int hw, int vs);
 const void *fused_kernel_ptr_h_i16(int hw, int vs);
 
 namespace {
 
-constexpr int kHwBuckets[] = { 6, 8, 16 };
+constexpr int kHwBuckets[] = { 6, 8, 12, 16 };
 constexpr int kVsBuckets[] = { 8, 12, 16, 24 };
 constexpr size_t kSmemBudget = 56 * 1024;   // preferred: four CTAs of 128 threads per SM
 constexpr size_t kSmemMax = 110 * 1024;     // hard limit: two CTAs per SM
-constexpr int kItemGroupsMax = 256;          // groups of one work item (a multiple of every step)
+constexpr int kBlockColumns = 4 * 66;       // columns of the intermediate block (fused_kernel.cuh)
 
 int bucket_index(const int *b, int n, int v)
 {
@@ -49,51 +35,32 @@ size_t align_up(size_t x, size_t a)
 	return (x + a - 1) / a * a;
 }
 
-// u16 sums in float are exact when every partial sum is an integer below 2^24
-// and each row's taps sum to exactly 1 << 14 (so re-centring the samples by
-// 2^(depth-1) shifts the sum by a multiple of 2^14).
-bool u16_exact_in_float(const FilterTable &t, unsigned depth)
-{
-	const double half = std::ldexp(1.0, static_cast<int>(depth) - 1);
-	for (unsigned i = 0; i < t.rows; ++i) {
-		double mag = 8192.0;
-		long sum = 0;
-		for (unsigned k = 0; k < t.width; ++k) {
-			const int16_t c = t.i16[static_cast<size_t>(i) * t.width + k];
-			mag += std::abs(static_cast<double>(c)) * half;
-			sum += c;
-		}
-		if (sum != 16384 || mag >= 16777216.0)
-			return false;
-	}
-	return true;
-}
-
-// zimg's int32 sums cannot overflow: sum |tap| * 2^15 + 8192 < 2^31 per row.
+// zimg's int32 sums cannot overflow (sum |tap| * 2^15 + 8192 < 2^31 per row),
+// and a row's taps sum to 1 << 14, so that centring the samples is a constant.
 bool u16_fits_int32(const FilterTable &t)
 {
 	for (unsigned i = 0; i < t.rows; ++i) {
-		long long mag = 8192;
-		for (unsigned k = 0; k < t.width; ++k)
-			mag += static_cast<long long>(std::abs(static_cast<int>(t.i16[static_cast<size_t>(i) * t.width + k]))) << 15;
-		if (mag >= (1LL << 31))
+		long long mag = 8192, sum = 0;
+		for (unsigned k = 0; k < t.width; ++k) {
+			const int c = t.i16[static_cast<size_t>(i) * t.width + k];
+			mag += static_cast<long long>(std::abs(c)) << 15;
+			sum += c;
+		}
+		if (mag >= (1LL << 31) || sum != (1 << 14))
 			return false;
 	}
 	return true;
 }
 
-// A tap as the kernel reads it: the f32 tap, the int16 tap as a float, or
-// (integer arithmetic) the int16 tap as int32 bits.
-float tap_value(const FilterTable &t, bool u16, bool integer, unsigned i, unsigned k)
+// A tap's 32 bits as the kernel reads them: the f32 tap or the int16 tap as int32.
+uint32_t tap_bits(const FilterTable &t, bool u16, unsigned i, unsigned k)
 {
 	const size_t at = static_cast<size_t>(i) * t.width + k;
-	if (integer) {
-		const int32_t v = t.i16[at];
-		float f;
-		std::memcpy(&f, &v, sizeof(f));
-		return f;
-	}
-	return u16 ? static_cast<float>(t.i16[at]) : t.f32[at];
+	if (u16)
+		return static_cast<uint32_t>(static_cast<int32_t>(t.i16[at]));
+	uint32_t v;
+	std::memcpy(&v, &t.f32[at], sizeof(v));
+	return v;
 }
 
 } // namespace
@@ -106,14 +73,14 @@ bool plan_fused(const FilterTable &first, const FilterTable &second, bool h_firs
 	const FilterTable &V = h_first ? second : first;
 	if (H.rows != dst_w || V.rows != dst_h || H.input_width != src_w || V.input_width != src_h)
 		return false;
-	// u16: exact float arithmetic where the planner can prove it, else zimg's int32
-	const bool integer = u16 && (!u16_exact_in_float(H, depth) || !u16_exact_in_float(V, depth));
-	if (integer && (!u16_fits_int32(H) || !u16_fits_int32(V)))
+	if (u16 && (!u16_fits_int32(H) || !u16_fits_int32(V)))
 		return false;
 
-	const int hw_i = bucket_index(kHwBuckets, 3, static_cast<int>(H.width));
+	int hw_i = bucket_index(kHwBuckets, 4, static_cast<int>(H.width));
 	if (hw_i < 0)
 		return false;
+	if (!u16 && kHwBuckets[hw_i] == 12)
+		hw_i = 3;  // F32: how far a NaN under a zero tap spreads is part of the result
 	const int HW = kHwBuckets[hw_i];
 
 	// dense vertical groups; streaming needs non-decreasing group bases
@@ -140,118 +107,133 @@ bool plan_fused(const FilterTable &first, const FilterTable &second, bool h_firs
 		return false;
 	const int VS = kVsBuckets[vs_i];
 
-	// source-column window of each strip
+	// strips: output columns (a multiple of 8, at most kStripW) whose inputs
+	// stay within the kernel's window; of those the width that needs the
+	// fewest warp passes per output: V first, the vertical pass's (quad of
+	// columns, half of a step's rows) items fill whole warps or not
 	const int col_align = u16 ? 8 : 4;
-	const int strips = static_cast<int>((dst_w + kStripW - 1) / kStripW);
-	std::vector<int> win_col(2 * strips);
-	int max_pxa = 0;
-	for (int s = 0; s < strips; ++s) {
-		int lo = INT_MAX, hi = INT_MIN;
-		for (unsigned c = s * kStripW; c < std::min<unsigned>(dst_w, (s + 1) * kStripW); ++c) {
-			lo = std::min(lo, static_cast<int>(H.left[c]));
-			hi = std::max(hi, static_cast<int>(H.left[c]) + HW);
+	auto windows = [&](int w, std::vector<int> &win) {
+		const int n = static_cast<int>((dst_w + w - 1) / w);
+		win.assign(2 * n, 0);
+		int widest = 0;
+		for (int s = 0; s < n; ++s) {
+			int lo = INT_MAX, hi = INT_MIN;
+			for (unsigned c = s * w; c < std::min<unsigned>(dst_w, (s + 1) * w); ++c) {
+				lo = std::min(lo, static_cast<int>(H.left[c]));
+				hi = std::max(hi, static_cast<int>(H.left[c]) + HW);
+			}
+			win[2 * s] = lo / col_align * col_align;
+			win[2 * s + 1] = hi;
+			widest = std::max(widest, (hi - win[2 * s] + 7) & ~7);
 		}
-		lo = lo / col_align * col_align;
-		win_col[2 * s] = lo;
-		win_col[2 * s + 1] = hi;
-		max_pxa = std::max(max_pxa, (hi - lo + 7) & ~7);
+		return widest;
+	};
+	int strip_w = 0;
+	double best = 0;
+	std::vector<int> win_col, win;
+	for (int w = kStripW; w >= 8; w -= 8) {
+		const int widest = windows(w, win);
+		if (widest > kStreamWindow)
+			continue;
+		const int v_warps = h_first ? 4 : (widest / 2 + 31) / 32, h_warps = (w + 31) / 32;
+		const double cost = (2.0 * v_warps * VS + h_warps * 2.0 * HW + 40) / w;
+		if (!strip_w || cost < 0.97 * best) {
+			strip_w = w;
+			best = cost;
+			win_col = win;
+		}
+	}
+	if (!strip_w)
+		return false;
+	const int strips = static_cast<int>(win_col.size() / 2);
+
+	// steps of four groups; the lines a step's windows span. H first: in
+	// multiples of four, the lines of a horizontal iteration
+	const int steps = (groups + 3) / 4;
+	std::vector<int> ranges(2 * steps);
+	for (int k = 0; k < steps; ++k) {
+		const int lo = gbase[4 * k], hi = gbase[std::min(groups, 4 * k + 4) - 1] + VS;
+		ranges[2 * k] = h_first ? lo / 4 * 4 : lo;
+		ranges[2 * k + 1] = h_first ? (hi + 3) / 4 * 4 : hi;
+	}
+	// any step may start an item, when its new lines are its whole range;
+	// early: the next step's lines arrive beside this one's
+	int rows_late = 4, rows_early = 4;
+	for (int k = 0; k < steps; ++k) {
+		rows_late = std::max(rows_late, ranges[2 * k + 1] - ranges[2 * k]);
+		rows_early = std::max(rows_early, ranges[2 * std::min(k + 1, steps - 1) + 1] - ranges[2 * k]);
 	}
 
-	// steps and rings: try the preferred step, then smaller ones
 	FusedPlan &p = *out;
 	p = FusedPlan{};
+	FusedJob &J = p.job;
+	J.h_first = h_first ? 1 : 0;
+	J.kind = static_cast<int>(u16 ? FusedKind::U16_INT : FusedKind::F32);
+	J.hw = HW;
+	J.vs = VS;
+	J.step_groups = 4;
+	J.groups = groups;
+	J.seg_groups = 4;  // work units: (strip, step) pairs
+	J.segments = steps;
+	J.ring_rows = h_first ? rows_late : 0;
+	// lines a step ahead where four CTAs still fit an SM, else only after the
+	// pass that reads the ring if that lets them fit
 	bool fits = false;
-	for (int attempt = 0; attempt < 2 && !fits; ++attempt)
-	for (int step_groups = 4; step_groups >= 1 && !fits; step_groups /= 2) {
-		const size_t budget = attempt == 0 ? kSmemBudget : kSmemMax;
-		const int nsteps = (groups + step_groups - 1) / step_groups;
-		auto hi_of = [&](int k) { return gbase[std::min(groups, (k + 1) * step_groups) - 1] + VS; };
-		int ring_need = 1, stage_need = 1, in_need = 1;
-		for (int k = 0; k < nsteps; ++k) {
-			const int win_lo = gbase[k * step_groups];
-			const int hi = hi_of(k);
-			const int hi_next = k + 1 < nsteps ? hi_of(k + 1) : hi;
-			// any step may start a segment, when its new lines are its whole window
-			if (h_first) {
-				ring_need = std::max(ring_need, hi - win_lo);
-				if (u16) {
-					in_need = std::max(in_need, hi - win_lo);
-					stage_need = std::max(stage_need, hi_next - win_lo);
-				} else {
-					in_need = std::max(in_need, hi_next - win_lo);
-				}
-			} else {
-				ring_need = std::max(ring_need, u16 ? hi - win_lo : hi_next - win_lo);
-				if (u16)
-					stage_need = std::max(stage_need, hi_next - win_lo);
-			}
+	for (size_t budget : { kSmemBudget, kSmemMax })
+		for (int ahead = 1; ahead >= 0 && !fits; --ahead) {
+			J.depth = ahead;
+			J.in_rows = ahead ? rows_early : rows_late;
+			const FusedPlan *pp = &p;
+			fits = static_cast<size_t>(fused_layout(&pp, 1).total_bytes) <= budget;
 		}
-		auto pow2 = [](int x) { int r = 1; while (r < x) r <<= 1; return r; };
-		FusedJob &J = p.job;
-		J.h_first = h_first ? 1 : 0;
-		J.kind = static_cast<int>(integer ? FusedKind::U16_INT : (u16 ? FusedKind::U16_EXACT : FusedKind::F32));
-		J.hw = HW;
-		J.vs = VS;
-		J.step_groups = step_groups;
-		J.groups = groups;
-		J.seg_groups = step_groups;  // work units: (strip, step) pairs, split evenly over the CTAs
-		J.segments = nsteps;
-		J.ring_rows = pow2(ring_need);
-		J.in_rows = h_first ? pow2(in_need) : 1;
-		p.max_pxa = max_pxa;
-		// staging ring for u16 lives in the layout's stage_rows (recorded below)
-		p.stage_rows = u16 ? pow2(stage_need) : 1;
-		const FusedPlan *pp = &p;
-		if (static_cast<size_t>(fused_layout(&pp, 1).total_bytes) <= budget)
-			fits = true;
-	}
 	if (!fits)
 		return false;
 
-	// host blob: h_taps | h_left | v_dense | v_base | win_col
+	// host blob: h_taps | h_left | records | ranges | win_col
+	const int padded = 4 * steps, rec_bytes = stream_record_bytes(h_first, VS);
 	size_t off = 0;
-	p.off_h_taps = off;  off = align_up(off + static_cast<size_t>(dst_w) * HW * sizeof(float), 256);
+	p.off_h_taps = off;  off = align_up(off + static_cast<size_t>(dst_w) * HW * 4, 256);
 	p.off_h_left = off;  off = align_up(off + static_cast<size_t>(dst_w) * sizeof(int), 256);
-	p.off_v_dense = off; off = align_up(off + static_cast<size_t>(groups) * VS * kGroup * sizeof(float), 256);
-	p.off_v_base = off;  off = align_up(off + static_cast<size_t>(groups) * sizeof(int), 256);
+	p.off_v_dense = off; off = align_up(off + static_cast<size_t>(padded) * rec_bytes, 256);
+	p.off_v_base = off;  off = align_up(off + ranges.size() * sizeof(int), 256);
 	p.off_win_col = off; off = align_up(off + win_col.size() * sizeof(int), 256);
 	p.blob.assign(off, 0);
 
-	float *h_taps = reinterpret_cast<float *>(p.blob.data() + p.off_h_taps);
+	uint32_t *h_taps = reinterpret_cast<uint32_t *>(p.blob.data() + p.off_h_taps);
 	int *h_left = reinterpret_cast<int *>(p.blob.data() + p.off_h_left);
 	for (unsigned c = 0; c < dst_w; ++c) {
 		for (unsigned k = 0; k < H.width; ++k)
-			h_taps[static_cast<size_t>(c) * HW + k] = tap_value(H, u16, integer, c, k);
+			h_taps[static_cast<size_t>(c) * HW + k] = tap_bits(H, u16, c, k);
 		h_left[c] = static_cast<int>(H.left[c]);
 	}
-	float *v_dense = reinterpret_cast<float *>(p.blob.data() + p.off_v_dense);
-	int *v_base = reinterpret_cast<int *>(p.blob.data() + p.off_v_base);
-	for (int g = 0; g < groups; ++g) {
-		v_base[g] = gbase[g];
-		for (int j = 0; j < kGroup; ++j) {
+	uint32_t *rec = reinterpret_cast<uint32_t *>(p.blob.data() + p.off_v_dense);
+	const int rows = h_first ? J.ring_rows : J.in_rows;
+	const int line_bytes = h_first ? kStripW * 4 : kStreamWindow * (u16 ? 2 : 4);
+	for (int g = 0; g < padded; ++g) {
+		const int base = gbase[std::min(g, groups - 1)];
+		uint32_t *r = rec + static_cast<size_t>(g) * (rec_bytes / 4);
+		for (int s = 0; s < VS; ++s)
+			r[VS * kGroup + s] = static_cast<uint32_t>((base + s) % rows * line_bytes);
+		for (int j = 0; j < kGroup && g < groups; ++j) {
 			const unsigned i = static_cast<unsigned>(g * kGroup + j);
 			if (i >= dst_h)
 				break;
-			const int d = static_cast<int>(V.left[i]) - gbase[g];
+			const int d = static_cast<int>(V.left[i]) - base;
 			for (unsigned k = 0; k < V.width; ++k)
-				v_dense[(static_cast<size_t>(g) * VS + d + k) * kGroup + j] = tap_value(V, u16, integer, i, k);
+				r[(d + k) * kGroup + j] = tap_bits(V, u16, i, k);
 		}
 	}
+	std::memcpy(p.blob.data() + p.off_v_base, ranges.data(), ranges.size() * sizeof(int));
 	std::memcpy(p.blob.data() + p.off_win_col, win_col.data(), win_col.size() * sizeof(int));
 
-	FusedJob &J = p.job;
 	J.src_w = static_cast<int>(src_w);
 	J.src_h = static_cast<int>(src_h);
 	J.dst_w = static_cast<int>(dst_w);
 	J.dst_h = static_cast<int>(dst_h);
 	J.strips = strips;
-	J.strip_w = kStripW;
-	// centring offset: 2^(depth-1) for exact float sums, zimg's 32768 for int32 ones
-	const float offset = integer ? 32768.0f : (u16 ? static_cast<float>(std::ldexp(1.0, static_cast<int>(depth) - 1)) : 0.0f);
-	J.offset = offset;
-	J.magic = 12582912.0f + offset;
+	J.strip_w = strip_w;
 	J.pixel_max = u16 ? static_cast<float>((1UL << depth) - 1) : 0.0f;
-	p.variant = ((J.h_first * 3 + (integer ? 2 : (u16 ? 1 : 0))) * 3 + hw_i) * 4 + vs_i;
+	p.variant = ((J.h_first * 2 + (u16 ? 1 : 0)) * 4 + hw_i) * 4 + vs_i;
 	return true;
 }
 
@@ -303,28 +285,19 @@ void fused_bind(FusedPlan &p, const void *device_blob)
 
 namespace {
 
-// kind: 0 f32, 1 u16 in exact float sums, 2 u16 in int32 sums
-void split_variant(int variant, int *hf, int *kind, int *hw_i, int *vs_i)
-{
-	*vs_i = variant % 4;
-	*hw_i = (variant / 4) % 3;
-	*kind = (variant / 12) % 3;
-	*hf = (variant / 36) % 2;
-}
-
 const void *kernel_ptr(int variant)
 {
 	if (variant >= 200)
 		return chain_kernel_ptr(variant);
 	if (variant >= 100)
 		return mma_kernel_ptr(variant);
-	int hf, kind, hw, vs;
-	split_variant(variant, &hf, &kind, &hw, &vs);
-	if (hf)
-		return kind == 2 ? fused_kernel_ptr_h_i16(hw, vs)
-		                 : (kind == 1 ? fused_kernel_ptr_h_u16(hw, vs) : fused_kernel_ptr_h_f32(hw, vs));
-	return kind == 2 ? fused_kernel_ptr_v_i16(hw, vs)
-	                 : (kind == 1 ? fused_kernel_ptr_v_u16(hw, vs) : fused_kernel_ptr_v_f32(hw, vs));
+	const int vs = variant % 4, hw = variant / 4 % 4;
+	switch (variant / 16) {
+	case 0: return fused_kernel_ptr_v_f32(hw, vs);
+	case 1: return fused_kernel_ptr_v_i16(hw, vs);
+	case 2: return fused_kernel_ptr_h_f32(hw, vs);
+	default: return fused_kernel_ptr_h_i16(hw, vs);
+	}
 }
 
 } // namespace
@@ -335,46 +308,22 @@ SmemLayout fused_layout(const FusedPlan *const *plans, int n)
 		return chain_layout(plans, n);
 	if (n > 0 && plans[0]->mma)
 		return mma_layout(plans, n);
-	int max_pxa = 0, hw = 0, vs = 0, ring = 1, in = 1, stage = 1, seg_groups = 1, step_groups = 1;
-	bool u16 = false, h_first = false;
+	int in = 0, ring = 0;
 	for (int i = 0; i < n; ++i) {
-		const FusedPlan &p = *plans[i];
-		max_pxa = std::max(max_pxa, p.max_pxa);
-		hw = std::max(hw, p.job.hw);
-		vs = std::max(vs, p.job.vs);
-		ring = std::max(ring, p.job.ring_rows);
-		in = std::max(in, p.job.in_rows);
-		stage = std::max(stage, p.stage_rows);
-		seg_groups = std::max(seg_groups, std::min(p.job.groups, kItemGroupsMax));
-		step_groups = std::max(step_groups, p.job.step_groups);
-		u16 = p.job.kind != static_cast<int>(FusedKind::F32);
-		h_first = p.job.h_first != 0;
+		in = std::max(in, plans[i]->job.in_rows);
+		ring = std::max(ring, plans[i]->job.ring_rows);
 	}
-	auto a16 = [](size_t x) { return static_cast<int>((x + 15) / 16 * 16); };
+	const FusedJob &J = plans[0]->job;  // one variant: what follows is the same for every plan
+	const bool h_first = J.h_first != 0;
+	const int sample = J.kind == static_cast<int>(FusedKind::F32) ? 4 : 2;
 	SmemLayout L{};
-	L.pitch = max_pxa + 8;
-	L.ring_rows = ring;
-	L.in_rows = h_first ? in : 1;
-	L.stage_rows = u16 ? stage : 1;
-	L.seg_groups = seg_groups;
-	L.step_groups = step_groups;
 	int off = 0;
-	L.ring_off = off;
-	off += a16(static_cast<size_t>(ring) * (h_first ? kStripW : L.pitch) * 4);
-	L.stage_off = off;
-	off += u16 ? a16(static_cast<size_t>(L.stage_rows) * L.pitch * 2) : 0;
 	L.in_off = off;
-	off += h_first ? a16(static_cast<size_t>(L.in_rows) * L.pitch * 4) : 0;
-	L.i_off = off;
-	off += h_first ? 0 : a16(static_cast<size_t>(step_groups) * group_rows(false) * L.pitch * 4);
-	L.htaps_off = off;
-	off += a16(static_cast<size_t>(kStripW) * hw * 4);
-	L.hleft_off = off;
-	off += a16(kStripW * 4);
+	off += in * kStreamWindow * sample;
+	L.ring_off = off;
+	off += h_first ? ring * kStripW * 4 : 2 * kBlockColumns * 16;
 	L.vcoef_off = off;
-	off += 2 * a16(static_cast<size_t>(step_groups) * vs * group_rows(h_first) * 4);
-	L.vbase_off = off;
-	off += a16(static_cast<size_t>(seg_groups) * 4);
+	off += 2 * 4 * stream_record_bytes(h_first, J.vs);
 	L.total_bytes = off;
 	return L;
 }
@@ -409,19 +358,18 @@ cudaError_t launch_fused(int variant, const FusedJob *jobs, int num_jobs, int to
 		return launch_chain(variant, jobs, num_jobs, total_tiles, smem_bytes, grid, single, stream);
 	if (variant >= 100)
 		return launch_mma(variant, jobs, num_jobs, total_tiles, smem_bytes, grid, single, stream);
-	int hf, kind, hw, vs;
-	split_variant(variant, &hf, &kind, &hw, &vs);
-	grid = std::max(1, std::min(grid, total_tiles));
+	grid = std::max(1, std::min(grid, chunks.sched ? chunks.num : total_tiles));
 	if (smem_bytes.total_bytes > static_cast<int>(kSmemMax))
 		return cudaErrorInvalidValue;
-	const WorkChunks &c = chunks;
-	if (hf)
-		return kind == 2 ? launch_fused_h_i16(hw, vs, jobs, num_jobs, total_tiles, smem_bytes, grid, single, c, stream)
-		     : kind == 1 ? launch_fused_h_u16(hw, vs, jobs, num_jobs, total_tiles, smem_bytes, grid, single, c, stream)
-		                 : launch_fused_h_f32(hw, vs, jobs, num_jobs, total_tiles, smem_bytes, grid, single, c, stream);
-	return kind == 2 ? launch_fused_v_i16(hw, vs, jobs, num_jobs, total_tiles, smem_bytes, grid, single, c, stream)
-	     : kind == 1 ? launch_fused_v_u16(hw, vs, jobs, num_jobs, total_tiles, smem_bytes, grid, single, c, stream)
-	                 : launch_fused_v_f32(hw, vs, jobs, num_jobs, total_tiles, smem_bytes, grid, single, c, stream);
+	const void *k = kernel_ptr(variant);
+	cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemMax));
+	if (e != cudaSuccess)
+		return e;
+	FusedJob one = single;
+	SmemLayout layout = smem_bytes;
+	WorkChunks c = chunks;
+	void *args[] = { &jobs, &num_jobs, &total_tiles, &one, &layout, &c };
+	return cudaLaunchKernel(k, dim3(grid), dim3(kStreamThreads), args, static_cast<size_t>(layout.total_bytes), stream);
 }
 
 void fused_set_io(FusedJob &j, const void *src, ptrdiff_t src_stride, void *dst, ptrdiff_t dst_stride)
@@ -432,6 +380,10 @@ void fused_set_io(FusedJob &j, const void *src, ptrdiff_t src_stride, void *dst,
 	j.dst_stride = dst_stride;
 	auto al = [](const void *p, ptrdiff_t s) { return reinterpret_cast<uintptr_t>(p) % 16 == 0 && s % 16 == 0; };
 	j.vec_ok = al(src, src_stride) && al(dst, dst_stride) ? 1 : 0;
+	const uintptr_t a = reinterpret_cast<uintptr_t>(src) | static_cast<uintptr_t>(src_stride);
+	j.src_align = a % 16 == 0 ? 16 : (a % 8 == 0 ? 8 : (a % 4 == 0 ? 4 : 2));
+	const uintptr_t d = reinterpret_cast<uintptr_t>(dst) | static_cast<uintptr_t>(dst_stride);
+	j.dst_vec = d % (j.kind == static_cast<int>(FusedKind::F32) ? 16 : 8) == 0;
 }
 
 } // namespace zg

@@ -19,29 +19,43 @@ namespace zg {
 // Arithmetic of a fused job.
 //   F32:       float samples, taps applied in zimg's order with one fused
 //              multiply-add each; float intermediate.
-//   U16_EXACT: u16 samples computed in float on exact integers: samples are
-//              re-centred (v - 2^(depth-1)), taps are zimg's int16 taps, and the
-//              planner has proved that every partial sum stays below 2^24, so
-//              each multiply-add is exact and the result equals zimg's int32
+//   U16_EXACT: tensor cores (mma and chained kernels): u16 samples as exact
+//              integers in fp16 and fp32: samples are re-centred
+//              (v - 2^(depth-1)), taps are zimg's int16 taps, and the planner
+//              has proved that every partial sum stays below 2^24, so each
+//              multiply-add is exact and the result equals zimg's int32
 //              arithmetic bit for bit (resize_impl.cpp:31-59,78-95).
-//   U16_INT:   u16 samples where that proof fails (deeper samples: 12-bit,
-//              16-bit): zimg's own int32 arithmetic, samples centred by 32768
-//              (unpack_pixel_u16), 8192 + sum(tap * sample) in int32, then
-//              (sum >> 14) + 32768 clamped to the depth (pack_pixel_u16);
-//              planned where |taps| * 2^15 + 8192 stays below 2^31.
+//   U16_INT:   CUDA cores, any depth: zimg's own int32 arithmetic (samples
+//              centred by 32768, 8192 + sum(tap * sample), (sum >> 14) + 32768
+//              clamped to the depth; unpack_pixel_u16, pack_pixel_u16);
+//              planned where |taps| * 2^15 + 8192 stays below 2^31 and every
+//              row's taps sum to 1 << 14.
 enum class FusedKind : int { F32 = 0, U16_EXACT = 1, U16_INT = 2 };
 
 // Vertical taps come in groups of group_rows() output rows laid out densely over a
 // window of VS input lines (VS = 8, 12, 16 or 24); horizontal taps per output
-// column are padded with zeros to HW (6, 8 or 16).
+// column are padded with zeros to HW (6, 8, 12 or 16).
 // Rows per vertical group: 4 for H-first conversions (upscales: one line load
 // feeds 4 rows), 2 for V-first ones (downscales: narrower dense windows).
 __host__ __device__ constexpr int group_rows(bool h_first)
 {
 	return h_first ? 4 : 2;
 }
-constexpr int kStripW = 128;      // output columns per strip
+constexpr int kStripW = 128;      // output columns per strip (the CUDA-core kernel: at most)
 constexpr int kStreamThreads = 128;
+constexpr int kStreamWindow = 256;  // CUDA-core kernel: source samples of a strip's lines
+// CUDA-core kernel: output rows per streaming step, four vertical groups.
+__host__ __device__ constexpr int stream_step_rows(bool h_first)
+{
+	return 4 * group_rows(h_first);
+}
+
+// CUDA-core kernel: bytes of one vertical group's record: per line of its
+// window the rows' taps and the line's ring offset.
+__host__ __device__ constexpr int stream_record_bytes(bool h_first, int vs)
+{
+	return vs * (4 * group_rows(h_first) + 4);
+}
 
 // One fused job as the kernel sees it (device-resident table entry).
 struct FusedJob {
@@ -57,25 +71,27 @@ struct FusedJob {
 
 	// work items: strips x row segments
 	int strips;             // ceil(dst_w / strip_w)
-	int strip_w;            // output columns per strip (kStripW for the CUDA-core kernel)
+	int strip_w;            // output columns per strip
 	int segments;           // row segments per strip (chained kernel: one per group)
 	int seg_groups;         // vertical groups per segment (last may be shorter)
 	int groups;             // vertical groups of the plane (ceil(dst_h / group_rows))
 	int step_groups;        // vertical groups per streaming step
 	int item_begin;         // first global item index of this job
 
-	// rings (lines), powers of two
-	int ring_rows;          // V-first: source lines; H-first: intermediate lines
-	int depth;              // steps of source lines in flight (tensor-core kernel)
-	int in_rows;            // H-first: source lines staged for the H pass
+	// rings (lines; powers of two in the tensor-core kernels)
+	int ring_rows;          // CUDA-core kernel, H first: intermediate lines
+	int depth;              // steps of source lines in flight (CUDA-core kernel: 0 loads a step's lines only
+	                        // after the pass that reads the ring)
+	int in_rows;            // source lines
 
 	// H pass: taps padded to hw per output column, left[] per output column
 	const float *h_taps;    // [dst_w][hw]
 	const int *h_left;      // [dst_w]
 	int hw;
 	// V pass: dense groups of group_rows output rows over vs input lines
-	const float *v_dense;   // [groups][vs][group_rows]
-	const int *v_base;      // [groups] first input line of each group (non-decreasing)
+	const float *v_dense;   // CUDA-core kernel: records of a group's lines, taps and ring offsets (fused_kernel.cuh)
+	const int *v_base;      // [groups] first input line of each group (non-decreasing); CUDA-core kernel: [steps][2]
+	                        // first line and end of a step's windows
 	int vs;
 
 	const int *win_col;     // [strips][2] source columns [lo, hi) (lo aligned down)
@@ -85,6 +101,8 @@ struct FusedJob {
 	float pixel_max;
 	float offset;           // 2^(depth-1)
 	int vec_ok;             // planes and strides 16-byte aligned: vector loads and stores
+	int src_align;          // the largest of 16, 8, 4, 2 that divides the source's base and stride
+	int dst_vec;            // destination base and stride: 8-byte (WORD) or 16-byte (FLOAT) aligned
 	const void *tmap;       // TMA-pipelined chained kernel: the source plane's tensor map (device memory)
 	int variant;            // chained kernel's variant - 200 ((H first, KV, KH)); mixed launches dispatch on it
 };
@@ -122,7 +140,7 @@ struct FusedPlan {
 	FusedJob job{};
 	int variant = 0;         // kernel instantiation index
 	int max_pxa = 0;         // widest strip patch (elements)
-	int stage_rows = 1;      // u16 raw staging lines
+	int stage_rows = 1;      // u16 raw staging lines (mma kernel)
 	int depth = 1;           // prefetch depth in steps
 	bool mma = false;        // tensor-core variant (mma_kernel.cuh or chain_kernel.cuh)
 	bool chain = false;      // tensor-core variant with the passes chained in registers (chain_kernel.cuh)

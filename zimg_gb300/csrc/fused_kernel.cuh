@@ -1,22 +1,44 @@
-// The fused two-pass streaming kernel (template). Instantiated per variant in
-// fused_inst_*.cu.
+// The fused two-pass streaming kernel on CUDA cores (template). Instantiated
+// per variant in fused_inst_*.cu.
 //
-// A work item is one strip of 128 output columns over one segment of output
-// rows. The CTA walks the segment in steps of step_groups * 4 output rows.
-// Source lines enter a ring of lines in shared memory by cp.async one step
-// ahead of use, as zimg's graph keeps a ring of lines per filter
-// (zimg.h:387-396), so each source line is read from HBM once per strip.
+// A work item is a strip of up to 128 output columns over consecutive
+// streaming steps. Source lines enter a ring in shared memory (256 samples of
+// each line) by cp.async a step ahead of use, as zimg's graph keeps a ring of
+// lines per filter (zimg.h:387-396), so each source line is read from HBM once
+// per strip.
 //
-//   V-first step:  ring (source lines) --V--> I (intermediate lines of the
-//                  step) --H--> destination rows
-//   H-first step:  new source lines --H--> ring (intermediate lines)
-//                  ring --V--> destination rows
+//   V-first step (8 output rows):   ring (source lines) --V--> I --H--> destination
+//   H-first step (16 output rows):  new source lines --H--> ring of
+//                                   intermediate lines --V--> destination
 //
-// u16 samples are staged raw and converted once to exact centred floats, or
-// (INT, depths the float proof cannot cover) to centred int32 values held as
-// float bits, summed in zimg's int32 arithmetic. The grid is persistent: in a
-// batch CTAs take guided chunks of the units (work_chunks.cuh), otherwise an
-// equal contiguous share each.
+// F32 planes: zimg's taps in its order, one fused multiply-add each. U16
+// planes, any depth: zimg's int32 arithmetic; with taps that sum to 1 << 14,
+// its sum(tap * (v - 32768)) + 8192 is sum(tap * v) + kInit, so raw samples
+// stay as they are.
+//
+// Bound: issue slots and shared-memory bandwidth, not HBM; hence the layout.
+//  - A thread's operands come in 16 bytes: in the vertical pass four columns
+//    of a line and, in one record of the host's, two rows' taps of the line
+//    with the line's place in the ring (no ring arithmetic in the loop); in
+//    the horizontal pass four rows of a column. The intermediate block I
+//    therefore holds four rows side by side per column, its columns dealt to
+//    four planes (column x in plane x mod 4, kPlane apart), so that the
+//    vertical pass's stores and the horizontal pass's loads at strides of 1
+//    and 2 columns fall in different banks.
+//  - A thread's horizontal taps and column offsets stay in registers for the
+//    whole item. Multiply-adds are paired (two independent round-to-nearest
+//    FMAs an instruction).
+//
+// Measured against the form before it (one row at a time through planar
+// lines, ring slots computed per line, tap and sample loads of 4 bytes, u16
+// lines of unaligned planes loaded sample by sample): 16 planes 3996x2160 ->
+// 1998x1080 16-bit Spline36 930 -> 214 us; 6 planes 64x64 -> 6400x6400 f32
+// Lanczos-3 275 -> 175 us; 96 planes 1920x1080 -> 1280x720 f32 bicubic 321 ->
+// 279 us (shared-memory data path 68 % busy, a quarter of it bank conflicts of
+// the horizontal pass at 1.5 columns' stride).
+//
+// The grid is persistent: in a batch CTAs take guided chunks of the units
+// (work_chunks.cuh), otherwise an equal contiguous share each.
 #pragma once
 
 #include "fused.h"
@@ -26,18 +48,27 @@ namespace zg {
 namespace fused_detail {
 
 constexpr int kThreads = kStreamThreads;
-constexpr int kWarps = kThreads / 32;
+constexpr int kWindow = kStreamWindow;               // source samples of a strip's line in the ring
+constexpr int kPlane = 66;                           // columns of a plane of I: 2 mod 4, see above
+constexpr int kBlockBytes = 4 * kPlane * 16;         // four rows of I
+constexpr int kMidBytes = kStripW * 4;               // H first: a line of the intermediate ring
+// 8192 - 32768 * (1 << 14): zimg's rounding term and the centring of raw samples
+constexpr int kInit = 8192 - (1 << 29);
 
-__device__ __forceinline__ void cp_async16(void *smem, const void *gmem, int src_bytes)
+__device__ __forceinline__ uint32_t shared_addr(const void *p)
 {
-	const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
-	asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(src_bytes) : "memory");
+	return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
-__device__ __forceinline__ void cp_async4(void *smem, const void *gmem, int src_bytes)
+template <int BYTES>
+__device__ __forceinline__ void cp_async(void *smem, const void *gmem, int src_bytes)
 {
 	const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
-	asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(s), "l"(gmem), "r"(src_bytes) : "memory");
+	if constexpr (BYTES == 16)
+		asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(src_bytes) : "memory");
+	else
+		asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"(s), "l"(gmem), "n"(BYTES), "r"(src_bytes)
+		             : "memory");
 }
 
 __device__ __forceinline__ void cp_async_commit()
@@ -51,19 +82,9 @@ __device__ __forceinline__ void cp_async_wait()
 	asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
-// u16 exact arithmetic: acc holds 8192 + sum(tap * (v - offset)) as an exact
-// integer; round down acc / 2^14 onto the integer grid of [2^23, 2^24) and
-// clamp there. The low 16 bits of the result are zimg's packed sample
-// ((sum + 8192) >> 14, clamped, resize_impl.cpp:36-42).
-__device__ __forceinline__ float u16_round(float acc, float magic, float pixel_max)
-{
-	float y = __fmaf_rd(acc, 6.103515625e-05f, magic);
-	return fminf(fmaxf(y, 12582912.0f), 12582912.0f + pixel_max);
-}
-
-// zimg's int32 rounding (pack_pixel_u16, resize_impl.cpp:36-42): acc holds
-// 8192 + sum(tap * (v - 32768)); (acc >> 14) + 32768 clamped to [0, pixel_max].
-__device__ __forceinline__ int u16_round_int(int acc, int pixel_max)
+// zimg's rounding (pack_pixel_u16, resize_impl.cpp:36-42) of
+// 8192 + sum(tap * (v - 32768)), clamped to [0, pixel_max].
+__device__ __forceinline__ int u16_round(int acc, int pixel_max)
 {
 	return min(max((acc >> 14) + 32768, 0), pixel_max);
 }
@@ -87,456 +108,501 @@ struct Item {
 	ptrdiff_t src_stride;
 	char *dst;
 	ptrdiff_t dst_stride;
-	const char *v_dense;
-	const int *v_base;
-	int src_w, src_h, dst_h, vec_ok;
+	const char *records;
+	const int2 *ranges;
+	int src_w, src_h, dst_h, src_align, dst_vec;
 	int c0, cols_valid, xlo, pxa;
-	int g_begin, g_end, step_groups, units;
-	float magic, pixel_max, offset;
+	int step0, steps, ring_rows, in_rows;
+	bool late;
+	int pixel_max;
 };
 
-// Units t .. t_end - 1 of job J that lie in the strip of unit t, at most
-// L.seg_groups groups of them: a work item. A job's units are its (strip,
-// streaming step) pairs, strip-major.
-template <int HW>
-__device__ __forceinline__ Item make_item(const FusedJob &J, int t, int t_end, char *smem, const SmemLayout &L)
+// Units t .. t_end - 1 of job J that lie in the strip of unit t: a work item.
+// A job's units are its (strip, streaming step) pairs, strip-major.
+__device__ __forceinline__ Item make_item(const FusedJob &J, int t, int t_end)
 {
 	Item it;
 	const int local = t - J.item_begin;
 	const int strip = local / J.segments;
-	const int step0 = local - strip * J.segments;
-	it.units = max(1, min(min(J.segments - step0, t_end - t), L.seg_groups / J.step_groups));
+	it.step0 = local - strip * J.segments;
+	it.steps = min(J.segments - it.step0, t_end - t);
 	it.src = static_cast<const char *>(J.src);
 	it.src_stride = J.src_stride;
 	it.dst = static_cast<char *>(J.dst);
 	it.dst_stride = J.dst_stride;
-	it.v_dense = reinterpret_cast<const char *>(J.v_dense);
-	it.v_base = J.v_base;
+	it.records = reinterpret_cast<const char *>(J.v_dense);
+	it.ranges = reinterpret_cast<const int2 *>(J.v_base);
 	it.src_w = J.src_w;
 	it.src_h = J.src_h;
 	it.dst_h = J.dst_h;
-	it.vec_ok = J.vec_ok;
-	it.c0 = strip * kStripW;
-	it.cols_valid = min(kStripW, J.dst_w - it.c0);
+	it.src_align = J.src_align;
+	it.dst_vec = J.dst_vec;
+	it.c0 = strip * J.strip_w;
+	it.cols_valid = min(J.strip_w, J.dst_w - it.c0);
 	it.xlo = __ldg(J.win_col + 2 * strip);
 	it.pxa = (__ldg(J.win_col + 2 * strip + 1) - it.xlo + 7) & ~7;
-	it.g_begin = step0 * J.step_groups;
-	it.g_end = min(J.groups, (step0 + it.units) * J.step_groups);
-	it.step_groups = J.step_groups;
-	it.magic = J.magic;
-	it.pixel_max = J.pixel_max;
-	it.offset = J.offset;
-
-	// per-item tables: h taps and left offsets of the strip, group bases
-	const char *ht = reinterpret_cast<const char *>(J.h_taps) + static_cast<size_t>(it.c0) * HW * 4;
-	const int tap_bytes = it.cols_valid * HW * 4;
-	for (int i = threadIdx.x; i < kStripW * HW / 4; i += kThreads) {
-		const int n = max(0, min(16, tap_bytes - i * 16));
-		cp_async16(smem + L.htaps_off + i * 16, n ? ht + i * 16 : ht, n);
-	}
-	for (int i = threadIdx.x; i < kStripW / 4; i += kThreads) {
-		const int n = max(0, min(4, it.cols_valid - 4 * i));
-		cp_async16(smem + L.hleft_off + i * 16, n ? J.h_left + it.c0 + 4 * i : J.h_left, n * 4);
-	}
-	int *vb = reinterpret_cast<int *>(smem + L.vbase_off);
-	for (int g = it.g_begin + threadIdx.x; g < it.g_end; g += kThreads)
-		vb[g - it.g_begin] = __ldg(J.v_base + g);
+	it.ring_rows = J.ring_rows;
+	it.in_rows = J.in_rows;
+	it.late = J.depth == 0;
+	it.pixel_max = static_cast<int>(J.pixel_max);
 	return it;
 }
 
-// Lines [a, b) of the source strip into ring slots (line & mask) of `ring`
-// (pitch elements of E bytes per line), zero outside the plane. Aligned
-// planes: thread t copies 16-byte chunk t % chunks of lines a + t / chunks,
-// then every kThreads / chunks lines further (one address step per line).
-// Otherwise warp w takes lines a + w, a + w + 4, ... sample by sample.
-template <bool U16>
-__device__ __forceinline__ void load_lines(const Item &it, int a, int b, char *ring, int mask, int pitch)
+// A 16-byte chunk of a line whose samples start 2 mod 4 bytes off a word, or
+// on one: aligned 4-byte loads and a shift where the chunk and the samples
+// beside it lie in the line, else sample by sample. Zeros outside the plane.
+__device__ __forceinline__ uint4 load_chunk_u16(const uint16_t *row, int gx, int src_w)
 {
-	constexpr int E = U16 ? 2 : 4;
-	constexpr int PER = 16 / E;
-	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-	if (it.vec_ok) {
-		const int chunks = it.pxa / PER;
-		const int lpp = kThreads / chunks;
-		if (lpp == 0) {
-			// strips wider than kThreads chunks: warp per line
-			for (int y = a + warp; y < b; y += kWarps) {
-				const bool row_ok = y < it.src_h;
-				const char *row = it.src + static_cast<ptrdiff_t>(row_ok ? y : 0) * it.src_stride;
-				char *srow = ring + (y & mask) * pitch * E;
-				for (int q = lane; q < chunks; q += 32) {
-					const int gx = it.xlo + q * PER;
-					const int n = row_ok ? max(0, min(PER, it.src_w - gx)) : 0;
-					cp_async16(srow + q * 16, n ? row + static_cast<ptrdiff_t>(gx) * E : it.src, n * E);
-				}
+	uint32_t w[4];
+	const bool odd = (reinterpret_cast<uintptr_t>(row + gx) & 2) != 0;
+	if (gx >= 1 && gx + 9 <= src_w) {
+		const uint32_t *p = reinterpret_cast<const uint32_t *>(row + gx - (odd ? 1 : 0));
+		uint32_t v[5];
+#pragma unroll
+		for (int k = 0; k < 4; ++k)
+			v[k] = __ldg(p + k);
+		v[4] = odd ? __ldg(p + 4) : 0u;
+#pragma unroll
+		for (int k = 0; k < 4; ++k)
+			w[k] = odd ? __byte_perm(v[k], v[k + 1], 0x5432) : v[k];
+	} else {
+#pragma unroll
+		for (int k = 0; k < 4; ++k) {
+			const int x = gx + 2 * k;
+			const uint32_t lo = x < src_w ? __ldg(row + x) : 0u, hi = x + 1 < src_w ? __ldg(row + x + 1) : 0u;
+			w[k] = lo | (hi << 16);
+		}
+	}
+	return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// Source lines [a, b) of the strip into slots of a ring of `rows` lines, zero
+// outside the plane; line a goes to slot `slot`. A thread copies one 16-byte
+// chunk of every kLines-th line, with the widest copies that the plane's
+// alignment allows.
+template <int E>
+__device__ __forceinline__ void load_lines(const Item &it, int a, int b, char *ring, int rows, int slot)
+{
+	constexpr int kPer = 16 / E;                       // samples a chunk
+	constexpr int kChunks = kWindow / kPer;            // chunks a line
+	constexpr int kLines = kThreads / kChunks;         // lines a pass
+	const int q = threadIdx.x % kChunks, l0 = threadIdx.x / kChunks;
+	if (q * kPer >= it.pxa)
+		return;
+	const int gx = it.xlo + q * kPer;
+	const int nb = max(0, min(kPer, it.src_w - gx)) * E;
+	slot += l0;
+	slot = slot >= rows ? slot - rows : slot;
+	const char *src = it.src + static_cast<ptrdiff_t>(a + l0) * it.src_stride + static_cast<ptrdiff_t>(gx) * E;
+	const ptrdiff_t step = kLines * it.src_stride;
+	if (it.src_align == 16) {
+		const uint32_t base = shared_addr(ring) + q * 16, end = base + rows * (kWindow * E);
+		uint32_t d = base + slot * (kWindow * E);
+		if (nb == 16 && b <= it.src_h) {
+#pragma unroll 2
+			for (int y = a + l0; y < b; y += kLines) {
+				asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
+				src += step;
+				d += kLines * (kWindow * E);
+				d = d >= end ? d - rows * (kWindow * E) : d;
 			}
 			return;
 		}
-		const int q = threadIdx.x % chunks, l0 = threadIdx.x / chunks;
-		if (l0 >= lpp)
-			return;
-		const int gx = it.xlo + q * PER;
-		const int nb = max(0, min(PER, it.src_w - gx)) * E;
-		const char *src = it.src + (nb ? static_cast<ptrdiff_t>(gx) * E : 0) + static_cast<ptrdiff_t>(a + l0) * it.src_stride;
-		const ptrdiff_t step = static_cast<ptrdiff_t>(lpp) * it.src_stride;
-		for (int y = a + l0; y < b; y += lpp, src += step) {
-			const bool ok = y < it.src_h && nb;
-			cp_async16(ring + ((y & mask) * pitch * E) + q * 16, ok ? src : it.src, ok ? nb : 0);
+		if (!nb)
+			src = it.src;
+		for (int y = a + l0; y < b; y += kLines) {
+			const int n = y < it.src_h ? nb : 0;
+			asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(n ? src : it.src), "r"(n) : "memory");
+			src += step;
+			d += kLines * (kWindow * E);
+			d = d >= end ? d - rows * (kWindow * E) : d;
 		}
 		return;
 	}
-	for (int y = a + warp; y < b; y += kWarps) {
-		const bool row_ok = y < it.src_h;
-		const char *row = it.src + static_cast<ptrdiff_t>(row_ok ? y : 0) * it.src_stride;
-		char *srow = ring + (y & mask) * pitch * E;
-		if (!U16) {
-			for (int x = lane; x < it.pxa; x += 32) {
-				const int gx = it.xlo + x;
-				const bool ok = row_ok && gx < it.src_w;
-				cp_async4(srow + x * 4, ok ? row + static_cast<ptrdiff_t>(gx) * 4 : it.src, ok ? 4 : 0);
+	for (int y = a + l0; y < b; y += kLines, src += step) {
+		char *d = ring + slot * (kWindow * E) + q * 16;
+		slot += kLines;
+		slot = slot >= rows ? slot - rows : slot;
+		const int n = y < it.src_h ? nb : 0;
+		if (it.src_align == 8) {
+#pragma unroll
+			for (int k = 0; k < 2; ++k) {
+				const int m = max(0, min(8, n - 8 * k));
+				cp_async<8>(d + 8 * k, m ? src + 8 * k : it.src, m);
+			}
+		} else if (E == 4 || it.src_align == 4) {
+#pragma unroll
+			for (int k = 0; k < 4; ++k) {
+				const int m = max(0, min(4, n - 4 * k));
+				cp_async<4>(d + 4 * k, m ? src + 4 * k : it.src, m);
 			}
 		} else {
-			for (int x = lane; x < it.pxa; x += 32) {
-				const int gx = it.xlo + x;
-				const bool ok = row_ok && gx < it.src_w;
-				reinterpret_cast<uint16_t *>(srow)[x] =
-					ok ? __ldg(reinterpret_cast<const uint16_t *>(row) + gx) : static_cast<uint16_t>(0);
-			}
+			uint4 v = make_uint4(0, 0, 0, 0);
+			if (n)
+				v = load_chunk_u16(reinterpret_cast<const uint16_t *>(src) - gx, gx, it.src_w);
+			*reinterpret_cast<uint4 *>(d) = v;
 		}
 	}
 }
 
-// Convert the u16 lines this thread loaded with load_lines(a, b) from the
-// raw staging ring to centred floats in `ring` (INT: v - 32768 as int32 bits).
-template <bool INT>
-__device__ __forceinline__ void convert_chunk(const char *srow, float *drow, int q, float bias)
+// `bytes` (a multiple of 16) of a step's records.
+__device__ __forceinline__ void load_records(const char *src, char *dst, int bytes)
 {
-	const uint4 u = *reinterpret_cast<const uint4 *>(srow + q * 16);
-	const uint32_t w[4] = { u.x, u.y, u.z, u.w };
-	float f[8];
-#pragma unroll
-	for (int k = 0; k < 8; ++k) {
-		const uint32_t v = (w[k >> 1] >> (16 * (k & 1))) & 0xFFFFu;
-		f[k] = INT ? __int_as_float(static_cast<int>(v) - 32768) : __int_as_float(0x4B000000 | v) - bias;
-	}
-	*reinterpret_cast<float4 *>(drow + q * 8) = make_float4(f[0], f[1], f[2], f[3]);
-	*reinterpret_cast<float4 *>(drow + q * 8 + 4) = make_float4(f[4], f[5], f[6], f[7]);
+	for (int i = threadIdx.x * 16; i < bytes; i += kThreads * 16)
+		cp_async<16>(dst + i, src + i, 16);
 }
 
-// Convert the u16 lines [a, b) from the raw staging ring to centred floats
-// in `ring`. With cp.async copies each thread converts exactly the chunks it
-// copied (the mapping of load_lines); plain loads were made visible by a
-// CTA barrier, so any mapping serves.
-template <bool INT>
-__device__ __forceinline__ void convert_lines(const Item &it, int a, int b, const char *stage, int smask,
-                                              float *ring, int rmask, int pitch)
+// Loads by 32-bit shared address (no generic address arithmetic in the loops).
+__device__ __forceinline__ float4 lds_f4(uint32_t a)
 {
-	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-	const float bias = 8388608.0f + it.offset;
-	const int chunks = it.pxa / 8;
-	const int lpp = kThreads / chunks;
-	if (it.vec_ok && lpp) {
-		const int q = threadIdx.x % chunks, l0 = threadIdx.x / chunks;
-		if (l0 >= lpp)
-			return;
-		for (int y = a + l0; y < b; y += lpp)
-			convert_chunk<INT>(stage + (y & smask) * pitch * 2, ring + (y & rmask) * pitch, q, bias);
+	float4 v;
+	asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];\n" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
+	return v;
+}
+
+__device__ __forceinline__ int4 lds_i4(uint32_t a)
+{
+	int4 v;
+	asm volatile("ld.shared.v4.s32 {%0, %1, %2, %3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
+	return v;
+}
+
+__device__ __forceinline__ uint2 lds_u2(uint32_t a)
+{
+	uint2 v;
+	asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];\n" : "=r"(v.x), "=r"(v.y) : "r"(a));
+	return v;
+}
+
+__device__ __forceinline__ uint32_t lds_u1(uint32_t a)
+{
+	uint32_t v;
+	asm volatile("ld.shared.u32 %0, [%1];\n" : "=r"(v) : "r"(a));
+	return v;
+}
+
+__device__ __forceinline__ int lds_u16(uint32_t a)
+{
+	uint16_t v;
+	asm volatile("ld.shared.u16 %0, [%1];\n" : "=h"(v) : "r"(a));
+	return v;
+}
+
+__device__ __forceinline__ void sts_f4(uint32_t a, float x, float y, float z, float w)
+{
+	asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};\n" ::"r"(a), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
+}
+
+__device__ __forceinline__ float2 dup(float x)
+{
+	return make_float2(x, x);
+}
+
+// V first, vertical pass: thread = four columns (quad q) of four rows (half 0
+// or 1 of the step's eight), two groups of two rows. A group's record: the two rows' taps of each line of its
+// window, then the lines' byte offsets in the ring. The paired FMAs take the
+// two rows of a column, so that four rows end up side by side as I has them.
+template <bool INT, int VS>
+__device__ __forceinline__ void vfirst_v(const Item &it, uint32_t ring, uint32_t records, uint32_t I, int q, int half)
+{
+	if (half >= 2)
 		return;
+	constexpr int kRecord = stream_record_bytes(false, VS), kTaps = 8;
+	const uint32_t col = ring + q * (INT ? 8 : 16);
+	float2 out[2][4];  // [group][column]: the group's two rows (INT: int bits)
+#pragma unroll
+	for (int g = 0; g < 2; ++g) {
+		const uint32_t rec = records + (2 * half + g) * kRecord;
+		if constexpr (INT) {
+			int acc[2][4];
+#pragma unroll
+			for (int j = 0; j < 2; ++j)
+#pragma unroll
+				for (int e = 0; e < 4; ++e)
+					acc[j][e] = kInit;
+#pragma unroll (VS <= 8 ? 2 : 1)
+			for (int s4 = 0; s4 < VS; s4 += 4) {
+				const int4 o = lds_i4(rec + VS * kTaps + s4 * 4);
+				const int at[4] = { o.x, o.y, o.z, o.w };
+#pragma unroll
+				for (int s2 = 0; s2 < 4; s2 += 2) {
+					const int4 r = lds_i4(rec + (s4 + s2) * kTaps);
+					const int tap[2][2] = { { r.x, r.y }, { r.z, r.w } };
+#pragma unroll
+					for (int i = 0; i < 2; ++i) {
+						const uint2 x = lds_u2(col + at[s2 + i]);
+						const int v[4] = { static_cast<int>(x.x & 0xFFFFu), static_cast<int>(x.x >> 16),
+						                   static_cast<int>(x.y & 0xFFFFu), static_cast<int>(x.y >> 16) };
+#pragma unroll
+						for (int e = 0; e < 4; ++e) {
+							acc[0][e] += tap[i][0] * v[e];
+							acc[1][e] += tap[i][1] * v[e];
+						}
+					}
+				}
+			}
+#pragma unroll
+			for (int e = 0; e < 4; ++e)
+				out[g][e] = make_float2(__int_as_float(u16_round(acc[0][e], it.pixel_max)),
+				                        __int_as_float(u16_round(acc[1][e], it.pixel_max)));
+		} else {
+#pragma unroll
+			for (int e = 0; e < 4; ++e)
+				out[g][e] = dup(0.0f);
+#pragma unroll (VS <= 8 ? 2 : 1)
+			for (int s4 = 0; s4 < VS; s4 += 4) {
+				const int4 o = lds_i4(rec + VS * kTaps + s4 * 4);
+				const int at[4] = { o.x, o.y, o.z, o.w };
+#pragma unroll
+				for (int s2 = 0; s2 < 4; s2 += 2) {
+					const float4 r = lds_f4(rec + (s4 + s2) * kTaps);
+					const float2 tap[2] = { make_float2(r.x, r.y), make_float2(r.z, r.w) };
+#pragma unroll
+					for (int i = 0; i < 2; ++i) {
+						const float4 x = lds_f4(col + at[s2 + i]);
+						out[g][0] = __ffma2_rn(dup(x.x), tap[i], out[g][0]);
+						out[g][1] = __ffma2_rn(dup(x.y), tap[i], out[g][1]);
+						out[g][2] = __ffma2_rn(dup(x.z), tap[i], out[g][2]);
+						out[g][3] = __ffma2_rn(dup(x.w), tap[i], out[g][3]);
+					}
+				}
+			}
+		}
 	}
-	for (int y = a + warp; y < b; y += kWarps) {
-		const char *srow = stage + (y & smask) * pitch * 2;
-		float *drow = ring + (y & rmask) * pitch;
-		for (int q = lane; q < chunks; q += 32)
-			convert_chunk<INT>(srow, drow, q, bias);
-	}
+	const uint32_t d = I + half * kBlockBytes + q * 16;
+#pragma unroll
+	for (int e = 0; e < 4; ++e)
+		sts_f4(d + e * (kPlane * 16), out[0][e].x, out[0][e].y, out[1][e].x, out[1][e].y);
 }
 
-// Horizontal pass over lines [a, b): out[y][c] = sum_k taps[c][k] * in[y][left[c] - xlo + k].
-// Thread = output column; two lines per iteration for independent chains.
-// FINAL: write destination rows (row index = r0 + (y - a)); else write ring
-// slots (y & omask) of `out`.
-template <bool U16, bool FINAL, int HW, bool INT = false>
-__device__ __forceinline__ void h_pass(const Item &it, const char *smem, const SmemLayout &L, const float *in,
-                                       int imask, int a, int b, float *out, int omask, int r0)
+// V first, horizontal pass: thread = one output column of eight rows.
+// at[k]: address in I of the column of tap k.
+template <bool INT, int HW>
+__device__ __forceinline__ void vfirst_h(const Item &it, const float (&taps)[HW], const uint32_t (&at)[HW], int row0)
 {
 	const int c = threadIdx.x;
-	const bool col_ok = c < it.cols_valid;
-	float taps[HW];
-	const float2 *tp = reinterpret_cast<const float2 *>(smem + L.htaps_off) + c * (HW / 2);
+	if (c >= it.cols_valid)
+		return;
+	constexpr int E = INT ? 2 : 4;
+	char *d = it.dst + static_cast<ptrdiff_t>(row0) * it.dst_stride + static_cast<ptrdiff_t>(it.c0 + c) * E;
+	const int rows = it.dst_h - row0;
 #pragma unroll
-	for (int k = 0; k < HW / 2; ++k) {
-		const float2 t2 = tp[k];
-		taps[2 * k] = t2.x;
-		taps[2 * k + 1] = t2.y;
+	for (int b = 0; b < 2; ++b) {
+		float v[4];
+		if constexpr (INT) {
+			int acc[4] = { kInit, kInit, kInit, kInit };
+#pragma unroll
+			for (int k = 0; k < HW; ++k) {
+				const int4 x = lds_i4(at[k] + b * kBlockBytes);
+				const int t = __float_as_int(taps[k]);
+				acc[0] += t * x.x;
+				acc[1] += t * x.y;
+				acc[2] += t * x.z;
+				acc[3] += t * x.w;
+			}
+#pragma unroll
+			for (int j = 0; j < 4; ++j)
+				v[j] = __int_as_float(u16_round(acc[j], it.pixel_max));
+		} else {
+			float2 a01 = dup(0.0f), a23 = dup(0.0f);
+#pragma unroll
+			for (int k = 0; k < HW; ++k) {
+				const float4 x = lds_f4(at[k] + b * kBlockBytes);
+				a01 = __ffma2_rn(dup(taps[k]), make_float2(x.x, x.y), a01);
+				a23 = __ffma2_rn(dup(taps[k]), make_float2(x.z, x.w), a23);
+			}
+			v[0] = a01.x;
+			v[1] = a01.y;
+			v[2] = a23.x;
+			v[3] = a23.y;
+		}
+		auto store = [&](int j) {
+			if constexpr (INT)
+				*reinterpret_cast<uint16_t *>(d) = static_cast<uint16_t>(__float_as_int(v[j]));
+			else
+				*reinterpret_cast<float *>(d) = v[j];
+			d += it.dst_stride;
+		};
+		if (4 * b + 4 <= rows) {
+#pragma unroll
+			for (int j = 0; j < 4; ++j)
+				store(j);
+		} else {
+			for (int j = 0; j < 4; ++j)
+				if (4 * b + j < rows)
+					store(j);
+		}
 	}
-	const int l = col_ok ? reinterpret_cast<const int *>(smem + L.hleft_off)[c] - it.xlo : 0;
-	const float init = U16 ? 8192.0f : 0.0f;
-	const int pitch = L.pitch;
-	if constexpr (INT) {
-		// zimg's int32 sums (taps and centred samples as int32 bits)
-		const int pmax = static_cast<int>(it.pixel_max);
-		for (int y = a; y < b; y += 2) {
-			const bool two = y + 1 < b;
-			const float *r0p = in + (y & imask) * pitch + l;
-			const float *r1p = in + ((y + 1) & imask) * pitch + l;
-			int acc0 = 8192, acc1 = 8192;
+}
+
+// H first, horizontal pass: lines [a, b) (multiples of 4) from the ring of
+// source lines into the intermediate ring; thread = one output column, four
+// lines at a time. l: the column's first input in the strip's lines.
+template <bool INT, int HW>
+__device__ __forceinline__ void hfirst_h(const Item &it, uint32_t in, const float (&taps)[HW], int l, int a, int b,
+                                         int in_slot, char *mid, int mid_slot)
+{
+	constexpr int E = INT ? 2 : 4, LB = kWindow * E;
+	const int c = threadIdx.x;
+	for (int y = a; y < b; y += 4) {
+		const uint32_t r = in + in_slot * LB + l * E;
+		float v[4];
+		if constexpr (INT) {
+			int acc[4] = { kInit, kInit, kInit, kInit };
 #pragma unroll
 			for (int k = 0; k < HW; ++k) {
 				const int t = __float_as_int(taps[k]);
-				acc0 += t * __float_as_int(r0p[k]);
-				acc1 += t * __float_as_int(r1p[k]);
+#pragma unroll
+				for (int i = 0; i < 4; ++i)
+					acc[i] += t * lds_u16(r + i * LB + k * 2);
 			}
-			const int q0 = u16_round_int(acc0, pmax), q1 = u16_round_int(acc1, pmax);
-			if (!FINAL) {
-				out[(y & omask) * kStripW + c] = __int_as_float(q0 - 32768);
-				if (two)
-					out[((y + 1) & omask) * kStripW + c] = __int_as_float(q1 - 32768);
-			} else if (col_ok) {
-				const int oy = r0 + (y - a);
-				char *d0 = it.dst + static_cast<ptrdiff_t>(oy) * it.dst_stride;
-				if (oy < it.dst_h)
-					reinterpret_cast<uint16_t *>(d0)[it.c0 + c] = static_cast<uint16_t>(q0);
-				if (two && oy + 1 < it.dst_h)
-					reinterpret_cast<uint16_t *>(d0 + it.dst_stride)[it.c0 + c] = static_cast<uint16_t>(q1);
+#pragma unroll
+			for (int i = 0; i < 4; ++i)
+				v[i] = __int_as_float(u16_round(acc[i], it.pixel_max));
+		} else {
+			float2 a01 = dup(0.0f), a23 = dup(0.0f);
+#pragma unroll
+			for (int k = 0; k < HW; ++k) {
+				float x[4];
+#pragma unroll
+				for (int i = 0; i < 4; ++i)
+					x[i] = __uint_as_float(lds_u1(r + i * LB + k * 4));
+				a01 = __ffma2_rn(dup(taps[k]), make_float2(x[0], x[1]), a01);
+				a23 = __ffma2_rn(dup(taps[k]), make_float2(x[2], x[3]), a23);
 			}
+			v[0] = a01.x;
+			v[1] = a01.y;
+			v[2] = a23.x;
+			v[3] = a23.y;
 		}
+		char *d = mid + mid_slot * kMidBytes + c * 4;
+#pragma unroll
+		for (int i = 0; i < 4; ++i)
+			*reinterpret_cast<float *>(d + i * kMidBytes) = v[i];
+		in_slot = in_slot + 4 >= it.in_rows ? 0 : in_slot + 4;
+		mid_slot = mid_slot + 4 >= it.ring_rows ? 0 : mid_slot + 4;
+	}
+}
+
+// H first, vertical pass: a warp takes a group of four output rows, a lane
+// four columns. A group's record: the four rows' taps of each line of its
+// window, then the lines' byte offsets in the intermediate ring.
+template <bool INT, int VS>
+__device__ __forceinline__ void hfirst_v(const Item &it, uint32_t mid, uint32_t records, int row0)
+{
+	const int warp = threadIdx.x >> 5, q = threadIdx.x & 31;
+	const int r0 = row0 + 4 * warp;
+	if (r0 >= it.dst_h || 4 * q >= it.cols_valid)
 		return;
-	}
-	for (int y = a; y < b; y += 2) {
-		const bool two = y + 1 < b;
-		const float *r0p = in + (y & imask) * pitch + l;
-		const float *r1p = in + ((y + 1) & imask) * pitch + l;
-		// the two lines in one paired FMA per tap (two independent
-		// round-to-nearest FMAs, as the scalar form)
-		float2 acc = make_float2(init, init);
+	constexpr int E = INT ? 2 : 4;
+	constexpr int kTaps = 16;
+	const uint32_t rec = records + warp * stream_record_bytes(true, VS);
+	const uint32_t col = mid + q * 16;
+	char *d = it.dst + static_cast<ptrdiff_t>(r0) * it.dst_stride + static_cast<ptrdiff_t>(it.c0 + 4 * q) * E;
+	const bool wide = it.dst_vec && 4 * q + 4 <= it.cols_valid;
+	float out[4][4];  // [row][column]
+	if constexpr (INT) {
+		int acc[4][4];
 #pragma unroll
-		for (int k = 0; k < HW; ++k)
-			acc = __ffma2_rn(make_float2(taps[k], taps[k]), make_float2(r0p[k], r1p[k]), acc);
-		const float acc0 = acc.x, acc1 = acc.y;
-		if (!FINAL) {
-			float v0 = acc0, v1 = acc1;
-			if (U16) {
-				v0 = u16_round(acc0, it.magic, it.pixel_max) - it.magic;
-				v1 = u16_round(acc1, it.magic, it.pixel_max) - it.magic;
-			}
-			out[(y & omask) * kStripW + c] = v0;
-			if (two)
-				out[((y + 1) & omask) * kStripW + c] = v1;
-		} else if (col_ok) {
-			const int oy = r0 + (y - a);
-			char *d0 = it.dst + static_cast<ptrdiff_t>(oy) * it.dst_stride;
-			if (U16) {
-				const uint32_t q0 = __float_as_uint(u16_round(acc0, it.magic, it.pixel_max)) & 0xFFFFu;
-				const uint32_t q1 = __float_as_uint(u16_round(acc1, it.magic, it.pixel_max)) & 0xFFFFu;
-				if (oy < it.dst_h)
-					reinterpret_cast<uint16_t *>(d0)[it.c0 + c] = static_cast<uint16_t>(q0);
-				if (two && oy + 1 < it.dst_h)
-					reinterpret_cast<uint16_t *>(d0 + it.dst_stride)[it.c0 + c] = static_cast<uint16_t>(q1);
-			} else {
-				if (oy < it.dst_h)
-					reinterpret_cast<float *>(d0)[it.c0 + c] = acc0;
-				if (two && oy + 1 < it.dst_h)
-					reinterpret_cast<float *>(d0 + it.dst_stride)[it.c0 + c] = acc1;
+		for (int j = 0; j < 4; ++j)
+#pragma unroll
+			for (int e = 0; e < 4; ++e)
+				acc[j][e] = kInit;
+#pragma unroll (VS <= 8 ? 2 : 1)
+		for (int s4 = 0; s4 < VS; s4 += 4) {
+			const int4 o = lds_i4(rec + VS * kTaps + s4 * 4);
+			const int at[4] = { o.x, o.y, o.z, o.w };
+#pragma unroll
+			for (int i = 0; i < 4; ++i) {
+				const int4 t = lds_i4(rec + (s4 + i) * kTaps);
+				const int4 x = lds_i4(col + at[i]);
+				const int tj[4] = { t.x, t.y, t.z, t.w };
+#pragma unroll
+				for (int j = 0; j < 4; ++j) {
+					acc[j][0] += tj[j] * x.x;
+					acc[j][1] += tj[j] * x.y;
+					acc[j][2] += tj[j] * x.z;
+					acc[j][3] += tj[j] * x.w;
+				}
 			}
 		}
-	}
-}
-
-// Vertical pass for groups [g0, g1): out line (g - g0)*4 + j, columns 4q..4q+3:
-//   sum_s dense[g][s][j] * in[(base[g] + s) & imask][4q + e]
-// FINAL: destination rows g*4 + j (columns c0 + 4q ...); else lines of I.
-template <bool U16, bool FINAL, int VS, int kGroup, bool INT = false>
-__device__ __forceinline__ void v_pass(const Item &it, const char *smem, const SmemLayout &L, const float *in,
-                                       int imask, int in_pitch, int g0, int g1, const float *coef, int quads,
-                                       float *I, int i_pitch)
-{
-	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-	const float init = U16 ? 8192.0f : 0.0f;
-	const int ng = g1 - g0;
-	const int wpg = ng >= kWarps ? 1 : kWarps / ng;  // warps per group
-	const int *vb = reinterpret_cast<const int *>(smem + L.vbase_off);
-	for (int gi = warp / wpg; gi < ng; gi += kWarps / wpg) {
-		const int g = g0 + gi;
-		const int base = vb[g - it.g_begin];
-		const float *cf = coef + gi * VS * kGroup;  // [line][row] taps of the group's rows
-		int off[VS];
 #pragma unroll
-		for (int s = 0; s < VS; ++s)
-			off[s] = ((base + s) & imask) * in_pitch;
-		for (int q = (warp % wpg) * 32 + lane; q < quads; q += wpg * 32) {
-			if constexpr (INT) {
-				// zimg's int32 sums (taps and centred samples as int32 bits)
-				int acc[kGroup][4];
+		for (int j = 0; j < 4; ++j)
 #pragma unroll
-				for (int j = 0; j < kGroup; ++j)
-					acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 8192;
+			for (int e = 0; e < 4; ++e)
+				out[j][e] = __int_as_float(u16_round(acc[j][e], it.pixel_max));
+	} else {
+		float2 acc[4][2];
 #pragma unroll
-				for (int s = 0; s < VS; ++s) {
-					const int4 x = *reinterpret_cast<const int4 *>(in + off[s] + 4 * q);
+		for (int j = 0; j < 4; ++j)
+			acc[j][0] = acc[j][1] = dup(0.0f);
+#pragma unroll (VS <= 8 ? 2 : 1)
+		for (int s4 = 0; s4 < VS; s4 += 4) {
+			const int4 o = lds_i4(rec + VS * kTaps + s4 * 4);
+			const int at[4] = { o.x, o.y, o.z, o.w };
 #pragma unroll
-					for (int j = 0; j < kGroup; ++j) {
-						const int cj = __float_as_int(cf[s * kGroup + j]);
-						acc[j][0] += cj * x.x;
-						acc[j][1] += cj * x.y;
-						acc[j][2] += cj * x.z;
-						acc[j][3] += cj * x.w;
-					}
-				}
-				const int pmax = static_cast<int>(it.pixel_max);
-#pragma unroll
-				for (int j = 0; j < kGroup; ++j) {
-					int u[4];
-#pragma unroll
-					for (int e = 0; e < 4; ++e)
-						u[e] = u16_round_int(acc[j][e], pmax);
-					if (!FINAL) {
-						*reinterpret_cast<int4 *>(I + (gi * kGroup + j) * i_pitch + 4 * q) =
-							make_int4(u[0] - 32768, u[1] - 32768, u[2] - 32768, u[3] - 32768);
-					} else {
-						const int r = g * kGroup + j;
-						if (r >= it.dst_h)
-							continue;
-						const int x0 = 4 * q;
-						uint16_t *d = reinterpret_cast<uint16_t *>(it.dst + static_cast<ptrdiff_t>(r) * it.dst_stride) +
-						              it.c0 + x0;
-						if (it.vec_ok && x0 + 3 < it.cols_valid) {
-							*reinterpret_cast<uint2 *>(d) = make_uint2(static_cast<uint32_t>(u[0]) | (static_cast<uint32_t>(u[1]) << 16),
-							                                           static_cast<uint32_t>(u[2]) | (static_cast<uint32_t>(u[3]) << 16));
-						} else {
-#pragma unroll
-							for (int e = 0; e < 4; ++e)
-								if (x0 + e < it.cols_valid)
-									d[e] = static_cast<uint16_t>(u[e]);
-						}
-					}
-				}
-				continue;
-			}
-			// columns (0, 1) and (2, 3) of each row in paired FMAs: two
-			// independent round-to-nearest FMAs per instruction, the same
-			// results as four scalar ones
-			float2 acc2[kGroup][2];
-#pragma unroll
-			for (int j = 0; j < kGroup; ++j)
-				acc2[j][0] = acc2[j][1] = make_float2(init, init);
-#pragma unroll
-			for (int s = 0; s < VS; ++s) {
-				const float4 x = *reinterpret_cast<const float4 *>(in + off[s] + 4 * q);
+			for (int i = 0; i < 4; ++i) {
+				const float4 t = lds_f4(rec + (s4 + i) * kTaps);
+				const float4 x = lds_f4(col + at[i]);
 				const float2 x01 = make_float2(x.x, x.y), x23 = make_float2(x.z, x.w);
-				float cj[kGroup];
-				if constexpr (kGroup == 4) {
-					const float4 c4 = reinterpret_cast<const float4 *>(cf)[s];
-					cj[0] = c4.x;
-					cj[1] = c4.y;
-					cj[2] = c4.z;
-					cj[3] = c4.w;
-				} else {
-					const float2 c2 = reinterpret_cast<const float2 *>(cf)[s];
-					cj[0] = c2.x;
-					cj[1] = c2.y;
-				}
+				const float tj[4] = { t.x, t.y, t.z, t.w };
 #pragma unroll
-				for (int j = 0; j < kGroup; ++j) {
-					const float2 cc = make_float2(cj[j], cj[j]);
-					acc2[j][0] = __ffma2_rn(cc, x01, acc2[j][0]);
-					acc2[j][1] = __ffma2_rn(cc, x23, acc2[j][1]);
+				for (int j = 0; j < 4; ++j) {
+					acc[j][0] = __ffma2_rn(dup(tj[j]), x01, acc[j][0]);
+					acc[j][1] = __ffma2_rn(dup(tj[j]), x23, acc[j][1]);
 				}
 			}
-			float acc[kGroup][4];
+		}
 #pragma unroll
-			for (int j = 0; j < kGroup; ++j) {
-				acc[j][0] = acc2[j][0].x;
-				acc[j][1] = acc2[j][0].y;
-				acc[j][2] = acc2[j][1].x;
-				acc[j][3] = acc2[j][1].y;
+		for (int j = 0; j < 4; ++j) {
+			out[j][0] = acc[j][0].x;
+			out[j][1] = acc[j][0].y;
+			out[j][2] = acc[j][1].x;
+			out[j][3] = acc[j][1].y;
+		}
+	}
+#pragma unroll
+	for (int j = 0; j < 4; ++j, d += it.dst_stride) {
+		if (r0 + j >= it.dst_h)
+			break;
+		if constexpr (INT) {
+			uint32_t u[4];
+#pragma unroll
+			for (int e = 0; e < 4; ++e)
+				u[e] = static_cast<uint32_t>(__float_as_int(out[j][e]));
+			if (wide) {
+				*reinterpret_cast<uint2 *>(d) = make_uint2(u[0] | (u[1] << 16), u[2] | (u[3] << 16));
+			} else {
+#pragma unroll
+				for (int e = 0; e < 4; ++e)
+					if (4 * q + e < it.cols_valid)
+						reinterpret_cast<uint16_t *>(d)[e] = static_cast<uint16_t>(u[e]);
 			}
+		} else if (wide) {
+			*reinterpret_cast<float4 *>(d) = make_float4(out[j][0], out[j][1], out[j][2], out[j][3]);
+		} else {
 #pragma unroll
-			for (int j = 0; j < kGroup; ++j) {
-				if (!FINAL) {
-					float4 v;
-					if (U16) {
-						v.x = u16_round(acc[j][0], it.magic, it.pixel_max) - it.magic;
-						v.y = u16_round(acc[j][1], it.magic, it.pixel_max) - it.magic;
-						v.z = u16_round(acc[j][2], it.magic, it.pixel_max) - it.magic;
-						v.w = u16_round(acc[j][3], it.magic, it.pixel_max) - it.magic;
-					} else {
-						v = make_float4(acc[j][0], acc[j][1], acc[j][2], acc[j][3]);
-					}
-					*reinterpret_cast<float4 *>(I + (gi * kGroup + j) * i_pitch + 4 * q) = v;
-				} else {
-					const int r = g * kGroup + j;
-					if (r >= it.dst_h)
-						continue;
-					const int x0 = 4 * q;
-					char *drow = it.dst + static_cast<ptrdiff_t>(r) * it.dst_stride;
-					if (U16) {
-						uint32_t u[4];
-#pragma unroll
-						for (int e = 0; e < 4; ++e)
-							u[e] = __float_as_uint(u16_round(acc[j][e], it.magic, it.pixel_max)) & 0xFFFFu;
-						uint16_t *d = reinterpret_cast<uint16_t *>(drow) + it.c0 + x0;
-						if (it.vec_ok && x0 + 3 < it.cols_valid) {
-							*reinterpret_cast<uint2 *>(d) = make_uint2(u[0] | (u[1] << 16), u[2] | (u[3] << 16));
-						} else {
-#pragma unroll
-							for (int e = 0; e < 4; ++e)
-								if (x0 + e < it.cols_valid)
-									d[e] = static_cast<uint16_t>(u[e]);
-						}
-					} else {
-						float *d = reinterpret_cast<float *>(drow) + it.c0 + x0;
-						if (it.vec_ok && x0 + 3 < it.cols_valid) {
-							*reinterpret_cast<float4 *>(d) = make_float4(acc[j][0], acc[j][1], acc[j][2], acc[j][3]);
-						} else {
-#pragma unroll
-							for (int e = 0; e < 4; ++e)
-								if (x0 + e < it.cols_valid)
-									d[e] = acc[j][e];
-						}
-					}
-				}
-			}
+			for (int e = 0; e < 4; ++e)
+				if (4 * q + e < it.cols_valid)
+					reinterpret_cast<float *>(d)[e] = out[j][e];
 		}
 	}
 }
 
-// Source-line range a step needs: groups [g0, g1) read lines
-// [base[g0], base[g1 - 1] + VS) (bases are non-decreasing).
-template <int VS>
-__device__ __forceinline__ int step_end(const Item &it, const char *smem, const SmemLayout &L, int g1)
-{
-	return reinterpret_cast<const int *>(smem + L.vbase_off)[g1 - 1 - it.g_begin] + VS;
-}
-
-template <int VS, int kGroup>
-__device__ __forceinline__ void load_coef(const Item &it, int g0, int g1, char *dst)
-{
-	// kGroup floats per line: (g1 - g0) * VS * kGroup * 4 bytes, a multiple of 16 (VS even)
-	const char *src = it.v_dense + static_cast<size_t>(g0) * VS * kGroup * 4;
-	for (int i = threadIdx.x; i < (g1 - g0) * VS * kGroup / 4; i += kThreads)
-		cp_async16(dst + i * 16, src + i * 16, 16);
-}
-
-template <bool H_FIRST, bool U16, int HW, int VS, bool INT = false>
-__global__ void __launch_bounds__(kThreads, H_FIRST ? 4 : 5)
+template <bool H_FIRST, bool INT, int HW, int VS>
+__global__ void __launch_bounds__(kThreads, HW <= 8 ? 5 : 4)
 fused_kernel(const FusedJob *__restrict__ jobs, int num_jobs, int total_items, const __grid_constant__ FusedJob single,
              const __grid_constant__ SmemLayout L, const __grid_constant__ WorkChunks C)
 {
-	constexpr int kGroup = group_rows(H_FIRST);
+	constexpr int E = INT ? 2 : 4;
+	constexpr int kStepRows = stream_step_rows(H_FIRST);
+	constexpr int kRecordBytes = 4 * stream_record_bytes(H_FIRST, VS);  // a step's four groups
 	extern __shared__ float4 smem4[];
 	char *smem = reinterpret_cast<char *>(smem4);
-	float *ring = reinterpret_cast<float *>(smem + L.ring_off);
-	char *stage = smem + L.stage_off;
-	float *in = reinterpret_cast<float *>(smem + L.in_off);
-	float *I = reinterpret_cast<float *>(smem + L.i_off);
-	const int rmask = L.ring_rows - 1;
-	const int smask = L.stage_rows - 1;
-	const int imask = L.in_rows - 1;
-
-	// Lines a step reads but does not load keep finite values: clear the rings once.
-	for (int i = threadIdx.x; i < L.vcoef_off / 16; i += kThreads)
-		smem4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-	__syncthreads();
+	char *in = smem + L.in_off;      // source lines
+	char *mid = smem + L.ring_off;   // V first: I; H first: the intermediate ring
+	char *records = smem + L.vcoef_off;
+	const uint32_t in_a = shared_addr(in), mid_a = shared_addr(mid), records_a = shared_addr(records);
 
 	// the launch's units in job / strip / step order: guided chunks
 	// (C.sched), or this CTA's equal share
@@ -553,74 +619,85 @@ fused_kernel(const FusedJob *__restrict__ jobs, int num_jobs, int total_items, c
 		} else if (!first) {
 			break;
 		}
-		const int t_end = c_end;
-		for (int t = c_begin; t < t_end;) {
-			const FusedJob *Jp = jobs ? &jobs[find_job(jobs, num_jobs, t)] : &single;
-			const Item it = make_item<HW>(*Jp, t, t_end, smem, L);
-			t += it.units;
-			__syncthreads();  // group bases visible
+		for (int t = c_begin; t < c_end;) {
+			const FusedJob &J = jobs ? jobs[find_job(jobs, num_jobs, t)] : single;
+			const Item it = make_item(J, t, c_end);
+			t += it.steps;
 
-			const int nsteps = (it.g_end - it.g_begin + it.step_groups - 1) / it.step_groups;
-			// step k covers groups [gk, gk1); its new source lines are [lo_k, hi_k)
-			int hi_prev = reinterpret_cast<const int *>(smem + L.vbase_off)[0];
-			auto step_groups_of = [&](int k, int *g0, int *g1) {
-				*g0 = it.g_begin + k * it.step_groups;
-				*g1 = min(it.g_end, *g0 + it.step_groups);
+			// lines and records of a step, one cp.async group; `next`, `slot`:
+			// the first line not yet in the ring and its slot
+			int next, slot;
+			auto load_step = [&](int k) {
+				const int hi = __ldg(it.ranges + it.step0 + k).y;
+				if (hi > next) {
+					load_lines<E>(it, next, hi, in, it.in_rows, slot);
+					slot += hi - next;
+					while (slot >= it.in_rows)
+						slot -= it.in_rows;
+					next = hi;
+				}
+				load_records(it.records + static_cast<size_t>(it.step0 + k) * kRecordBytes,
+				             records + (k & 1) * kRecordBytes, kRecordBytes);
+				cp_async_commit();
 			};
-			// prologue: step 0's lines and taps
-			{
-				int g0, g1;
-				step_groups_of(0, &g0, &g1);
-				const int hi = step_end<VS>(it, smem, L, g1);
-				if (U16)
-					load_lines<true>(it, hi_prev, hi, stage, smask, L.pitch);
-				else
-					load_lines<false>(it, hi_prev, hi, reinterpret_cast<char *>(H_FIRST ? in : ring),
-					                  H_FIRST ? imask : rmask, L.pitch);
-				load_coef<VS, kGroup>(it, g0, g1, smem + L.vcoef_off);
-				cp_async_commit();
+			next = __ldg(it.ranges + it.step0).x;
+			slot = next % it.in_rows;
+			int h_line = next, h_in = slot, h_mid = H_FIRST ? next % it.ring_rows : 0;
+			load_step(0);
+
+			// this thread's output column: taps, and where its inputs are
+			const int c = min(static_cast<int>(threadIdx.x), it.cols_valid - 1);
+			const int left = __ldg(J.h_left + it.c0 + c) - it.xlo;
+			float taps[HW];
+			const float *tp = J.h_taps + static_cast<size_t>(it.c0 + c) * HW;
+#pragma unroll
+			for (int k = 0; k < HW; ++k)
+				taps[k] = __ldg(tp + k);
+			// V first: this thread's part of the vertical pass, its inputs in I
+			uint32_t at[H_FIRST ? 1 : HW];
+			int q = 0, half = 0;
+			if constexpr (!H_FIRST) {
+				const int quads = it.pxa / 4;
+				q = static_cast<int>(threadIdx.x) % quads;
+				half = static_cast<int>(threadIdx.x) / quads;
+#pragma unroll
+				for (int k = 0; k < HW; ++k)
+					at[k] = mid_a + (((left + k) & 3) * kPlane + ((left + k) >> 2)) * 16;
 			}
-			__syncthreads();  // lines stored by plain loads (unaligned u16) are visible to every converter
-			int lo_cur = hi_prev;
-			int hi_cur = step_end<VS>(it, smem, L, min(it.g_end, it.g_begin + it.step_groups));
 
-			for (int k = 0; k < nsteps; ++k) {
-				int g0, g1;
-				step_groups_of(k, &g0, &g1);
-				// prefetch step k+1
-				int hi_next = hi_cur;
-				if (k + 1 < nsteps) {
-					int n0, n1;
-					step_groups_of(k + 1, &n0, &n1);
-					hi_next = step_end<VS>(it, smem, L, n1);
-					if (U16)
-						load_lines<true>(it, hi_cur, hi_next, stage, smask, L.pitch);
-					else
-						load_lines<false>(it, hi_cur, hi_next, reinterpret_cast<char *>(H_FIRST ? in : ring),
-						                  H_FIRST ? imask : rmask, L.pitch);
-					load_coef<VS, kGroup>(it, n0, n1, smem + L.vcoef_off + ((k + 1) & 1) * (L.vbase_off - L.vcoef_off) / 2);
-				}
-				cp_async_commit();
-				cp_async_wait<1>();
-				if (U16)
-					convert_lines<INT>(it, lo_cur, hi_cur, stage, smask, H_FIRST ? in : ring, H_FIRST ? imask : rmask, L.pitch);
-				__syncthreads();
-
-				const float *coef = reinterpret_cast<const float *>(smem + L.vcoef_off + (k & 1) * (L.vbase_off - L.vcoef_off) / 2);
-				if (H_FIRST) {
-					// new source lines -> intermediate ring
-					h_pass<U16, false, HW, INT>(it, smem, L, in, imask, lo_cur, hi_cur, ring, rmask, 0);
-					__syncthreads();
-					v_pass<U16, true, VS, kGroup, INT>(it, smem, L, ring, rmask, kStripW, g0, g1, coef, kStripW / 4, nullptr, 0);
+			for (int k = 0; k < it.steps; ++k) {
+				// early: the next step's lines go into slots that no line of
+				// this one's windows holds; late: only after its vertical
+				// pass (H first: horizontal pass)
+				const bool more = k + 1 < it.steps;
+				if (more && !it.late) {
+					load_step(k + 1);
+					cp_async_wait<1>();
 				} else {
-					v_pass<U16, false, VS, kGroup, INT>(it, smem, L, ring, rmask, L.pitch, g0, g1, coef, it.pxa / 4, I, L.pitch);
-					__syncthreads();
-					h_pass<U16, true, HW, INT>(it, smem, L, I, 0x7fffffff, 0, (g1 - g0) * kGroup, nullptr, 0, g0 * kGroup);
+					cp_async_wait<0>();
 				}
-				lo_cur = hi_cur;
-				hi_cur = hi_next;
+				__syncthreads();
+				const int row0 = (it.step0 + k) * kStepRows;
+				const uint32_t rec = records_a + (k & 1) * kRecordBytes;
+				if constexpr (H_FIRST) {
+					const int hi = __ldg(it.ranges + it.step0 + k).y;
+					if (hi > h_line) {
+						hfirst_h<INT, HW>(it, in_a, taps, left, h_line, hi, h_in, mid, h_mid);
+						h_in = (h_in + (hi - h_line)) % it.in_rows;
+						h_mid = (h_mid + (hi - h_line)) % it.ring_rows;
+						h_line = hi;
+					}
+				} else {
+					vfirst_v<INT, VS>(it, in_a, rec, mid_a, q, half);
+				}
+				__syncthreads();
+				if (more && it.late)
+					load_step(k + 1);
+				if constexpr (H_FIRST)
+					hfirst_v<INT, VS>(it, mid_a, rec, row0);
+				else
+					vfirst_h<INT, HW>(it, taps, at, row0);
 			}
-			cp_async_wait<0>();
 			__syncthreads();  // the next item reuses every buffer
 		}
 	}
