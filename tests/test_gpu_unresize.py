@@ -42,3 +42,28 @@ def test_unresize_full_hd(cuda, oracle):
     src = make_src(np.random.default_rng(99), 1080, 1920)
     np.testing.assert_array_equal(run(src, 1280, 720).view(np.uint32),
                                   oracle.unresize_plane(src, 1280, 720).view(np.uint32))
+
+
+@pytest.mark.parametrize("uw,uh,ow,oh,sw,sh", [
+    (31, 45, 30, 31, 0.0, 0.0), (64, 64, 63, 33, 0.0, 0.0), (200, 130, 150, 65, 0.3, -0.2),
+    (1733, 97, 1301, 70, 0.0, 0.0), (97, 1733, 70, 1301, 0.0, 0.0), (600, 400, 600, 400, 0.25, -0.25),
+    (600, 400, 600, 400, 0.5, 0.5), (1, 9, 1, 5, 0.0, 0.0), (40000, 6, 30000, 4, 0.0, 0.0)])
+@pytest.mark.parametrize("content", ["noise", "black", "special"])
+def test_unresize_chunks(cuda, oracle, uw, uh, ow, oh, sw, sh, content):
+    """Lines cut into chunks that run side by side: around the chunk's length
+    and the block's lines and columns, contexts whose recurrences do not die
+    out (half-sample shifts), lines beyond shared memory; noise, black borders
+    (where the recurrence dies out through the denormals, sample after
+    sample), and NaN, infinities and huge values that reach the whole line."""
+    rng = np.random.default_rng(uw * 131 + oh)
+    src = rng.random((uh, uw), dtype=np.float32) - 0.25
+    if content == "black":
+        src[:, uw // 4:uw * 7 // 8] = 0.0
+        src[uh // 3:uh * 5 // 6, :] = 0.0
+    elif content == "special":
+        for v in (np.nan, np.inf, -np.inf, 3e38, -0.0):
+            src[rng.integers(0, uh), rng.integers(0, uw)] = v
+    got, want = run(src, ow, oh, sw, sh), oracle.unresize_plane(src, ow, oh, sw, sh)
+    nan = np.isnan(want)
+    np.testing.assert_array_equal(np.isnan(got), nan)
+    np.testing.assert_array_equal(got[~nan].view(np.uint32), want[~nan].view(np.uint32))

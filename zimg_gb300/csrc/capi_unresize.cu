@@ -39,6 +39,7 @@ struct DeviceUnresize {
 		t.up = ctx.up;
 		t.orig = ctx.orig;
 		t.row_size = ctx.row_size;
+		t.reach = ctx.reach;
 	}
 };
 

@@ -17,7 +17,12 @@ struct UnresizeContext {
 	std::vector<float> coef;        // [orig][row_size]: row r of A', from offset[r]
 	std::vector<unsigned> offset;   // [orig]
 	std::vector<float> lu_c, lu_l, lu_u;  // tridiagonal LU of A'A (lu_l inverted)
+	// steps after which whatever the substitutions started from has shrunk by
+	// 2^60, forward and backward (0: not within kMaxReach steps)
+	unsigned reach = 0;
 };
+
+constexpr unsigned kMaxReach = 96;
 
 // Returns false when orig > up (zimg: "unresize can not upscale").
 bool build_unresize_context(unsigned orig, unsigned up, double shift, UnresizeContext *out);
@@ -31,6 +36,7 @@ struct UnresizeTables {
 	const unsigned *offset;
 	const float *lu_c, *lu_l, *lu_u;
 	unsigned up, orig, row_size;
+	unsigned reach;
 };
 
 // One pass over a FLOAT plane: horizontal (lines of `up` -> `orig` samples,

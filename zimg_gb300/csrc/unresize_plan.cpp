@@ -129,6 +129,21 @@ bool build_unresize_context(unsigned orig, unsigned up, double shift, UnresizeCo
 		x.lu_l[r] = static_cast<float>(1.0 / (l[r] + eps));
 		x.lu_u[r] = static_cast<float>(u[r]);
 	}
+	// the steps' factors: z_i holds -c_i l_i z_{i-1}, w_i holds -u_i w_{i+1}
+	x.reach = 0;
+	for (unsigned k = 1; k <= kMaxReach && !x.reach; ++k) {
+		bool within = true;
+		for (unsigned r = k; r <= N && within; ++r) {
+			double f = 1.0, b = 1.0;
+			for (unsigned i = r - k; i < r; ++i) {
+				f *= std::abs(static_cast<double>(x.lu_c[i]) * x.lu_l[i]);
+				b *= std::abs(static_cast<double>(x.lu_u[i]));
+			}
+			within = f <= 0x1p-60 && b <= 0x1p-60;
+		}
+		if (within)
+			x.reach = k;
+	}
 	return true;
 }
 
