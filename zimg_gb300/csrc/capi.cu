@@ -479,44 +479,88 @@ zg_error_code zg_resize_process(const zg_resize *r, const void *src, ptrdiff_t s
                                 ptrdiff_t dst_stride, void *tmp, zg_stream stream)
 {
 	return guarded([&] {
-		if (!r)
-			throw Error(kErrIllegalArgument, "null pointer");
-		check_device(r->device);
-		cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-		const zg_resize_params &q = r->params;
-		check_plane(src, src_stride, q.src_width, r->sample, "src");
-		check_plane(dst, dst_stride, q.dst_width, r->sample, "dst");
-		if (r->num_passes == 0) {
-			copy_plane(dst, dst_stride, src, src_stride, static_cast<size_t>(q.dst_width) * bytes_of(r->sample),
-			           q.dst_height, st);
-			return;
-		}
-		if (r->num_passes == 1) {
-			run_pass(*r->pass[0], src, src_stride, dst, dst_stride, st);
-			return;
-		}
-		if (r->fused) {
-			FusedJob j = r->fplan.job;
-			fused_set_io(j, src, src_stride, dst, dst_stride);
-			j.item_begin = 0;
-			CUtensorMap map;
-			if (r->tma && chain_tma_source_map(&map, j, r->tlayout)) {
-				cuda_check(launch_chain_tma(r->fplan.variant, nullptr, 1, fused_items(j), nullptr, r->tlayout, r->tgrid, j, &map,
-				                            st),
-				           "fused resize launch");
-				return;
-			}
-			cuda_check(launch_fused(r->fplan.variant, nullptr, 1, fused_items(j), r->flayout, r->fgrid,
-			                        j, st), "fused resize launch");
-			return;
-		}
-		if (!tmp)
-			throw Error(kErrIllegalArgument, "tmp buffer required (zg_resize_get_tmp_size)");
-		if (reinterpret_cast<uintptr_t>(tmp) % 256)
-			throw Error(kErrIllegalArgument, "tmp buffer must be 256-byte aligned");
-		run_pass(*r->pass[0], src, src_stride, tmp, r->tmp_stride, st);
-		run_pass(*r->pass[1], tmp, r->tmp_stride, dst, dst_stride, st);
+		const ResizeIo io{ r, src, src_stride, dst, dst_stride, tmp };
+		resize_planes(&io, 1, reinterpret_cast<cudaStream_t>(stream));
 	});
 }
 
 } // extern "C"
+
+namespace zg {
+
+void resize_planes(const ResizeIo *io, int n, cudaStream_t st)
+{
+	bool done[kFewJobs] = {};
+	if (n > kFewJobs)
+		throw Error(kErrLogic, "too many planes");
+	for (int k = 0; k < n; ++k) {
+		const zg_resize *r = io[k].r;
+		if (!r)
+			throw Error(kErrIllegalArgument, "null pointer");
+		check_device(r->device);
+		check_plane(io[k].src, io[k].src_stride, r->params.src_width, r->sample, "src");
+		check_plane(io[k].dst, io[k].dst_stride, r->params.dst_width, r->sample, "dst");
+		if (r->tmp_size && !io[k].tmp)
+			throw Error(kErrIllegalArgument, "tmp buffer required (zg_resize_get_tmp_size)");
+		if (r->tmp_size && reinterpret_cast<uintptr_t>(io[k].tmp) % 256)
+			throw Error(kErrIllegalArgument, "tmp buffer must be 256-byte aligned");
+	}
+	for (int a = 0; a < n; ++a) {
+		if (done[a])
+			continue;
+		const ResizeIo &x = io[a];
+		const zg_resize *r = x.r;
+		if (r->num_passes == 0) {
+			copy_plane(x.dst, x.dst_stride, x.src, x.src_stride,
+			           static_cast<size_t>(r->params.dst_width) * bytes_of(r->sample), r->params.dst_height, st);
+			continue;
+		}
+		if (r->num_passes == 1) {
+			run_pass(*r->pass[0], x.src, x.src_stride, x.dst, x.dst_stride, st);
+			continue;
+		}
+		if (!r->fused) {
+			run_pass(*r->pass[0], x.src, x.src_stride, x.tmp, r->tmp_stride, st);
+			run_pass(*r->pass[1], x.tmp, r->tmp_stride, x.dst, x.dst_stride, st);
+			continue;
+		}
+		// the planes of this plan's variant that follow ride in the same
+		// launch (the tensor-core kernels of variants 100-199 take one)
+		FewJobs few{};
+		const FusedPlan *plans[kFewJobs];
+		int count = 0, items = 0, grid = r->tma ? r->tgrid : r->fgrid;
+		for (int b = a; b < n; ++b) {
+			const zg_resize *q = io[b].r;
+			if (done[b] || !q->fused || q->fplan.variant != r->fplan.variant || q->tma != r->tma ||
+			    (b > a && r->fplan.mma && !r->fplan.chain))
+				continue;
+			done[b] = true;
+			FusedJob &j = few.job[count];
+			j = q->fplan.job;
+			fused_set_io(j, io[b].src, io[b].src_stride, io[b].dst, io[b].dst_stride);
+			j.item_begin = items;
+			items += fused_items(j);
+			grid = std::min(grid, r->tma ? q->tgrid : q->fgrid);
+			plans[count++] = &q->fplan;
+		}
+		if (r->tma) {
+			SmemLayout L = r->tlayout;
+			FewMaps maps;
+			bool mapped = count == 1 || chain_tma_layout(plans, count, &L);
+			for (int k = 0; k < count && mapped; ++k)
+				mapped = chain_tma_source_map(&maps.map[k], few.job[k], L);
+			if (mapped) {
+				cuda_check(launch_chain_tma(r->fplan.variant, nullptr, count, items, nullptr, L, grid, few, &maps, st),
+				           "fused resize launch");
+				continue;
+			}
+		}
+		if (r->tma)
+			grid = r->fgrid;
+		cuda_check(launch_fused(r->fplan.variant, nullptr, count, items, count == 1 ? r->flayout : fused_layout(plans, count),
+		                        grid, few, st),
+		           "fused resize launch");
+	}
+}
+
+} // namespace zg

@@ -148,7 +148,7 @@ void batch_launch(const zg_batch *b, void *tmp, cudaStream_t st)
 			c.sched = static_cast<unsigned *>(b->sched_dev.get()) + g.sched;
 		}
 		work.push_back([&g, table, ranges, c](cudaStream_t s) {
-			FusedJob unused{};
+			FewJobs unused{};
 			if (g.tma_now)
 				cuda_check(launch_chain_tma(g.variant, table + g.first, g.count, g.tiles, ranges, g.tlayout, g.tgrid,
 				                            unused, nullptr, s),

@@ -179,3 +179,21 @@ struct zg_resize {
 	zg::SmemLayout tlayout{};
 	int tgrid = 0;
 };
+
+namespace zg {
+
+// One plane of a conversion.
+struct ResizeIo {
+	const ::zg_resize *r;
+	const void *src;
+	ptrdiff_t src_stride;
+	void *dst;
+	ptrdiff_t dst_stride;
+	void *tmp;
+};
+
+// Independent planes (each with its own tmp), in as few launches as their
+// plans allow. Throws on bad arguments and failed launches.
+void resize_planes(const ResizeIo *io, int n, cudaStream_t stream);
+
+} // namespace zg

@@ -186,61 +186,91 @@ zg_error_code zg_depth_process(const zg_depth *d, const void *src, ptrdiff_t src
                                ptrdiff_t dst_stride, zg_stream stream)
 {
 	return guarded([&] {
+		const DepthIo io{ d, src, src_stride, dst, dst_stride };
+		depth_planes(&io, 1, reinterpret_cast<cudaStream_t>(stream));
+	});
+}
+
+} // extern "C"
+
+namespace zg {
+
+void depth_planes(const DepthIo *io, int n, cudaStream_t st)
+{
+	bool done[kDepthMaxPlanes] = {};
+	if (n > kDepthMaxPlanes)
+		throw Error(kErrLogic, "too many planes");
+	for (int k = 0; k < n; ++k) {
+		const zg_depth *d = io[k].d;
 		if (!d)
 			throw Error(kErrIllegalArgument, "null pointer");
 		if (current_device() != d->device)
 			throw Error(kErrLogic, "object used on a different device than the one it was created on");
-		const zg_depth_params &q = d->params;
-		const int ci = type_code(q.pixel_in.type), co = type_code(q.pixel_out.type);
-		const unsigned bi = type_bytes(ci), bo = type_bytes(co);
-		auto check = [](const void *p, ptrdiff_t stride, unsigned w, unsigned b, const char *what) {
+		auto check = [&](const void *p, ptrdiff_t stride, int type, const char *what) {
+			const unsigned b = type_bytes(type);
 			if (!p)
 				throw Error(kErrIllegalArgument, std::string(what) + " is null");
-			if (abs_stride(stride) < static_cast<ptrdiff_t>(w) * static_cast<ptrdiff_t>(b))
+			if (abs_stride(stride) < static_cast<ptrdiff_t>(d->params.width) * static_cast<ptrdiff_t>(b))
 				throw Error(kErrIllegalArgument, std::string(what) + " stride smaller than a line");
 			if (reinterpret_cast<uintptr_t>(p) % b || stride % b)
 				throw Error(kErrIllegalArgument, std::string(what) + " not aligned to the sample size");
 		};
-		check(src, src_stride, q.width, bi, "src");
-		check(dst, dst_stride, q.width, bo, "dst");
-		cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+		check(io[k].src, io[k].src_stride, type_code(d->params.pixel_in.type), "src");
+		check(io[k].dst, io[k].dst_stride, type_code(d->params.pixel_out.type), "dst");
+	}
+	for (int a = 0; a < n; ++a) {
+		if (done[a])
+			continue;
+		const zg_depth *d = io[a].d;
+		const zg_depth_params &q = d->params;
+		const int ci = type_code(q.pixel_in.type), co = type_code(q.pixel_out.type);
 		if (d->mode == 0) {
-			copy_plane(dst, dst_stride, src, src_stride, static_cast<size_t>(q.width) * bo, q.height, st);
-			return;
+			copy_plane(io[a].dst, io[a].dst_stride, io[a].src, io[a].src_stride,
+			           static_cast<size_t>(q.width) * type_bytes(co), q.height, st);
+			continue;
 		}
 		if (d->mode == 3 && q.dither_type == ZG_DITHER_ERROR_DIFFUSION) {
 			EdLaunch E{};
 			E.planes[0] = d->ed;
-			E.planes[0].src = src;
-			E.planes[0].src_stride = src_stride;
-			E.planes[0].dst = dst;
-			E.planes[0].dst_stride = dst_stride;
+			E.planes[0].src = io[a].src;
+			E.planes[0].src_stride = io[a].src_stride;
+			E.planes[0].dst = io[a].dst;
+			E.planes[0].dst_stride = io[a].dst_stride;
 			E.num_planes = 1;
 			E.in_type = ci;
 			E.out_type = co;
 			E.warps = d->ed_warps;
 			E.ring = d->ed_ring;
 			cuda_check(launch_error_diffusion(E, st), "error diffusion launch");
-			return;
+			continue;
 		}
-		DepthLaunch L{};
-		L.src = src;
-		L.src_stride = src_stride;
-		L.dst = dst;
-		L.dst_stride = dst_stride;
-		L.width = static_cast<int>(q.width);
-		L.height = static_cast<int>(q.height);
-		L.scale = d->scale;
-		L.offset = d->offset;
-		L.vmax = d->vmax;
-		L.shift = d->shift;
-		L.seq = q.plane;
-		L.dither = q.dither_type == ZG_DITHER_ORDERED ? 1 : (q.dither_type == ZG_DITHER_RANDOM ? 2 : 0);
-		// 8 samples per vector: 8-byte loads of BYTE, 16-byte loads of WORD, HALF and FLOAT
-		L.vec_in = aligned(src, src_stride, bi == 1 ? 8 : 16);
-		L.vec_out = aligned(dst, dst_stride, bo == 1 ? 8 : 16);
-		cuda_check(launch_depth(ci, co, d->mode, L, st), "depth conversion launch");
-	});
+		DepthPlanes P{};
+		for (int b = a; b < n; ++b) {
+			const zg_depth *e = io[b].d;
+			const zg_depth_params &r = e->params;
+			if (done[b] || e->mode != d->mode || type_code(r.pixel_in.type) != ci || type_code(r.pixel_out.type) != co ||
+			    (d->mode == 3 && r.dither_type != q.dither_type))
+				continue;
+			done[b] = true;
+			DepthLaunch &L = P.plane[P.num++];
+			L.src = io[b].src;
+			L.src_stride = io[b].src_stride;
+			L.dst = io[b].dst;
+			L.dst_stride = io[b].dst_stride;
+			L.width = static_cast<int>(r.width);
+			L.height = static_cast<int>(r.height);
+			L.scale = e->scale;
+			L.offset = e->offset;
+			L.vmax = e->vmax;
+			L.shift = e->shift;
+			L.seq = r.plane;
+			L.dither = r.dither_type == ZG_DITHER_ORDERED ? 1 : (r.dither_type == ZG_DITHER_RANDOM ? 2 : 0);
+			// 8 samples per vector: 8-byte loads of BYTE, 16-byte loads of WORD, HALF and FLOAT
+			L.vec_in = aligned(L.src, L.src_stride, type_bytes(ci) == 1 ? 8 : 16);
+			L.vec_out = aligned(L.dst, L.dst_stride, type_bytes(co) == 1 ? 8 : 16);
+		}
+		cuda_check(launch_depth(ci, co, d->mode, P, st), "depth conversion launch");
+	}
 }
 
-} // extern "C"
+} // namespace zg

@@ -417,32 +417,66 @@ Chain make_chain(const PlaneGeom &sp, const PlaneGeom &dp, const PixFmt &fs, con
 		off += c.mid_pitch * dp.height;
 	}
 	c.off_rtmp = off;
-	c.scratch = off + rtmp;
+	c.scratch = (off + rtmp + 255) & ~static_cast<size_t>(255);
 	return c;
 }
 
-void run_chain(const Chain &c, const void *src, ptrdiff_t ss, void *dst, ptrdiff_t ds, char *scratch, zg_stream st)
+// A frame's planes go through the steps of their conversions side by side:
+// each step is one launch, or a few, for all of them (depth_planes,
+// resize_planes), and so a plane's intermediates have scratch of their own.
+struct Stage {
+	DepthIo depth[4];
+	ResizeIo resize[4];
+	int depths = 0, resizes = 0;
+
+	void add(const zg_depth *d, const void *src, ptrdiff_t ss, void *dst, ptrdiff_t ds)
+	{
+		depth[depths++] = DepthIo{ d, src, ss, dst, ds };
+	}
+	void add(const zg_resize *r, const void *src, ptrdiff_t ss, void *dst, ptrdiff_t ds, void *tmp)
+	{
+		resize[resizes++] = ResizeIo{ r, src, ss, dst, ds, tmp };
+	}
+	void run(cudaStream_t st)
+	{
+		depth_planes(depth, depths, st);
+		resize_planes(resize, resizes, st);
+		depths = resizes = 0;
+	}
+};
+
+// The chains of up to four planes: chain k from src[k] to dst[k], its
+// intermediates at scratch + off[k].
+void run_chains(const Chain *c, int n, const void *const *src, const ptrdiff_t *ss, void *const *dst,
+                const ptrdiff_t *ds, char *scratch, const size_t *off, cudaStream_t st)
 {
-	if (c.kind == 0) {
-		copy_plane(dst, ds, src, ss, static_cast<size_t>(c.dw) * c.out_bytes, c.dh, reinterpret_cast<cudaStream_t>(st));
-		return;
+	Stage before, resize, after;
+	for (int k = 0; k < n; ++k) {
+		if (c[k].kind == 0) {
+			copy_plane(dst[k], ds[k], src[k], ss[k], static_cast<size_t>(c[k].dw) * c[k].out_bytes, c[k].dh, st);
+			continue;
+		}
+		if (c[k].kind == 1) {
+			before.add(c[k].only, src[k], ss[k], dst[k], ds[k]);
+			continue;
+		}
+		char *t = scratch + off[k];
+		const void *rs = src[k];
+		ptrdiff_t rss = ss[k];
+		if (c[k].pre) {
+			before.add(c[k].pre, rs, rss, t, static_cast<ptrdiff_t>(c[k].pre_pitch));
+			rs = t;
+			rss = static_cast<ptrdiff_t>(c[k].pre_pitch);
+		}
+		void *rd = c[k].post ? static_cast<void *>(t + c[k].off_mid) : dst[k];
+		const ptrdiff_t rds = c[k].post ? static_cast<ptrdiff_t>(c[k].mid_pitch) : ds[k];
+		resize.add(c[k].resize, rs, rss, rd, rds, t + c[k].off_rtmp);
+		if (c[k].post)
+			after.add(c[k].post, rd, rds, dst[k], ds[k]);
 	}
-	if (c.kind == 1) {
-		run_depth(c.only, src, ss, dst, ds, st);
-		return;
-	}
-	const void *rs = src;
-	ptrdiff_t rss = ss;
-	if (c.pre) {
-		run_depth(c.pre, src, ss, scratch, static_cast<ptrdiff_t>(c.pre_pitch), st);
-		rs = scratch;
-		rss = static_cast<ptrdiff_t>(c.pre_pitch);
-	}
-	void *rd = c.post ? static_cast<void *>(scratch + c.off_mid) : dst;
-	const ptrdiff_t rds = c.post ? static_cast<ptrdiff_t>(c.mid_pitch) : ds;
-	run_resize(c.resize, rs, rss, rd, rds, scratch + c.off_rtmp, st);
-	if (c.post)
-		run_depth(c.post, rd, rds, dst, ds, st);
+	before.run(st);
+	resize.run(st);
+	after.run(st);
 }
 
 // Error-diffusion conversions of a frame's planes, side by side: one launch
@@ -536,15 +570,13 @@ struct zg_graph {
 		zg_unresize *unresize = nullptr;  // instead of resize when the filter is ZG_RESIZE_UNRESIZE
 		// depth conversions around resize (graphbuilder.cpp:943-950): into
 		// the resize format before, to the output format after; their
-		// planes live in tmp (pre at 0, mid next, resize scratch last)
+		// planes live in tmp: pre, mid, resize scratch, the plane's own
 		zg_depth *pre = nullptr, *post = nullptr, *only = nullptr;
-		size_t pre_pitch = 0, mid_pitch = 0, off_mid = 0, off_tmp = 0;
+		size_t pre_pitch = 0, mid_pitch = 0, off_pre = 0, off_mid = 0, off_tmp = 0;
 		// the last step diffuses errors: it runs after every plane's other
-		// steps, in one launch with the frame's other such planes (a resize
-		// before it writes into a region of tmp of the plane's own)
+		// steps, in one launch with the frame's other such planes
 		bool ed_last = false;
-		size_t off_mid_own = 0;
-		size_t tmp = 0;
+		size_t tmp = 0;  // bytes of tmp of the plane's own
 		// ring-buffer (line-masked) planes: the plane's full size, its
 		// vertical subsampling shift, and whole-plane staging copies in tmp
 		unsigned src_w = 0, src_h = 0, src_ssh = 0, dst_ssh = 0;
@@ -576,13 +608,14 @@ struct zg_graph {
 	// the colour planes to FLOAT 4:4:4 at the work geometry (each dimension
 	// the smaller side's), GREY duplicated into three planes, the colorspace
 	// operations in place, then each output plane from the work planes to
-	// its geometry and format. Work planes and the chains' shared scratch in
-	// tmp from off_work.
+	// its geometry and format. Work planes, then the chains' scratch (the input
+	// and the output chains share theirs), in tmp from off_work.
 	struct Color {
 		bool on = false;
 		int n_in = 0, n_out = 0;  // colour planes read / written
 		unsigned ww = 0, wh = 0;
 		size_t w_pitch = 0, off_work = 0, off_scratch = 0;
+		size_t in_off[3] = {}, out_off[3] = {};  // each chain's intermediates, from off_scratch
 		Chain in[3], out[3];
 		csp::Plan plan;
 	} color;
@@ -591,6 +624,7 @@ struct zg_graph {
 	// copy of the luma output
 	int out_fill[4] = {};
 	uint32_t fill_value = 0;
+	bool unresizes = false;  // every plane of mode 2 is unresized
 	size_t tmp_size = 0;
 	// lines and widths the callbacks are called with (the luma plane's), and
 	// the vertical subsampling step of the source and destination formats
@@ -869,6 +903,7 @@ zg_graph *zg_graph_build(const zg_image_format *src_format, const zg_image_forma
 			zg_error_code rc;
 			if (unresize) {
 				const zg_unresize_params up{ sp.width, sp.height, dp.width, dp.height, rp.shift_w, rp.shift_h };
+				g->unresizes = true;
 				rc = zg_unresize_create(&up, &gpl.unresize);
 				if (rc == ZG_ERROR_SUCCESS)
 					zg_unresize_get_tmp_size(gpl.unresize, &rtmp);
@@ -882,10 +917,11 @@ zg_graph *zg_graph_build(const zg_image_format *src_format, const zg_image_forma
 				zg_get_last_error(msg, sizeof(msg));
 				throw Error(rc, msg);
 			}
-			size_t off = 0;
+			size_t off = g->tmp_size;
 			if (!fmt_equal(fs, fr)) {
 				gpl.pre = make_depth(sp.width, sp.height, fs, fr, dither, p);
 				gpl.pre_pitch = pitch_of(sp.width, bytes(fr.type));
+				gpl.off_pre = off;
 				off += gpl.pre_pitch * sp.height;
 			}
 			if (!fmt_equal(fr, fd)) {
@@ -895,23 +931,15 @@ zg_graph *zg_graph_build(const zg_image_format *src_format, const zg_image_forma
 				off += gpl.mid_pitch * dp.height;
 			}
 			gpl.off_tmp = off;
-			gpl.tmp = off + rtmp;
-			g->tmp_size = std::max(g->tmp_size, gpl.tmp);
-		}
-		{
-			size_t off = (g->tmp_size + 255) & ~static_cast<size_t>(255);
-			for (auto &gpl : g->planes) {
-				EdPlane ep;
-				int it = 0, ot = 0;
-				if ((gpl.mode == 3 || gpl.mode == 4) && depth_ed_plane(gpl.only, &ep, &it, &ot)) {
-					gpl.ed_last = true;
-				} else if (gpl.mode == 2 && gpl.post && depth_ed_plane(gpl.post, &ep, &it, &ot)) {
-					gpl.ed_last = true;
-					gpl.off_mid_own = off;
-					off += gpl.mid_pitch * gpl.h;
-				}
-			}
+			off += (rtmp + 255) & ~static_cast<size_t>(255);
+			gpl.tmp = off - g->tmp_size;
 			g->tmp_size = off;
+		}
+		for (auto &gpl : g->planes) {
+			EdPlane ep;
+			int it = 0, ot = 0;
+			gpl.ed_last = ((gpl.mode == 3 || gpl.mode == 4) && depth_ed_plane(gpl.only, &ep, &it, &ot)) ||
+			              (gpl.mode == 2 && gpl.post && depth_ed_plane(gpl.post, &ep, &it, &ot));
 		}
 		// GREY to YUV / RGB without a colorspace change: the chroma outputs
 		// are the neutral value in the output format, or copies of the luma
@@ -954,7 +982,7 @@ zg_graph *zg_graph_build(const zg_image_format *src_format, const zg_image_forma
 			// after the conversion the planes are YUV unless the output
 			// matrix is RGB (convert_colorspace, graphbuilder.cpp:853-861)
 			const bool yuv_work = d.cs.m != csp::M_RGB;
-			size_t scratch = 0;
+			size_t scratch_in = 0, scratch_out = 0;
 			for (int p = 0; p < cm.n_in; ++p) {
 				const bool chroma = p != PLANE_Y;
 				const int q = (s.color == COLOR_RGB && chroma) ? PLANE_Y : p;
@@ -963,7 +991,8 @@ zg_graph *zg_graph_build(const zg_image_format *src_format, const zg_image_forma
 				                      uv ? gp.resample_filter_uv : gp.resample_filter,
 				                      uv ? gp.filter_param_a_uv : gp.filter_param_a,
 				                      uv ? gp.filter_param_b_uv : gp.filter_param_b, dither, p);
-				scratch = std::max(scratch, cm.in[p].scratch);
+				cm.in_off[p] = scratch_in;
+				scratch_in += cm.in[p].scratch;
 				auto &gpl = g->planes[p];
 				gpl.present = gpl.has_src = true;
 				gpl.mode = 6;
@@ -980,7 +1009,8 @@ zg_graph *zg_graph_build(const zg_image_format *src_format, const zg_image_forma
 				                       uv ? gp.resample_filter_uv : gp.resample_filter,
 				                       uv ? gp.filter_param_a_uv : gp.filter_param_a,
 				                       uv ? gp.filter_param_b_uv : gp.filter_param_b, dither, p);
-				scratch = std::max(scratch, cm.out[p].scratch);
+				cm.out_off[p] = scratch_out;
+				scratch_out += cm.out[p].scratch;
 				auto &gpl = g->planes[p];
 				gpl.present = gpl.has_dst = true;
 				gpl.mode = 6;
@@ -1000,7 +1030,7 @@ zg_graph *zg_graph_build(const zg_image_format *src_format, const zg_image_forma
 			                         v25 && gp.scene_referred != 0, v25 && gp.chromatic_adaptation != 0);
 			cm.off_work = (g->tmp_size + 255) & ~static_cast<size_t>(255);
 			cm.off_scratch = cm.off_work + 3 * cm.w_pitch * cm.wh;
-			g->tmp_size = cm.off_scratch + scratch;
+			g->tmp_size = cm.off_scratch + std::max(scratch_in, scratch_out);
 		}
 		// staging planes for ring buffers, after the largest per-plane scratch
 		size_t off = (g->tmp_size + 255) & ~static_cast<size_t>(255);
@@ -1173,6 +1203,7 @@ zg_error_code zg_graph_process_cb(const zg_graph *g, const zg_image_buffer_const
 			ptrdiff_t ds;
 		};
 		std::vector<Deferred> deferred;
+		Stage before, resize, after;
 		for (int p = 0; p < 4; ++p) {
 			const auto &pl = g->planes[p];
 			if (!pl.present)
@@ -1189,7 +1220,7 @@ zg_error_code zg_graph_process_cb(const zg_graph *g, const zg_image_buffer_const
 				if (pl.ed_last)
 					deferred.push_back({ pl.only, from, sst, dp, dst_st });
 				else
-					run_depth(pl.only, from, sst, dp, dst_st, stream);
+					before.add(pl.only, from, sst, dp, dst_st);
 				continue;
 			}
 			if (pl.mode >= 5)
@@ -1199,25 +1230,36 @@ zg_error_code zg_graph_process_cb(const zg_graph *g, const zg_image_buffer_const
 			const void *rs = sp;
 			ptrdiff_t rss = sst;
 			if (pl.pre) {
-				run_depth(pl.pre, sp, sst, t, static_cast<ptrdiff_t>(pl.pre_pitch), stream);
-				rs = t;
+				before.add(pl.pre, sp, sst, t + pl.off_pre, static_cast<ptrdiff_t>(pl.pre_pitch));
+				rs = t + pl.off_pre;
 				rss = static_cast<ptrdiff_t>(pl.pre_pitch);
 			}
-			void *rd = pl.post ? static_cast<void *>(t + (pl.ed_last ? pl.off_mid_own : pl.off_mid)) : static_cast<void *>(dp);
+			void *rd = pl.post ? static_cast<void *>(t + pl.off_mid) : static_cast<void *>(dp);
 			const ptrdiff_t rds = pl.post ? static_cast<ptrdiff_t>(pl.mid_pitch) : dst_st;
-			zg_error_code rc = pl.unresize
-			                       ? zg_unresize_process(pl.unresize, rs, rss, rd, rds, t ? t + pl.off_tmp : nullptr, stream)
-			                       : zg_resize_process(pl.resize, rs, rss, rd, rds, t ? t + pl.off_tmp : nullptr, stream);
-			if (rc != ZG_ERROR_SUCCESS) {
-				char msg[256];
-				zg_get_last_error(msg, sizeof(msg));
-				throw Error(rc, msg);
-			}
+			resize.add(pl.resize, rs, rss, rd, rds, t ? t + pl.off_tmp : nullptr);
 			if (pl.post && pl.ed_last)
 				deferred.push_back({ pl.post, rd, rds, dp, dst_st });
 			else if (pl.post)
-				run_depth(pl.post, rd, rds, dp, dst_st, stream);
+				after.add(pl.post, rd, rds, dp, dst_st);
 		}
+		before.run(st);
+		if (g->unresizes) {
+			for (int k = 0, p = 0; p < 4; ++p) {
+				const auto &pl = g->planes[p];
+				if (!pl.present || pl.mode != 2)
+					continue;
+				const ResizeIo &x = resize.resize[k++];
+				zg_error_code rc = zg_unresize_process(pl.unresize, x.src, x.src_stride, x.dst, x.dst_stride, x.tmp, stream);
+				if (rc != ZG_ERROR_SUCCESS) {
+					char msg[256];
+					zg_get_last_error(msg, sizeof(msg));
+					throw Error(rc, msg);
+				}
+			}
+		} else {
+			resize.run(st);
+		}
+		after.run(st);
 		run_ed_planes(deferred.data(), static_cast<int>(deferred.size()), stream);
 
 		if (g->premul.on) {
@@ -1291,8 +1333,13 @@ zg_error_code zg_graph_process_cb(const zg_graph *g, const zg_image_buffer_const
 			const ptrdiff_t wp = static_cast<ptrdiff_t>(cm.w_pitch);
 			auto work = [&](int p) { return t + cm.off_work + static_cast<size_t>(p) * cm.w_pitch * cm.wh; };
 			char *scratch = t + cm.off_scratch;
-			for (int p = 0; p < cm.n_in; ++p)
-				run_chain(cm.in[p], from_data[p], from_stride[p], work(p), wp, scratch, stream);
+			void *work_data[3];
+			ptrdiff_t work_stride[3];
+			for (int p = 0; p < 3; ++p) {
+				work_data[p] = work(p);
+				work_stride[p] = wp;
+			}
+			run_chains(cm.in, cm.n_in, from_data, from_stride, work_data, work_stride, scratch, cm.in_off, st);
 			for (int p = cm.n_in; p < 3; ++p)
 				copy_plane(work(p), wp, work(0), wp, static_cast<size_t>(cm.ww) * 4, cm.wh, st);
 			if (cm.plan.num_ops) {
@@ -1308,8 +1355,7 @@ zg_error_code zg_graph_process_cb(const zg_graph *g, const zg_image_buffer_const
 				L.plan = cm.plan;
 				cuda_check(csp::launch_colorspace(L, st), "colorspace launch");
 			}
-			for (int p = 0; p < cm.n_out; ++p)
-				run_chain(cm.out[p], work(p), wp, to_data[p], to_stride[p], scratch, stream);
+			run_chains(cm.out, cm.n_out, work_data, work_stride, to_data, to_stride, scratch, cm.out_off, st);
 		}
 		for (int p = 0; p < 4; ++p) {
 			if (g->out_fill[p] == 1) {

@@ -378,7 +378,7 @@ int chain_threads(int variant)
 }
 
 cudaError_t launch_chain(int variant, const FusedJob *jobs, int num_jobs, int total_items, const SmemLayout &L, int grid,
-                         const FusedJob &single, cudaStream_t stream)
+                         const FewJobs &few, cudaStream_t stream)
 {
 	if (L.total_bytes > static_cast<int>(kChainSmemMax))
 		return cudaErrorInvalidValue;
@@ -386,9 +386,9 @@ cudaError_t launch_chain(int variant, const FusedJob *jobs, int num_jobs, int to
 	cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kChainSmemMax));
 	if (e != cudaSuccess)
 		return e;
-	FusedJob one = single;
+	FewJobs by_value = few;
 	SmemLayout layout = L;
-	void *args[] = { &jobs, &num_jobs, &total_items, &one, &layout };
+	void *args[] = { &jobs, &num_jobs, &total_items, &by_value, &layout };
 	grid = std::max(1, std::min(grid, total_items));
 	return cudaLaunchKernel(k, dim3(grid), dim3(chain_threads(variant)), args, static_cast<size_t>(L.total_bytes),
 	                        stream);

@@ -378,7 +378,7 @@ __device__ __forceinline__ void store_chunk(const Item &it, const char *ld_addr,
 // of group k + 1 + depth: the planner sizes the ring and the slots for that.
 template <bool H_FIRST, int KV, int KH>
 __global__ void __launch_bounds__(warps_per_cta(H_FIRST) * 32, 2)
-chain_kernel(const FusedJob *__restrict__ jobs, int num_jobs, int total_items, const __grid_constant__ FusedJob single,
+chain_kernel(const FusedJob *__restrict__ jobs, int num_jobs, int total_items, const __grid_constant__ FewJobs few,
              const __grid_constant__ SmemLayout L)
 {
 	extern __shared__ float4 smem4[];
@@ -415,7 +415,8 @@ chain_kernel(const FusedJob *__restrict__ jobs, int num_jobs, int total_items, c
 	// order: whole strips where they fit, split at most at its two ends
 	const int t_end = static_cast<int>(static_cast<long long>(blockIdx.x + 1) * total_items / gridDim.x);
 	for (int t = static_cast<int>(static_cast<long long>(blockIdx.x) * total_items / gridDim.x); t < t_end;) {
-		const FusedJob *Jp = jobs ? &jobs[find_job(jobs, num_jobs, t)] : &single;
+		const FusedJob *table = jobs ? jobs : few.job;
+		const FusedJob *Jp = &table[find_job(table, num_jobs, t)];
 		const Item it = make_item(*Jp, t, t_end, kStripTiles, kThreads);
 		t += it.g_end - it.g_begin;
 		for (int g = it.g_begin + threadIdx.x; g < it.g_end; g += kThreads)

@@ -201,21 +201,21 @@ int chain_tma_grid_size(int variant, size_t smem_bytes)
 }
 
 cudaError_t launch_chain_tma(int variant, const FusedJob *jobs, int num_jobs, int total_items, const int *ranges,
-                             const SmemLayout &L, int grid, const FusedJob &single, const CUtensorMap *single_map,
+                             const SmemLayout &L, int grid, const FewJobs &few, const FewMaps *few_maps,
                              cudaStream_t stream)
 {
-	if (static_cast<size_t>(L.total_bytes) > kTmaSmemMax || (!jobs && !single_map))
+	if (static_cast<size_t>(L.total_bytes) > kTmaSmemMax || (!jobs && !few_maps))
 		return cudaErrorInvalidValue;
 	const void *k = chain_tma_kernel_ptr(variant);
 	cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kTmaSmemMax));
 	if (e != cudaSuccess)
 		return e;
-	FusedJob one = single;
+	FewJobs by_value = few;
 	SmemLayout layout = L;
-	CUtensorMap map{};
-	if (single_map)
-		map = *single_map;
-	void *args[] = { &jobs, &num_jobs, &total_items, &ranges, &one, &layout, &map };
+	FewMaps maps{};
+	if (few_maps)
+		maps = *few_maps;
+	void *args[] = { &jobs, &num_jobs, &total_items, &ranges, &by_value, &layout, &maps };
 	if (!ranges)
 		grid = std::max(1, std::min(grid, total_items));
 	return cudaLaunchKernel(k, dim3(grid), dim3(tma_threads(variant)), args, static_cast<size_t>(L.total_bytes),

@@ -615,8 +615,8 @@ __device__ __forceinline__ void load_bases(Pipe &p, const FusedJob &J, int g_beg
 template <bool H_FIRST, int KV, int KH>
 __global__ void __launch_bounds__(tma_threads(H_FIRST), 2)
 chain_tma_kernel(const FusedJob *__restrict__ jobs, int num_jobs, int total_items, const int *__restrict__ ranges,
-                 const __grid_constant__ FusedJob single, const __grid_constant__ SmemLayout L,
-                 const __grid_constant__ CUtensorMap single_map)
+                 const __grid_constant__ FewJobs few, const __grid_constant__ SmemLayout L,
+                 const __grid_constant__ FewMaps few_maps)
 {
 	extern __shared__ float4 smem4[];
 	__shared__ int abort_item;
@@ -636,14 +636,16 @@ chain_tma_kernel(const FusedJob *__restrict__ jobs, int num_jobs, int total_item
 	for (int r = 0; r < 2 && !abort_item; ++r) {
 		const int t_end = r_end[r];
 		for (int t = r_begin[r]; t < t_end;) {
-			const FusedJob &J = jobs ? jobs[find_job(jobs, num_jobs, t)] : single;
+			const FusedJob *table = jobs ? jobs : few.job;
+			const int job = find_job(table, num_jobs, t);
+			const FusedJob &J = table[job];
 			const int local = t - J.item_begin;
 			const int strip = local / J.groups;
 			const int g_begin = local - strip * J.groups;
 			const int ngroups = min(J.groups - g_begin, t_end - t);
 			t += ngroups;
 			load_bases(p, J, g_begin, ngroups);
-			chain_item<H_FIRST, KV, KH, true>(p, L, J, jobs ? J.tmap : static_cast<const void *>(&single_map), strip,
+			chain_item<H_FIRST, KV, KH, true>(p, L, J, jobs ? J.tmap : static_cast<const void *>(&few_maps.map[job]), strip,
 			                                  g_begin, ngroups);
 			p.base += ngroups;
 			__syncthreads();  // the next item rewrites the group bases and the ring

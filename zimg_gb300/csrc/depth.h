@@ -22,9 +22,17 @@ struct DepthLaunch {
 	int vec_in, vec_out;  // planes aligned for 8-sample vector loads / stores
 };
 
+// Planes of one launch: the same types, mode and dither kind.
+constexpr int kDepthMaxPlanes = 4;
+
+struct DepthPlanes {
+	DepthLaunch plane[kDepthMaxPlanes];
+	int num;
+};
+
 // in_type / out_type: 0 BYTE, 1 WORD, 2 HALF, 3 FLOAT; mode 1 left shift,
 // 2 to FLOAT or HALF, 3 dither to integer.
-cudaError_t launch_depth(int in_type, int out_type, int mode, const DepthLaunch &L, cudaStream_t stream);
+cudaError_t launch_depth(int in_type, int out_type, int mode, const DepthPlanes &P, cudaStream_t stream);
 
 // Error diffusion (ed_kernel.cu). One thread block per plane; in a block,
 // warp w takes bands of 32 lines b = w, w + warps, ..., one line per lane.
@@ -74,6 +82,20 @@ int ed_wait_error(bool reset);
 struct zg_depth;
 
 namespace zg {
+
+// One plane of a depth conversion object.
+struct DepthIo {
+	const ::zg_depth *d;
+	const void *src;
+	ptrdiff_t src_stride;
+	void *dst;
+	ptrdiff_t dst_stride;
+};
+
+// Independent planes, in as few launches as their types, modes and dither
+// kinds allow (error diffusion: a launch a plane). Throws on bad arguments and
+// failed launches.
+void depth_planes(const DepthIo *io, int n, cudaStream_t stream);
 
 // The error-diffusion plane of a depth conversion object (its size, scale,
 // offset and range; pointers unset) and its pixel types; false when the

@@ -157,11 +157,16 @@ __device__ __forceinline__ void store_run(U *p, const uint32_t (&r)[kRun], int n
 }
 
 // MODE 1: left shift; 2: to float; 3: dither to integer. DITHER (MODE 3):
-// 0 none, 1 ordered, 2 random.
+// 0 none, 1 ordered, 2 random. Row y of the grid is the launch's plane y.
 template <class T, class U, int MODE, int DITHER>
 __global__ void __launch_bounds__(kThreads)
-depth_kernel(DepthLaunch L)
+depth_kernel(const __grid_constant__ DepthPlanes P)
 {
+	const DepthLaunch &L = P.plane[blockIdx.y];
+	const int runs = (L.width + kRun - 1) / kRun;
+	const long long total = static_cast<long long>(runs) * L.height;
+	if (static_cast<long long>(blockIdx.x) * kThreads >= total)
+		return;  // a larger plane of the launch sets the grid
 	// ORDERED: this plane's 16 x 16 dither values, row-major. RANDOM: the
 	// values (m + 1) / 257 - 1/2 of the 256 matrix entries m, and the
 	// plane's 64 x 64 entries already moved by its offsets, four per word.
@@ -197,8 +202,6 @@ depth_kernel(DepthLaunch L)
 	}
 	// the plane's runs of 8 samples, line by line, strided over the grid;
 	// (line, run) advance by the stride's fixed quotient and remainder
-	const int runs = (L.width + kRun - 1) / kRun;
-	const long long total = static_cast<long long>(runs) * L.height;
 	const long long stride = static_cast<long long>(gridDim.x) * kThreads;
 	long long u = static_cast<long long>(blockIdx.x) * kThreads + threadIdx.x;
 	int i = static_cast<int>(u / runs), r = static_cast<int>(u % runs);
@@ -297,29 +300,29 @@ template <class T>
 constexpr bool is_fp = std::is_same_v<T, float> || std::is_same_v<T, Half>;
 
 template <class T, class U>
-cudaError_t launch_tu(int mode, const DepthLaunch &L, int grid, cudaStream_t st)
+cudaError_t launch_tu(int mode, const DepthPlanes &P, dim3 grid, cudaStream_t st)
 {
 	switch (mode) {
 	case 1:
 		if constexpr (is_int<T> && is_int<U>) {
-			depth_kernel<T, U, 1, 0><<<grid, kThreads, 0, st>>>(L);
+			depth_kernel<T, U, 1, 0><<<grid, kThreads, 0, st>>>(P);
 			return cudaGetLastError();
 		}
 		return cudaErrorInvalidValue;
 	case 2:
 		if constexpr (is_fp<U>) {
-			depth_kernel<T, U, 2, 0><<<grid, kThreads, 0, st>>>(L);
+			depth_kernel<T, U, 2, 0><<<grid, kThreads, 0, st>>>(P);
 			return cudaGetLastError();
 		}
 		return cudaErrorInvalidValue;
 	case 3:
 		if constexpr (is_int<U>) {
-			if (L.dither == 1)
-				depth_kernel<T, U, 3, 1><<<grid, kThreads, 0, st>>>(L);
-			else if (L.dither == 2)
-				depth_kernel<T, U, 3, 2><<<grid, kThreads, 0, st>>>(L);
+			if (P.plane[0].dither == 1)
+				depth_kernel<T, U, 3, 1><<<grid, kThreads, 0, st>>>(P);
+			else if (P.plane[0].dither == 2)
+				depth_kernel<T, U, 3, 2><<<grid, kThreads, 0, st>>>(P);
 			else
-				depth_kernel<T, U, 3, 0><<<grid, kThreads, 0, st>>>(L);
+				depth_kernel<T, U, 3, 0><<<grid, kThreads, 0, st>>>(P);
 			return cudaGetLastError();
 		}
 		return cudaErrorInvalidValue;
@@ -328,23 +331,26 @@ cudaError_t launch_tu(int mode, const DepthLaunch &L, int grid, cudaStream_t st)
 }
 
 template <class T>
-cudaError_t launch_t(int out_type, int mode, const DepthLaunch &L, int grid, cudaStream_t st)
+cudaError_t launch_t(int out_type, int mode, const DepthPlanes &P, dim3 grid, cudaStream_t st)
 {
 	switch (out_type) {
-	case 0: return launch_tu<T, uint8_t>(mode, L, grid, st);
-	case 1: return launch_tu<T, uint16_t>(mode, L, grid, st);
-	case 2: return launch_tu<T, Half>(mode, L, grid, st);
-	case 3: return launch_tu<T, float>(mode, L, grid, st);
+	case 0: return launch_tu<T, uint8_t>(mode, P, grid, st);
+	case 1: return launch_tu<T, uint16_t>(mode, P, grid, st);
+	case 2: return launch_tu<T, Half>(mode, P, grid, st);
+	case 3: return launch_tu<T, float>(mode, P, grid, st);
 	default: return cudaErrorInvalidValue;
 	}
 }
 
 } // namespace
 
-cudaError_t launch_depth(int in_type, int out_type, int mode, const DepthLaunch &L, cudaStream_t stream)
+cudaError_t launch_depth(int in_type, int out_type, int mode, const DepthPlanes &P, cudaStream_t stream)
 {
-	if (L.width <= 0 || L.height <= 0)
-		return cudaSuccess;
+	long long most = 0;
+	for (int k = 0; k < P.num; ++k)
+		most = std::max(most, static_cast<long long>((P.plane[k].width + kRun - 1) / kRun) * P.plane[k].height);
+	if (P.num < 1 || P.num > kDepthMaxPlanes || most <= 0)
+		return P.num == 0 || most <= 0 ? cudaSuccess : cudaErrorInvalidValue;
 	static int sms = 0;
 	if (!sms) {
 		int dev = 0;
@@ -353,13 +359,13 @@ cudaError_t launch_depth(int in_type, int out_type, int mode, const DepthLaunch 
 		if (sms < 1)
 			sms = 1;
 	}
-	const long long runs = static_cast<long long>((L.width + kRun - 1) / kRun) * L.height;
-	const int grid = static_cast<int>(std::min<long long>((runs + kThreads - 1) / kThreads, static_cast<long long>(sms) * 8));
+	const dim3 grid(static_cast<unsigned>(std::min<long long>((most + kThreads - 1) / kThreads, static_cast<long long>(sms) * 8)),
+	                static_cast<unsigned>(P.num));
 	switch (in_type) {
-	case 0: return launch_t<uint8_t>(out_type, mode, L, grid, stream);
-	case 1: return launch_t<uint16_t>(out_type, mode, L, grid, stream);
-	case 2: return launch_t<Half>(out_type, mode, L, grid, stream);
-	case 3: return launch_t<float>(out_type, mode, L, grid, stream);
+	case 0: return launch_t<uint8_t>(out_type, mode, P, grid, stream);
+	case 1: return launch_t<uint16_t>(out_type, mode, P, grid, stream);
+	case 2: return launch_t<Half>(out_type, mode, P, grid, stream);
+	case 3: return launch_t<float>(out_type, mode, P, grid, stream);
 	default: return cudaErrorInvalidValue;
 	}
 }

@@ -352,12 +352,12 @@ bool fused_takes_chunks(int variant)
 }
 
 cudaError_t launch_fused(int variant, const FusedJob *jobs, int num_jobs, int total_tiles, const SmemLayout &smem_bytes,
-                         int grid, const FusedJob &single, cudaStream_t stream, const WorkChunks &chunks)
+                         int grid, const FewJobs &few, cudaStream_t stream, const WorkChunks &chunks)
 {
 	if (variant >= 200)
-		return launch_chain(variant, jobs, num_jobs, total_tiles, smem_bytes, grid, single, stream);
+		return launch_chain(variant, jobs, num_jobs, total_tiles, smem_bytes, grid, few, stream);
 	if (variant >= 100)
-		return launch_mma(variant, jobs, num_jobs, total_tiles, smem_bytes, grid, single, stream);
+		return launch_mma(variant, jobs, num_jobs, total_tiles, smem_bytes, grid, few.job[0], stream);
 	grid = std::max(1, std::min(grid, chunks.sched ? chunks.num : total_tiles));
 	if (smem_bytes.total_bytes > static_cast<int>(kSmemMax))
 		return cudaErrorInvalidValue;
@@ -365,10 +365,10 @@ cudaError_t launch_fused(int variant, const FusedJob *jobs, int num_jobs, int to
 	cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemMax));
 	if (e != cudaSuccess)
 		return e;
-	FusedJob one = single;
+	FewJobs by_value = few;
 	SmemLayout layout = smem_bytes;
 	WorkChunks c = chunks;
-	void *args[] = { &jobs, &num_jobs, &total_tiles, &one, &layout, &c };
+	void *args[] = { &jobs, &num_jobs, &total_tiles, &by_value, &layout, &c };
 	return cudaLaunchKernel(k, dim3(grid), dim3(kStreamThreads), args, static_cast<size_t>(layout.total_bytes), stream);
 }
 

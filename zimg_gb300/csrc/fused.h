@@ -107,6 +107,14 @@ struct FusedJob {
 	int variant;            // chained kernel's variant - 200 ((H first, KV, KH)); mixed launches dispatch on it
 };
 
+// The jobs of a launch without a device table, by value (a plane, or the
+// planes of a frame that share a variant).
+constexpr int kFewJobs = 4;
+
+struct FewJobs {
+	FusedJob job[kFewJobs];
+};
+
 // Guided work chunks of a persistent launch (work_chunks.cuh): chunk m is
 // the work units [bounds[m], bounds[m + 1]) (device memory, strictly
 // increasing, num chunks); CTAs take chunks from the counter sched[0] in the
@@ -171,10 +179,11 @@ void fused_bind(FusedPlan &p, const void *device_blob);
 SmemLayout fused_layout(const FusedPlan *const *plans, int n);
 
 // Launch all items of `jobs` (a device array of num_jobs FusedJob, all of the
-// same variant) as one persistent grid; with jobs == nullptr, run `single`
-// (passed by value as a kernel parameter).
+// same variant) as one persistent grid; with jobs == nullptr, the num_jobs
+// jobs of `few` (passed by value as a kernel parameter; the tensor-core kernels
+// of variants 100-199 take one).
 cudaError_t launch_fused(int variant, const FusedJob *jobs, int num_jobs, int total_items, const SmemLayout &L,
-                         int grid, const FusedJob &single, cudaStream_t stream, const WorkChunks &chunks = {});
+                         int grid, const FewJobs &few, cudaStream_t stream, const WorkChunks &chunks = {});
 // Whether launch_fused takes guided chunks for this variant (the CUDA-core
 // streaming kernel does; the tensor-core forms launched through it split
 // their units statically).
@@ -204,7 +213,7 @@ SmemLayout chain_layout(const FusedPlan *const *plans, int n);
 const void *chain_kernel_ptr(int variant);
 int chain_threads(int variant);
 cudaError_t launch_chain(int variant, const FusedJob *jobs, int num_jobs, int total_items, const SmemLayout &L, int grid,
-                         const FusedJob &single, cudaStream_t stream);
+                         const FewJobs &few, cudaStream_t stream);
 // The same kernel with source lines and tap fragments brought in by tensor
 // copies on an mbarrier pipeline (chain_tma_kernel.cuh). Usable when the
 // layout fits (box width <= 256) and the source plane has a tensor map
@@ -216,8 +225,12 @@ int chain_tma_grid_size(int variant, size_t smem_bytes);
 // ranges: null (each CTA an equal contiguous range of the units), or 4 ints
 // per CTA of `grid`, two unit ranges each CTA runs in order
 // (chain_tma_lockstep_ranges).
+// Without `jobs`: the num_jobs jobs of `few` and their tensor maps, by value.
+struct FewMaps {
+	CUtensorMap map[kFewJobs];
+};
 cudaError_t launch_chain_tma(int variant, const FusedJob *jobs, int num_jobs, int total_items, const int *ranges,
-                             const SmemLayout &L, int grid, const FusedJob &single, const CUtensorMap *single_map,
+                             const SmemLayout &L, int grid, const FewJobs &few, const FewMaps *few_maps,
                              cudaStream_t stream);
 // Per-CTA unit ranges for `grid` CTAs over jobs of `groups` units per strip
 // and `total_items` units: CTA b first the whole strip b, then an equal share

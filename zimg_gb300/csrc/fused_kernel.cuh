@@ -94,7 +94,7 @@ __device__ __forceinline__ int find_job(const FusedJob *__restrict__ jobs, int n
 	int lo = 0, hi = num_jobs - 1;
 	while (lo < hi) {
 		const int mid = (lo + hi + 1) >> 1;
-		if (__ldg(&jobs[mid].item_begin) <= t)
+		if (jobs[mid].item_begin <= t)
 			lo = mid;
 		else
 			hi = mid - 1;
@@ -591,7 +591,7 @@ __device__ __forceinline__ void hfirst_v(const Item &it, uint32_t mid, uint32_t 
 
 template <bool H_FIRST, bool INT, int HW, int VS>
 __global__ void __launch_bounds__(kThreads, HW <= 8 ? 5 : 4)
-fused_kernel(const FusedJob *__restrict__ jobs, int num_jobs, int total_items, const __grid_constant__ FusedJob single,
+fused_kernel(const FusedJob *__restrict__ jobs, int num_jobs, int total_items, const __grid_constant__ FewJobs few,
              const __grid_constant__ SmemLayout L, const __grid_constant__ WorkChunks C)
 {
 	constexpr int E = INT ? 2 : 4;
@@ -620,7 +620,8 @@ fused_kernel(const FusedJob *__restrict__ jobs, int num_jobs, int total_items, c
 			break;
 		}
 		for (int t = c_begin; t < c_end;) {
-			const FusedJob &J = jobs ? jobs[find_job(jobs, num_jobs, t)] : single;
+			const FusedJob *table = jobs ? jobs : few.job;
+			const FusedJob &J = table[find_job(table, num_jobs, t)];
 			const Item it = make_item(J, t, c_end);
 			t += it.steps;
 

@@ -123,7 +123,7 @@ __device__ __forceinline__ int find_job(const FusedJob *__restrict__ jobs, int n
 	int lo = 0, hi = num_jobs - 1;
 	while (lo < hi) {
 		const int mid = (lo + hi + 1) >> 1;
-		if (__ldg(&jobs[mid].item_begin) <= t)
+		if (jobs[mid].item_begin <= t)
 			lo = mid;
 		else
 			hi = mid - 1;
