@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import struct
 
 _PKG = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_PKG, "_lib", "libzimg_gb300.so")
@@ -109,6 +110,13 @@ class ImageBuffer(C.Structure):
 
 
 API_VERSION_2_4 = (2 << 8) | 4
+
+_IMAGE_BUFFER = struct.Struct("@I" + "PqI" * 4 + "0P")  # ImageBuffer's layout
+
+
+def image_buffer(fields) -> ImageBuffer:
+    """An ImageBuffer of four planes' (data, stride, mask), in one list."""
+    return ImageBuffer.from_buffer_copy(_IMAGE_BUFFER.pack(API_VERSION_2_4, *fields))
 
 # zg_graph_callback: int (*)(void *user, unsigned i, unsigned left, unsigned right)
 GRAPH_CALLBACK = C.CFUNCTYPE(C.c_int, C.c_void_p, C.c_uint, C.c_uint, C.c_uint)

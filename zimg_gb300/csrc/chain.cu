@@ -383,9 +383,6 @@ cudaError_t launch_chain(int variant, const FusedJob *jobs, int num_jobs, int to
 	if (L.total_bytes > static_cast<int>(kChainSmemMax))
 		return cudaErrorInvalidValue;
 	const void *k = chain_kernel_ptr(variant);
-	cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kChainSmemMax));
-	if (e != cudaSuccess)
-		return e;
 	FewJobs by_value = few;
 	SmemLayout layout = L;
 	void *args[] = { &jobs, &num_jobs, &total_items, &by_value, &layout };

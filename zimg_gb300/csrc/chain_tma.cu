@@ -207,9 +207,6 @@ cudaError_t launch_chain_tma(int variant, const FusedJob *jobs, int num_jobs, in
 	if (static_cast<size_t>(L.total_bytes) > kTmaSmemMax || (!jobs && !few_maps))
 		return cudaErrorInvalidValue;
 	const void *k = chain_tma_kernel_ptr(variant);
-	cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kTmaSmemMax));
-	if (e != cudaSuccess)
-		return e;
 	FewJobs by_value = few;
 	SmemLayout layout = L;
 	FewMaps maps{};
@@ -265,9 +262,6 @@ cudaError_t launch_chain_mixed(const FusedJob *jobs, int num_jobs, const WorkChu
 	    chunks.num < 1 || grid < 1)
 		return cudaErrorInvalidValue;
 	const void *k = reinterpret_cast<const void *>(&chain_detail::chain_mixed_kernel);
-	cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kTmaSmemMax));
-	if (e != cudaSuccess)
-		return e;
 	SmemLayout layout = L;
 	WorkChunks C = chunks;
 	grid = std::min(grid, C.num);

@@ -25,6 +25,7 @@
 
 #include "depth.h"
 #include "depth_device.cuh"
+#include "launch_attr.h"
 #include "pipeline.cuh"
 
 namespace zg {
@@ -663,8 +664,9 @@ cudaError_t launch_cluster(const EdLaunch &L, int warps, cudaStream_t st)
 		C.ring = std::max(C.ring, hand_off_floats(band_chunks(L.planes[k].width)));
 	}
 	C.warps = cluster * warps;
-	cudaError_t e = cudaFuncSetAttribute(ed_cluster_kernel<T, U>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-	                                     static_cast<int>(kMaxSmem));
+	static std::atomic<unsigned long long> devices{ 0 };
+	cudaError_t e = allow_shared_memory(reinterpret_cast<const void *>(&ed_cluster_kernel<T, U>),
+	                                    static_cast<int>(kMaxSmem), devices);
 	if (e != cudaSuccess)
 		return e;
 	cudaLaunchConfig_t cfg{};
@@ -686,14 +688,11 @@ cudaError_t launch_tu(const EdLaunch &L, size_t smem, cudaStream_t st)
 {
 	if (const int warps = cluster_warps(L))
 		return launch_cluster<T, U>(L, warps, st);
-	static bool raised = false;
-	if (!raised) {
-		cudaError_t e = cudaFuncSetAttribute(ed_kernel<T, U>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-		                                     static_cast<int>(kMaxSmem));
-		if (e != cudaSuccess)
-			return e;
-		raised = true;
-	}
+	static std::atomic<unsigned long long> devices{ 0 };
+	cudaError_t e = allow_shared_memory(reinterpret_cast<const void *>(&ed_kernel<T, U>), static_cast<int>(kMaxSmem),
+	                                    devices);
+	if (e != cudaSuccess)
+		return e;
 	ed_kernel<T, U><<<L.num_planes, L.warps * 32, smem, st>>>(L);
 	return cudaGetLastError();
 }

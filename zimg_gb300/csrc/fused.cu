@@ -112,15 +112,21 @@ bool plan_fused(const FilterTable &first, const FilterTable &second, bool h_firs
 	// fewest warp passes per output: V first, the vertical pass's (quad of
 	// columns, half of a step's rows) items fill whole warps or not
 	const int col_align = u16 ? 8 : 4;
+	const int blocks = static_cast<int>((dst_w + 7) / 8);  // of 8 columns: their first and last inputs
+	std::vector<int> block_lo(blocks, INT_MAX), block_hi(blocks, INT_MIN);
+	for (unsigned c = 0; c < dst_w; ++c) {
+		block_lo[c / 8] = std::min(block_lo[c / 8], static_cast<int>(H.left[c]));
+		block_hi[c / 8] = std::max(block_hi[c / 8], static_cast<int>(H.left[c]) + HW);
+	}
 	auto windows = [&](int w, std::vector<int> &win) {
 		const int n = static_cast<int>((dst_w + w - 1) / w);
 		win.assign(2 * n, 0);
 		int widest = 0;
 		for (int s = 0; s < n; ++s) {
 			int lo = INT_MAX, hi = INT_MIN;
-			for (unsigned c = s * w; c < std::min<unsigned>(dst_w, (s + 1) * w); ++c) {
-				lo = std::min(lo, static_cast<int>(H.left[c]));
-				hi = std::max(hi, static_cast<int>(H.left[c]) + HW);
+			for (int k = s * w / 8; k < std::min(blocks, (s + 1) * w / 8); ++k) {
+				lo = std::min(lo, block_lo[k]);
+				hi = std::max(hi, block_hi[k]);
 			}
 			win[2 * s] = lo / col_align * col_align;
 			win[2 * s + 1] = hi;
@@ -362,9 +368,6 @@ cudaError_t launch_fused(int variant, const FusedJob *jobs, int num_jobs, int to
 	if (smem_bytes.total_bytes > static_cast<int>(kSmemMax))
 		return cudaErrorInvalidValue;
 	const void *k = kernel_ptr(variant);
-	cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemMax));
-	if (e != cudaSuccess)
-		return e;
 	FewJobs by_value = few;
 	SmemLayout layout = smem_bytes;
 	WorkChunks c = chunks;

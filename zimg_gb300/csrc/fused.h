@@ -190,6 +190,10 @@ cudaError_t launch_fused(int variant, const FusedJob *jobs, int num_jobs, int to
 bool fused_takes_chunks(int variant);
 
 size_t fused_max_smem();
+// CTAs that fill the current device. Also admits the launch's shared memory on
+// this device, which the launches of a variant rely on: every plan asks here
+// first (as do the chained kernels' plans, chain_tma_grid_size and
+// chain_mixed_grid_size).
 int fused_grid_size(int variant, size_t smem_bytes);
 int fused_items(const FusedJob &j);
 

@@ -31,6 +31,8 @@
 // here.
 #include "unresize.h"
 
+#include "launch_attr.h"
+
 #include <algorithm>
 
 namespace zg {
@@ -464,7 +466,8 @@ cudaError_t launch_unresize(const UnresizeTables &t, bool horizontal, unsigned l
 	const ChunkShape L = chunk_shape(t, horizontal, &smem);
 	if (L.series) {
 		const auto kernel = horizontal ? unresize_lines<true> : unresize_lines<false>;
-		cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+		static std::atomic<unsigned long long> devices[2] = {};
+		cudaError_t e = allow_shared_memory(reinterpret_cast<const void *>(kernel), 227 * 1024, devices[horizontal]);
 		if (e != cudaSuccess)
 			return e;
 		// the dot products and the copies out want more threads than the chunks

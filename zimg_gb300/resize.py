@@ -46,22 +46,40 @@ def _pixel_id(t) -> int:
 
 def _stream_handle(stream) -> int | None:
     if stream is None:
-        import torch
-        return torch.cuda.current_stream().cuda_stream
+        global _current_stream
+        if _current_stream is None:
+            _current_stream = _find_current_stream()
+        return _current_stream()
     if isinstance(stream, int):
         return stream
     return stream.cuda_stream
 
 
+_current_stream = None
+
+
+def _find_current_stream():
+    """The handle of the current stream of the current device, by PyTorch's raw
+    getters where it has them (a torch.cuda.Stream object costs 3 us a call)."""
+    import torch
+    raw, device = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
+    torch.cuda.current_stream()  # CUDA is initialised
+    if raw and device:
+        return lambda: raw(device())
+    return lambda: torch.cuda.current_stream().cuda_stream
+
+
 def _plane(t):
     """(device pointer, byte stride, width, height) of a 2-D CUDA tensor."""
-    if t.dim() != 2:
+    shape = t.shape
+    if len(shape) != 2:
         raise ValueError("planes are 2-D tensors [height, width]")
-    if t.stride(1) != 1:
+    rows, columns = t.stride()
+    if columns != 1:
         raise ValueError("plane rows must be contiguous")
     if not t.is_cuda:
         raise ValueError("planes must be CUDA tensors")
-    return t.data_ptr(), t.stride(0) * t.element_size(), t.shape[1], t.shape[0]
+    return t.data_ptr(), rows * t.element_size(), shape[1], shape[0]
 
 
 @dataclass
@@ -598,15 +616,13 @@ class Graph:
         pack: Python callables f(i, left, right) -> int, called as zimg's
         zimg_filter_graph_callback (zimg.h:455-484)."""
         def buf(planes, masks):
-            b = capi.ImageBuffer()
-            b.version = capi.API_VERSION_2_4
+            fields = [0, 0, 0] * 4
             for i, t in enumerate(planes):
                 if t is None:
                     continue
                 ptr, stride, _, _ = _plane(t)
-                mask = capi.BUFFER_MAX if not masks or masks[i] is None else masks[i]
-                b.plane[i] = capi._PlaneC(ptr, stride, mask)
-            return b
+                fields[3 * i:3 * i + 3] = ptr, stride, capi.BUFFER_MAX if not masks or masks[i] is None else masks[i]
+            return capi.image_buffer(fields)
         s, d = buf(src_planes, src_masks), buf(dst_planes, dst_masks)
         if tmp is None and self.tmp_size:
             import torch
