@@ -111,6 +111,57 @@ def test_cp_async_form_bitexact(cuda, oracle, tmp_path):
                                           err_msg=f"{mode} {BATCH[i]}")
 
 
+@pytest.mark.parametrize("sw,sh,dw,dh,kind", [
+    (240, 96, 480, 192, "lanczos"),     # 2x up: kept products, four tiles a warp
+    (1919, 70, 1279, 47, "spline36"),   # 1.5x down, odd lines
+    (641, 131, 961, 197, "spline36"),   # 1.5x up
+    (900, 65, 400, 29, "bicubic"),      # 2.25x down: strips narrower than seven warps' tiles
+    (33, 17, 66, 34, "lanczos"),        # one strip, fewer lines than a window
+    (320, 40, 426, 53, "bicubic"),      # a source for tensor copies, narrower strips, 4-byte stores
+    (320, 40, 424, 53, "bicubic"),      # ... 16-byte stores
+    (640, 64, 427, 43, "spline36"),     # ... single samples
+    (17, 300, 23, 200, "bicubic")])
+@pytest.mark.parametrize("pad,offset,flip", [(0, 0, False), (1, 1, False), (2, 4, False), (3, 7, False), (4, 2, True),
+                                             (8, 8, False)])
+def test_chained_kernel_any_alignment(cuda, oracle, sw, sh, dw, dh, kind, pad, offset, flip):
+    """Planes at every offset of their lines in a 16-byte chunk, sources and
+    destinations, bottom-up ones too, with all bits set between the lines
+    (nothing there may reach a result) and kept between the output lines;
+    single planes and a batch, bit for bit."""
+    import torch
+    import zimg_gb300 as zg
+    rng = np.random.default_rng(sw * 17 + pad)
+    src = rng.integers(0, 1024, size=(sh, sw), dtype=np.uint16)
+    want = oracle.resize_plane(src, dw, dh, kind, depth=10, mode="c", nthreads=16)
+
+    def plane(h, w):
+        buf = torch.full((h * (w + pad) + offset,), -1, dtype=torch.int16, device="cuda")
+        return buf, buf[offset:].view(h, w + pad)[:, :w]
+    conv = zg.ResizeConversion(sw, sh, "word").set_depth(10).set_filter(kind).set_dst_width(dw).set_dst_height(dh)
+    r = conv.create()
+    assert r.info["engine"] == "tensor"
+    sbuf, s = plane(sh, sw)
+    host = src[::-1].copy() if flip else src
+    s.copy_(torch.from_numpy(host.view(np.int16)))
+    lib, stream = zg.load(), torch.cuda.current_stream().cuda_stream
+    stride = (sw + pad) * 2
+    sp, ss = (s.data_ptr() + (sh - 1) * stride, -stride) if flip else (s.data_ptr(), stride)
+    dbuf, d = plane(dh, dw)
+    assert lib.zg_resize_process(r.handle, sp, ss, d.data_ptr(), (dw + pad) * 2, None, stream) == 0
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(d.cpu().numpy().view(np.uint16), want)
+    if pad:
+        assert (dbuf[offset:].view(dh, dw + pad)[:, dw:] == -1).all()
+    if not flip:
+        planes = [plane(dh, dw)[1] for _ in range(3)]
+        b = zg.Batch([conv] * 3)
+        b.set_io([s] * 3, planes)
+        b.process()
+        torch.cuda.synchronize()
+        for q in planes:
+            np.testing.assert_array_equal(q.cpu().numpy().view(np.uint16), want)
+
+
 FAULT_CHILD = r"""
 import json, os, sys, time
 import numpy as np

@@ -22,7 +22,8 @@ LIB = os.path.join(OUT_DIR, "libzimg_gb300.so")
 
 SOURCES = ["filter_plan.cpp", "capi.cu", "capi_graph.cu", "capi_batch.cu", "capi_static_tmp.cu",
            "pass_kernels.cu", "fused.cu", "fused_inst_v_f32.cu", "fused_inst_h_f32.cu",
-           "fused_inst_v_i16.cu", "fused_inst_h_i16.cu", "mma.cu", "chain.cu", "chain_tma.cu", "wide_kernel.cu", "wide_umma.cu", "copy_kernel.cu",
+           "fused_inst_v_i16.cu", "fused_inst_h_i16.cu", "mma.cu", "chain.cu", "chain_tma.cu", "chain_any_dst.cu",
+           "chain_lines.cu", "wide_kernel.cu", "wide_umma.cu", "copy_kernel.cu",
            "depth_kernel.cu", "ed_kernel.cu", "alpha_kernel.cu", "capi_depth.cu", "colorspace_plan.cpp",
            "colorspace_kernel.cu", "capi_colorspace.cu", "work_chunks.cpp", "unresize_plan.cpp", "unresize_kernel.cu", "capi_unresize.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]

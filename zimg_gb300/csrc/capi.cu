@@ -426,12 +426,13 @@ zg_error_code zg_resize_create(const zg_resize_params *params, zg_resize **out)
 				FusedPlan *mp = &r->fplan;
 				fused_segment(&mp, 1, fused_wave_items());
 				const FusedPlan *pp = &r->fplan;
-				r->flayout = fused_layout(&pp, 1);
-				r->fgrid = fused_grid_size(r->fplan.variant, static_cast<size_t>(r->flayout.total_bytes));
-				if (r->fplan.chain && chain_tma_enabled()) {
-					r->tma = chain_tma_layout(&pp, 1, &r->tlayout);
-					if (r->tma)
-						r->tgrid = chain_tma_grid_size(r->fplan.variant, static_cast<size_t>(r->tlayout.total_bytes));
+				if (r->fplan.chain) {
+					if (!chain_tma_layout(&pp, 1, &r->flayout))
+						throw Error(kErrUnknown, "chained plan without a layout");
+					r->fgrid = chain_tma_grid_size(r->fplan.variant, static_cast<size_t>(r->flayout.total_bytes));
+				} else {
+					r->flayout = fused_layout(&pp, 1);
+					r->fgrid = fused_grid_size(r->fplan.variant, static_cast<size_t>(r->flayout.total_bytes));
 				}
 				r->fused = true;
 				r->tmp_size = 0;
@@ -528,10 +529,10 @@ void resize_planes(const ResizeIo *io, int n, cudaStream_t st)
 		// launch (the tensor-core kernels of variants 100-199 take one)
 		FewJobs few{};
 		const FusedPlan *plans[kFewJobs];
-		int count = 0, items = 0, grid = r->tma ? r->tgrid : r->fgrid;
+		int count = 0, items = 0, grid = r->fgrid;
 		for (int b = a; b < n; ++b) {
 			const zg_resize *q = io[b].r;
-			if (done[b] || !q->fused || q->fplan.variant != r->fplan.variant || q->tma != r->tma ||
+			if (done[b] || !q->fused || q->fplan.variant != r->fplan.variant ||
 			    (b > a && r->fplan.mma && !r->fplan.chain))
 				continue;
 			done[b] = true;
@@ -540,23 +541,22 @@ void resize_planes(const ResizeIo *io, int n, cudaStream_t st)
 			fused_set_io(j, io[b].src, io[b].src_stride, io[b].dst, io[b].dst_stride);
 			j.item_begin = items;
 			items += fused_items(j);
-			grid = std::min(grid, r->tma ? q->tgrid : q->fgrid);
+			grid = std::min(grid, q->fgrid);
 			plans[count++] = &q->fplan;
 		}
-		if (r->tma) {
-			SmemLayout L = r->tlayout;
+		if (r->fplan.chain) {
+			SmemLayout L = r->flayout;
 			FewMaps maps;
-			bool mapped = count == 1 || chain_tma_layout(plans, count, &L);
+			bool mapped = true;
+			if (count > 1 && !chain_tma_layout(plans, count, &L))
+				throw Error(kErrUnknown, "chained plans without a layout");
 			for (int k = 0; k < count && mapped; ++k)
 				mapped = chain_tma_source_map(&maps.map[k], few.job[k], L);
-			if (mapped) {
-				cuda_check(launch_chain_tma(r->fplan.variant, nullptr, count, items, nullptr, L, grid, few, &maps, st),
-				           "fused resize launch");
-				continue;
-			}
+			cuda_check(launch_chain_tma(r->fplan.variant, chain_form(few.job, count, mapped), nullptr, count, items, nullptr,
+			                            L, grid, few, mapped ? &maps : nullptr, st),
+			           "fused resize launch");
+			continue;
 		}
-		if (r->tma)
-			grid = r->fgrid;
 		cuda_check(launch_fused(r->fplan.variant, nullptr, count, items, count == 1 ? r->flayout : fused_layout(plans, count),
 		                        grid, few, st),
 		           "fused resize launch");

@@ -24,12 +24,8 @@ struct zg_batch {
 		int first;  // first entry in the device job table
 		int count;
 		int tiles;
-		// chained groups: the TMA-pipelined kernel, when every source plane
-		// of the group has a tensor map (decided at each io upload)
-		bool tma_plan = false;
-		bool tma_now = false;
-		SmemLayout tlayout{};
-		int tgrid = 0;
+		bool chain = false;  // the chained kernel,
+		ChainForm form = ChainForm::LINES;  // in the form that its planes admit (decided at each io upload)
 		int ranges_off = -1;  // CTA unit ranges in ranges_dev (ints), or -1
 		// guided chunks (CUDA-core streaming groups): bounds at chunks_off in
 		// chunks_dev, num_chunks chunks, the counter pair at `sched` in
@@ -52,7 +48,7 @@ struct zg_batch {
 	DeviceBuffer sched_dev;  // two words per group (zero between launches)
 	std::vector<FusedJob> table_host;
 	DeviceBuffer table_dev;
-	std::vector<CUtensorMap> maps_host;  // per table entry (chained TMA groups)
+	std::vector<CUtensorMap> maps_host;  // per table entry (chained groups' source planes that admit one)
 	DeviceBuffer maps_dev;
 	// identity conversions: one batched copy launch
 	std::vector<int> copy_jobs;
@@ -61,7 +57,7 @@ struct zg_batch {
 	unsigned long long copy_chunks = 0;
 	// one launch for the chained groups and the identity copies together
 	// (chain_mixed_kernel), when every chained job's source plane has a
-	// tensor map: its own job table, tensor maps and per-CTA unit ranges
+	// tensor map: its own job table, tensor maps and work chunks
 	bool mixed_plan = false;
 	bool mixed_now = false;
 	SmemLayout mixed_layout{};
@@ -138,20 +134,20 @@ void batch_launch(const zg_batch *b, void *tmp, cudaStream_t st)
 		});
 	}
 	for (const auto &g : b->groups) {
-		if (b->mixed_now && g.tma_plan)
+		if (b->mixed_now && g.chain)
 			continue;  // in the mixed launch
 		const int *ranges = g.ranges_off < 0 ? nullptr : static_cast<const int *>(b->ranges_dev.get()) + g.ranges_off;
 		WorkChunks c;
-		if (!g.tma_now && g.num_chunks > 0) {
+		if (!g.chain && g.num_chunks > 0) {
 			c.bounds = static_cast<const int *>(b->chunks_dev.get()) + g.chunks_off;
 			c.num = g.num_chunks;
 			c.sched = static_cast<unsigned *>(b->sched_dev.get()) + g.sched;
 		}
 		work.push_back([&g, table, ranges, c](cudaStream_t s) {
 			FewJobs unused{};
-			if (g.tma_now)
-				cuda_check(launch_chain_tma(g.variant, table + g.first, g.count, g.tiles, ranges, g.tlayout, g.tgrid,
-				                            unused, nullptr, s),
+			if (g.chain)
+				cuda_check(launch_chain_tma(g.variant, g.form, table + g.first, g.count, g.tiles, ranges, g.layout,
+				                            g.grid, unused, nullptr, s),
 				           "fused batch launch");
 			else
 				cuda_check(launch_fused(g.variant, table + g.first, g.count, g.tiles, g.layout, g.grid, unused, s, c),
@@ -251,10 +247,10 @@ double unit_cost(const zg_resize *r, const FusedJob &j, bool copy)
 	return bytes / units / eff;
 }
 
-// The mixed launch (chain_mixed_kernel): every chained group whose layout
-// admits the TMA form and every identity copy in one persistent launch, the
-// units of each CTA balanced by estimated cost. Decided per plan here; used
-// when every source plane also has a tensor map (upload_io).
+// The mixed launch (chain_mixed_kernel): every chained group and every
+// identity copy in one persistent launch, the units of each CTA balanced by
+// estimated cost. Decided per plan here; used when every source plane also
+// has a tensor map (upload_io).
 void plan_mixed(zg_batch *b)
 {
 	b->mixed_plan = false;
@@ -266,24 +262,24 @@ void plan_mixed(zg_batch *b)
 	b->mixed_ranges_dev.release();
 	b->mixed_sched_dev.release();
 	b->mixed_chunks = 0;
-	if (!chain_tma_enabled())
-		return;
 	std::vector<const FusedPlan *> plans;
 	int chained_groups = 0;
+	bool taken = chain_tma_enabled();
 	for (const auto &g : b->groups) {
-		if (!g.tma_plan)
+		if (!g.chain)
 			continue;
 		++chained_groups;
 		for (int e = g.first; e < g.first + g.count; ++e) {
 			for (size_t i = 0; i < b->jobs.size(); ++i)
 				if (b->table_index[i] == e) {
 					plans.push_back(&b->jobs[i]->fplan);
+					taken = taken && chain_mixed_takes(b->jobs[i]->fplan.job);
 					b->mixed_jobs.push_back(static_cast<int>(i));
 				}
 		}
 	}
 	// worth one launch when it replaces more than one
-	if (plans.empty() || chained_groups + (b->copy_jobs.empty() ? 0 : 1) < 2 ||
+	if (!taken || plans.empty() || chained_groups + (b->copy_jobs.empty() ? 0 : 1) < 2 ||
 	    !chain_tma_layout(plans.data(), static_cast<int>(plans.size()), &b->mixed_layout)) {
 		b->mixed_jobs.clear();
 		return;
@@ -386,26 +382,27 @@ void regroup(zg_batch *b)
 			b->table_host.push_back(j);
 			++g.count;
 		}
-		g.layout = fused_layout(plans.data(), static_cast<int>(plans.size()));
-		g.grid = fused_grid_size(g.variant, static_cast<size_t>(g.layout.total_bytes));
-		if (plans[0]->chain && chain_tma_enabled()) {
-			g.tma_plan = chain_tma_layout(plans.data(), static_cast<int>(plans.size()), &g.tlayout);
-			if (g.tma_plan) {
-				g.tgrid = chain_tma_grid_size(g.variant, static_cast<size_t>(g.tlayout.total_bytes));
-				// jobs of one shape with at least a strip per CTA: strips in
-				// step across neighbouring CTAs
-				bool same = true;
-				for (unsigned i : kv.second)
-					same = same && b->jobs[i]->fplan.job.groups == b->jobs[kv.second[0]]->fplan.job.groups;
-				const char *order = std::getenv("ZG_CHAIN_ORDER");
-				const bool lockstep = !(order && std::string(order) == "equal");
-				const std::vector<int> r = same && lockstep ? chain_tma_lockstep_ranges(
-				                                                  g.tiles, b->jobs[kv.second[0]]->fplan.job.groups, g.tgrid)
-				                                            : std::vector<int>();
-				if (!r.empty()) {
-					g.ranges_off = static_cast<int>(b->ranges_host.size());
-					b->ranges_host.insert(b->ranges_host.end(), r.begin(), r.end());
-				}
+		g.chain = plans[0]->chain;
+		if (!g.chain) {
+			g.layout = fused_layout(plans.data(), static_cast<int>(plans.size()));
+			g.grid = fused_grid_size(g.variant, static_cast<size_t>(g.layout.total_bytes));
+		} else {
+			if (!chain_tma_layout(plans.data(), static_cast<int>(plans.size()), &g.layout))
+				throw Error(kErrUnknown, "chained plans without a layout");
+			g.grid = chain_tma_grid_size(g.variant, static_cast<size_t>(g.layout.total_bytes));
+			// jobs of one shape with at least a strip per CTA: strips in step
+			// across neighbouring CTAs
+			bool same = true;
+			for (unsigned i : kv.second)
+				same = same && b->jobs[i]->fplan.job.groups == b->jobs[kv.second[0]]->fplan.job.groups;
+			const char *order = std::getenv("ZG_CHAIN_ORDER");
+			const bool lockstep = !(order && std::string(order) == "equal");
+			const std::vector<int> r = same && lockstep ? chain_tma_lockstep_ranges(
+			                                                  g.tiles, b->jobs[kv.second[0]]->fplan.job.groups, g.grid)
+			                                            : std::vector<int>();
+			if (!r.empty()) {
+				g.ranges_off = static_cast<int>(b->ranges_host.size());
+				b->ranges_host.insert(b->ranges_host.end(), r.begin(), r.end());
 			}
 		}
 		// CUDA-core streaming groups: guided chunks of the group's units (cost
@@ -502,12 +499,13 @@ void upload_io(zg_batch *b, cudaStream_t st)
 	// tensor maps of the chained groups' source planes
 	bool any_map = false;
 	for (auto &g : b->groups) {
-		g.tma_now = g.tma_plan;
-		for (int e = g.first; g.tma_now && e < g.first + g.count; ++e)
-			g.tma_now = chain_tma_source_map(&b->maps_host[e], b->table_host[e], g.tlayout);
+		bool mapped = g.chain;
+		for (int e = g.first; mapped && e < g.first + g.count; ++e)
+			mapped = chain_tma_source_map(&b->maps_host[e], b->table_host[e], g.layout);
 		for (int e = g.first; e < g.first + g.count; ++e)
-			b->table_host[e].tmap = g.tma_now ? static_cast<const CUtensorMap *>(b->maps_dev.get()) + e : nullptr;
-		any_map = any_map || g.tma_now;
+			b->table_host[e].tmap = mapped ? static_cast<const CUtensorMap *>(b->maps_dev.get()) + e : nullptr;
+		g.form = chain_form(b->table_host.data() + g.first, g.count, mapped);
+		any_map = any_map || mapped;
 	}
 	if (any_map)
 		cuda_check(cudaMemcpyAsync(b->maps_dev.get(), b->maps_host.data(), b->maps_host.size() * sizeof(CUtensorMap),
@@ -826,7 +824,7 @@ zg_error_code zg_batch_get_launch_count(const zg_batch *b, unsigned *out)
 			// one launch for the chained groups and the copies; other groups apart
 			n = 1;
 			for (const auto &g : b->groups)
-				n += g.tma_plan ? 0u : 1u;
+				n += g.chain ? 0u : 1u;
 		} else {
 			n = static_cast<unsigned>(b->groups.size()) + (b->copy_jobs.empty() ? 0u : 1u);
 		}

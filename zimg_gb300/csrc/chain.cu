@@ -1,5 +1,4 @@
-// Host planning and launch of the chained tensor-core u16 kernel
-// (chain_kernel.cuh), plus its instantiations.
+// Host planning of the chained tensor-core u16 kernel (chain_tma_kernel.cuh).
 #include "chain_kernel.cuh"
 #include "fused.h"
 
@@ -12,9 +11,9 @@ namespace zg {
 
 namespace {
 
-constexpr size_t kChainSmemMax = 110 * 1024;  // two CTAs per SM
 constexpr int kChainKVMax = 3;
 constexpr int kChainKHMax = 4;
+constexpr int kChainWindow = 248;  // samples of a strip's lines
 
 size_t align_up(size_t x, size_t a)
 {
@@ -161,24 +160,34 @@ bool plan_chain(const FilterTable &first, const FilterTable &second, bool h_firs
 	if (KH < 1 || KH > kChainKHMax)
 		return false;
 
-	// strips of 8 warps' tiles; source columns [lo, hi) with lo a multiple of 8
-	const int strip_tiles = chain_detail::warps_per_cta(h_first) * chain_detail::tiles_per_warp(KV, KH);
-	const int strip_w = strip_tiles * chain_detail::kTileW;
-	const int strips = static_cast<int>((dst_w + strip_w - 1) / strip_w);
-	std::vector<int> win_col(2 * strips);
-	int max_pxa = 0;
-	for (int s = 0; s < strips; ++s) {
-		const int t0 = s * strip_tiles, t1 = std::min(tiles, t0 + strip_tiles);
-		int lo = INT_MAX, hi = INT_MIN;
-		for (int t = t0; t < t1; ++t) {
-			lo = std::min(lo, hstart[t]);
-			hi = std::max(hi, hstart[t] + 16 * KH);
+	// strips of up to 7 warps' tiles whose source columns [lo, hi), lo a
+	// multiple of 8, fit the widest window that both ways of copying lines
+	// take (31 chunks of 16 bytes for a warp; a tensor copy's 256 samples)
+	const int per_warp = chain_detail::tiles_per_warp(KV, KH);
+	int strip_tiles = chain_detail::warps_per_cta(h_first) * per_warp, strips = 0, max_pxa = 0;
+	std::vector<int> win_col;
+	for (; strip_tiles >= per_warp; strip_tiles -= per_warp) {
+		strips = (tiles + strip_tiles - 1) / strip_tiles;
+		win_col.assign(2 * strips, 0);
+		max_pxa = 0;
+		for (int s = 0; s < strips; ++s) {
+			const int t0 = s * strip_tiles, t1 = std::min(tiles, t0 + strip_tiles);
+			int lo = INT_MAX, hi = INT_MIN;
+			for (int t = t0; t < t1; ++t) {
+				lo = std::min(lo, hstart[t]);
+				hi = std::max(hi, hstart[t] + 16 * KH);
+			}
+			lo = lo / 8 * 8;
+			win_col[2 * s] = lo;
+			win_col[2 * s + 1] = hi;
+			max_pxa = std::max(max_pxa, (hi - lo + 7) & ~7);
 		}
-		lo = lo / 8 * 8;
-		win_col[2 * s] = lo;
-		win_col[2 * s + 1] = hi;
-		max_pxa = std::max(max_pxa, (hi - lo + 7) & ~7);
+		if (max_pxa <= kChainWindow)
+			break;
 	}
+	if (strip_tiles < per_warp)
+		return false;
+	const int strip_w = strip_tiles * chain_detail::kTileW;
 
 	// prefetch depth: about 32 KB of source lines in flight per CTA
 	auto hi_of = [&](int g) { return gbase[std::min(g, groups - 1)] + 16 * KV; };
@@ -218,7 +227,8 @@ bool plan_chain(const FilterTable &first, const FilterTable &second, bool h_firs
 		p.mma = true;
 		p.chain = true;
 		const FusedPlan *pp = &p;
-		if (static_cast<size_t>(chain_layout(&pp, 1).total_bytes) <= kChainSmemMax) {
+		SmemLayout layout;
+		if (chain_tma_layout(&pp, 1, &layout)) {
 			fits = true;
 			break;
 		}
@@ -294,101 +304,6 @@ bool plan_chain(const FilterTable &first, const FilterTable &second, bool h_firs
 	}
 	p.reuse_frac = groups > 1 ? static_cast<float>(kept / (groups - 1)) : 0.0f;
 	return true;
-}
-
-SmemLayout chain_layout(const FusedPlan *const *plans, int n)
-{
-	int max_pxa = 0, in = 1, seg_groups = 1, depth = 1, kv = 1, tiles = 1;
-	for (int i = 0; i < n; ++i) {
-		const FusedPlan &p = *plans[i];
-		max_pxa = std::max(max_pxa, p.max_pxa);
-		in = std::max(in, p.job.in_rows);
-		seg_groups = std::max(seg_groups, p.job.groups);  // an item spans up to a whole strip
-		depth = std::max(depth, p.depth);
-		kv = std::max(kv, p.job.vs);
-		tiles = std::max(tiles, chain_detail::tiles_per_warp(p.job.vs, p.job.hw));
-	}
-	auto a16 = [](size_t x) { return static_cast<int>((x + 15) / 16 * 16); };
-	SmemLayout L{};
-	// lines at 16 mod 32 bytes: the 8 rows of an ldmatrix phase fall in 8
-	// different 16-byte bank groups, and 4-byte fragment loads of 8 lines x 4
-	// pairs in 32 different banks
-	L.pitch = (max_pxa + 15) / 16 * 16 + 8;
-	L.in_rows = in;
-	L.ring_rows = 1;
-	L.stage_rows = 1;
-	L.seg_groups = seg_groups;
-	L.step_groups = 1;
-	L.depth = depth;
-	int off = 0;
-	L.in_off = off;
-	off += a16(static_cast<size_t>(in) * L.pitch * 2);
-	L.vcoef_off = off;
-	off += a16(static_cast<size_t>(depth + 2) * kv * 2 * 32 * 16);
-	L.tile_off = off;
-	L.tile_pitch = chain_detail::kStageBytes / 2;
-	off += a16(static_cast<size_t>(chain_detail::kMaxWarps) * tiles * chain_detail::kTileStage);
-	L.vbase_off = off;
-	off += a16(static_cast<size_t>(seg_groups) * 4);
-	L.ring_off = L.stage_off = L.i_off = L.htaps_off = L.hleft_off = off;
-	L.total_bytes = off;
-	return L;
-}
-
-namespace {
-
-template <bool HF, int KV, int KH>
-const void *chain_ptr()
-{
-	return reinterpret_cast<const void *>(&chain_detail::chain_kernel<HF, KV, KH>);
-}
-
-template <bool HF, int KV>
-const void *chain_ptr_kh(int kh)
-{
-	switch (kh) {
-	case 1: return chain_ptr<HF, KV, 1>();
-	case 2: return chain_ptr<HF, KV, 2>();
-	case 3: return chain_ptr<HF, KV, 3>();
-	default: return chain_ptr<HF, KV, 4>();
-	}
-}
-
-template <bool HF>
-const void *chain_ptr_kv(int kv, int kh)
-{
-	return kv == 1 ? chain_ptr_kh<HF, 1>(kh) : (kv == 2 ? chain_ptr_kh<HF, 2>(kh) : chain_ptr_kh<HF, 3>(kh));
-}
-
-} // namespace
-
-const void *chain_kernel_ptr(int variant)
-{
-	const int v = variant - 200;
-	const int per = kChainKVMax * kChainKHMax;
-	const bool hf = v >= per;
-	const int kv = (v % per) / kChainKHMax + 1, kh = v % kChainKHMax + 1;
-	return hf ? chain_ptr_kv<true>(kv, kh) : chain_ptr_kv<false>(kv, kh);
-}
-
-int chain_threads(int variant)
-{
-	const bool hf = variant - 200 >= kChainKVMax * kChainKHMax;
-	return chain_detail::warps_per_cta(hf) * 32;
-}
-
-cudaError_t launch_chain(int variant, const FusedJob *jobs, int num_jobs, int total_items, const SmemLayout &L, int grid,
-                         const FewJobs &few, cudaStream_t stream)
-{
-	if (L.total_bytes > static_cast<int>(kChainSmemMax))
-		return cudaErrorInvalidValue;
-	const void *k = chain_kernel_ptr(variant);
-	FewJobs by_value = few;
-	SmemLayout layout = L;
-	void *args[] = { &jobs, &num_jobs, &total_items, &by_value, &layout };
-	grid = std::max(1, std::min(grid, total_items));
-	return cudaLaunchKernel(k, dim3(grid), dim3(chain_threads(variant)), args, static_cast<size_t>(L.total_bytes),
-	                        stream);
 }
 
 } // namespace zg

@@ -1,7 +1,6 @@
 // Host side of the TMA-pipelined chained kernel (chain_tma_kernel.cuh):
 // shared-memory layout, source tensor maps, launch, instantiations.
-#include "chain_tma_kernel.cuh"
-#include "fused.h"
+#include "chain_inst.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -11,11 +10,74 @@
 
 namespace zg {
 
+namespace chain_detail {
+
+// Variant codes of mixed launches: the chained kernel's variant - 200
+// (H first, KV, KH), or kCopyVariant for an identity plane.
+constexpr int kCopyVariant = 1000;
+
+// One launch over a batch of mixed jobs: every chained variant and identity
+// copies. CTAs take chunks of units from a counter (guided sizes, cut by the
+// host from estimated costs: large chunks first, small ones last, so that
+// the CTAs end together); an item is dispatched on its job's variant.
+__global__ void __launch_bounds__(tma_threads(true), 2)
+chain_mixed_kernel(const FusedJob *__restrict__ jobs, int num_jobs, const __grid_constant__ WorkChunks C,
+                   const __grid_constant__ SmemLayout L)
+{
+	extern __shared__ float4 smem4[];
+	__shared__ int abort_item;
+	__shared__ int chunk;
+	Pipe p;
+	pipe_init(p, smem4, L, &abort_item);
+	// chunks in the order CTAs ask for them (guided sizes: large first)
+	for (;;) {
+		const int m = next_chunk(C, &chunk);
+		if (m < 0 || abort_item)
+			break;
+		const int t_end = __ldg(C.bounds + m + 1);
+		for (int t = __ldg(C.bounds + m); t < t_end;) {
+			const FusedJob &J = jobs[find_job(jobs, num_jobs, t)];
+			const int local = t - J.item_begin;
+			const int strip = local / J.groups;
+			const int g_begin = local - strip * J.groups;
+			const int ngroups = min(J.groups - g_begin, t_end - t);
+			t += ngroups;
+			const int v = J.variant;
+			if (v == kCopyVariant) {
+				copy_item(J, g_begin, ngroups);
+			} else {
+				load_bases(p, J, g_begin, ngroups);
+				switch (v) {
+#define ZG_CHAIN_CASE(HF, KV, KH)                                                                     \
+	case (HF ? 12 : 0) + (KV - 1) * 4 + (KH - 1):                                                      \
+		chain_item<HF, KV, KH, false, ChainForm::ALIGNED>(p, L, J, J.tmap, strip, g_begin, ngroups);  \
+		break;
+					ZG_CHAIN_CASE(true, 1, 1) ZG_CHAIN_CASE(true, 1, 2) ZG_CHAIN_CASE(true, 1, 3) ZG_CHAIN_CASE(true, 1, 4)
+					ZG_CHAIN_CASE(true, 2, 1) ZG_CHAIN_CASE(true, 2, 2) ZG_CHAIN_CASE(true, 2, 3) ZG_CHAIN_CASE(true, 2, 4)
+					ZG_CHAIN_CASE(true, 3, 1) ZG_CHAIN_CASE(true, 3, 2) ZG_CHAIN_CASE(true, 3, 3) ZG_CHAIN_CASE(true, 3, 4)
+					ZG_CHAIN_CASE(false, 1, 1) ZG_CHAIN_CASE(false, 1, 2) ZG_CHAIN_CASE(false, 1, 3) ZG_CHAIN_CASE(false, 1, 4)
+					ZG_CHAIN_CASE(false, 2, 1) ZG_CHAIN_CASE(false, 2, 2) ZG_CHAIN_CASE(false, 2, 3) ZG_CHAIN_CASE(false, 2, 4)
+					ZG_CHAIN_CASE(false, 3, 1) ZG_CHAIN_CASE(false, 3, 2) ZG_CHAIN_CASE(false, 3, 3) ZG_CHAIN_CASE(false, 3, 4)
+#undef ZG_CHAIN_CASE
+				default:
+					break;
+				}
+			}
+			p.base += J.variant == kCopyVariant ? 0 : ngroups;
+			__syncthreads();  // the next item rewrites the group bases and the ring
+			if (abort_item)
+				break;
+		}
+	}
+	pipe_finish(p);
+	chunks_finish(C);  // the last CTA out leaves the counter zero for the next launch
+}
+
+} // namespace chain_detail
+
 namespace {
 
 constexpr size_t kTmaSmemMax = 110 * 1024;  // two CTAs per SM
-constexpr int kKVMax = 3;
-constexpr int kKHMax = 4;
 constexpr int kMaxBoxW = 256;               // tensor-copy box limit per dimension
 constexpr int kAlignSlack = 128;            // the kernel aligns its shared-memory base to 128 bytes
 
@@ -38,29 +100,6 @@ EncodeTiled encoder()
 	return fn;
 }
 
-template <bool HF, int KV, int KH>
-const void *tma_ptr()
-{
-	return reinterpret_cast<const void *>(&chain_detail::chain_tma_kernel<HF, KV, KH>);
-}
-
-template <bool HF, int KV>
-const void *tma_ptr_kh(int kh)
-{
-	switch (kh) {
-	case 1: return tma_ptr<HF, KV, 1>();
-	case 2: return tma_ptr<HF, KV, 2>();
-	case 3: return tma_ptr<HF, KV, 3>();
-	default: return tma_ptr<HF, KV, 4>();
-	}
-}
-
-template <bool HF>
-const void *tma_ptr_kv(int kv, int kh)
-{
-	return kv == 1 ? tma_ptr_kh<HF, 1>(kh) : (kv == 2 ? tma_ptr_kh<HF, 2>(kh) : tma_ptr_kh<HF, 3>(kh));
-}
-
 int tma_threads(int variant)
 {
 	return chain_detail::tma_threads(variant - 200 >= kKVMax * kKHMax);
@@ -68,19 +107,25 @@ int tma_threads(int variant)
 
 } // namespace
 
-const void *chain_tma_kernel_ptr(int variant)
+const ChainKernels kChainAligned = { form_ptr<ChainForm::ALIGNED>, form_set_fault, form_error };
+
+namespace {
+
+const ChainKernels *const kForms[] = { &kChainAligned, &kChainAnyDst, &kChainLines };
+
+// A strip of the full width of its variant.
+bool full_strip(const FusedJob &j)
 {
-	const int v = variant - 200;
-	const int per = kKVMax * kKHMax;
-	const bool hf = v >= per;
-	const int kv = (v % per) / kKHMax + 1, kh = v % kKHMax + 1;
-	return hf ? tma_ptr_kv<true>(kv, kh) : tma_ptr_kv<false>(kv, kh);
+	const int tiles = chain_detail::tiles_per_warp(j.variant % (kKVMax * kKHMax) / kKHMax + 1, j.variant % kKHMax + 1);
+	return j.strip_w == chain_detail::kWsWarps * tiles * chain_detail::kTileW;
 }
+
+} // namespace
 
 bool chain_tma_enabled()
 {
-	// the default where the source planes admit a tensor map; ZG_CHAIN_TMA=0
-	// keeps the cp.async form
+	// tensor copies where the source planes admit a tensor map;
+	// ZG_CHAIN_TMA=0: every plane by the producer warp's loads
 	static const bool on = [] {
 		const char *e = std::getenv("ZG_CHAIN_TMA");
 		return !(e && e[0] == '0');
@@ -171,7 +216,7 @@ bool encode_tensor_map_2d(CUtensorMap *map, CUtensorMapDataType type, const void
 bool chain_tma_source_map(CUtensorMap *map, const FusedJob &j, const SmemLayout &L)
 {
 	const uintptr_t a = reinterpret_cast<uintptr_t>(j.src);
-	if (!j.src || a % 16 || j.src_stride <= 0 || j.src_stride % 16 || j.src_w < 1 || j.src_h < 1)
+	if (!chain_tma_enabled() || !j.src || a % 16 || j.src_stride <= 0 || j.src_stride % 16 || j.src_w < 1 || j.src_h < 1)
 		return false;
 	if (L.pitch > kMaxBoxW || (L.pitch * 2) % 16)
 		return false;
@@ -187,26 +232,42 @@ bool chain_tma_source_map(CUtensorMap *map, const FusedJob &j, const SmemLayout 
 	          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+ChainForm chain_form(const FusedJob *jobs, int n, bool mapped)
+{
+	if (!mapped)
+		return ChainForm::LINES;
+	for (int i = 0; i < n; ++i)
+		if (jobs[i].dst_align != 16 || !full_strip(jobs[i]))
+			return ChainForm::ANY_DST;
+	return ChainForm::ALIGNED;
+}
+
+bool chain_mixed_takes(const FusedJob &j)
+{
+	return full_strip(j);
+}
+
 int chain_tma_grid_size(int variant, size_t smem_bytes)
 {
 	int dev = 0, sms = 0, per_sm = 0;
 	cudaGetDevice(&dev);
 	cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-	const void *k = chain_tma_kernel_ptr(variant);
-	cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kTmaSmemMax));
-	if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, tma_threads(variant), smem_bytes) != cudaSuccess ||
+	for (const ChainKernels *f : kForms)
+		cudaFuncSetAttribute(f->ptr(variant), cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kTmaSmemMax));
+	if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kChainAligned.ptr(variant), tma_threads(variant),
+	                                                  smem_bytes) != cudaSuccess ||
 	    per_sm < 1)
 		per_sm = 1;
 	return std::max(1, sms) * per_sm;
 }
 
-cudaError_t launch_chain_tma(int variant, const FusedJob *jobs, int num_jobs, int total_items, const int *ranges,
+cudaError_t launch_chain_tma(int variant, ChainForm form, const FusedJob *jobs, int num_jobs, int total_items, const int *ranges,
                              const SmemLayout &L, int grid, const FewJobs &few, const FewMaps *few_maps,
                              cudaStream_t stream)
 {
-	if (static_cast<size_t>(L.total_bytes) > kTmaSmemMax || (!jobs && !few_maps))
+	if (static_cast<size_t>(L.total_bytes) > kTmaSmemMax)
 		return cudaErrorInvalidValue;
-	const void *k = chain_tma_kernel_ptr(variant);
+	const void *k = kForms[static_cast<int>(form)]->ptr(variant);
 	FewJobs by_value = few;
 	SmemLayout layout = L;
 	FewMaps maps{};
@@ -272,22 +333,21 @@ cudaError_t launch_chain_mixed(const FusedJob *jobs, int num_jobs, const WorkChu
 
 int chain_tma_set_fault(int drop_group, unsigned long long wait_ns)
 {
-	if (cudaMemcpyToSymbol(chain_detail::g_chain_drop_group, &drop_group, sizeof(drop_group)) != cudaSuccess ||
-	    cudaMemcpyToSymbol(chain_detail::g_chain_wait_ns, &wait_ns, sizeof(wait_ns)) != cudaSuccess)
-		return -1;
+	for (const ChainKernels *f : kForms)
+		if (f->set_fault(drop_group, wait_ns))
+			return -1;
 	return 0;
 }
 
 int chain_tma_pipeline_error(bool reset)
 {
-	int v = 0;
-	if (cudaMemcpyFromSymbol(&v, chain_detail::g_chain_pipeline_error, sizeof(v)) != cudaSuccess)
-		return -1;
-	if (reset && v) {
-		const int zero = 0;
-		cudaMemcpyToSymbol(chain_detail::g_chain_pipeline_error, &zero, sizeof(zero));
+	int first = 0;
+	for (const ChainKernels *f : kForms) {
+		const int v = f->error(reset);
+		if (v && !first)
+			first = v;
 	}
-	return v;
+	return first;
 }
 
 } // namespace zg

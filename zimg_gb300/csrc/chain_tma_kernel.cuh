@@ -1,19 +1,43 @@
-// Chained tensor-core u16 kernel, warp-specialised TMA form.
+// Chained tensor-core u16 kernel, warp-specialised.
 //
-// Arithmetic is that of chain_kernel.cuh (re-centred fp16 samples, int16
-// taps split into two exact fp16 halves, fp32 accumulators that the planner
-// proved hold exact integers, zimg's rounding and clamping per pass,
-// resize_impl.cpp:31-59,78-95), and so are the 16x16 output tiles, the tap
-// fragments and the strip plan. What differs is the feeding and the control
-// flow, cut to the few instructions a tile needs:
+// Arithmetic: chain_kernel.cuh (re-centred fp16 samples, int16 taps split
+// into two exact fp16 halves, fp32 accumulators that the planner proved hold
+// exact integers, zimg's rounding and clamping per pass,
+// resize_impl.cpp:31-59,78-95); the feeding and the control flow are cut to
+// the few instructions a tile needs:
 //
-//  - One producer warp (one lane) brings every group's data into shared
-//    memory: 16-line blocks of the strip's source columns as 2-D tensor
-//    copies (cp.async.bulk.tensor) into a ring of 2^n blocks, and the group's
-//    vertical tap fragments as one bulk copy into a stage. Group g of the
-//    CTA's pipeline uses stage g mod NS: a "full" mbarrier whose transaction
-//    count covers the group's copies, and an "empty" mbarrier on which every
-//    consumer warp arrives once it has read the group.
+//  - One producer warp brings every group's data into shared memory: 16-line
+//    blocks of the strip's source columns into a ring of 2^n blocks, and the
+//    group's vertical tap fragments as one bulk copy into a stage. Group g of
+//    the CTA's pipeline uses stage g mod NS: a "full" mbarrier whose
+//    transaction count covers the group's copies, and an "empty" mbarrier on
+//    which every consumer warp arrives once it has read the group.
+//    Source planes that admit a tensor map (16-byte aligned base and stride)
+//    are copied by one lane, a 2-D tensor copy (cp.async.bulk.tensor) per
+//    block (forms ALIGNED and ANY_DST). The lines of any other plane start
+//    anywhere in a 16-byte chunk (form LINES): every warp takes lines of an
+//    item's first blocks (fill_first), then the producer warp alone loads the
+//    aligned chunks of a block while the block before it is in its slot, asks
+//    L2 for a later one, and moves them into place with a funnel shift when
+//    the slot is free (produce_lines).
+//  - Results leave as 16-byte rows; ANY_DST and LINES also store to planes
+//    that are not 16-byte aligned, consecutive lanes along a row
+//    (store_words). ALIGNED leaves that code out: with it in, the aligned
+//    cases took 2 to 3 % longer. Without it (the mixed launch) such planes
+//    are stored sample by sample.
+//    Measured, 10-bit planes, before (unaligned sources in a kernel of its
+//    own, its computing warps copying sample by sample; sample-wise stores)
+//    and now:
+//      50 of 1918x1080 -> 1278x720     438 -> 241 us   (LINES)
+//      50 of 1919x1079 -> 1279x719     447 -> 256 us   (LINES)
+//      50 of 1279x719 -> 1919x1079     502 -> 199 us   (LINES)
+//      one of 641x361 -> 1279x719      8.9 -> 7.8 us   (LINES)
+//      50 of 1920x1080 -> 1278x720     301 -> 126 us   (ANY_DST)
+//      50 of 1280x720 -> 1918x1080     475 -> 154 us   (ANY_DST)
+//      50 of 1920x1080 -> 1280x720     106 -> 106 us   (ALIGNED)
+//    LINES is bound by its one producer warp: a block's loads, shuffles and
+//    stores one after the other (at 1918x1080 -> 1278x720 the issue slots
+//    were 30 % busy, and waits for loads the longest stall).
 //  - Seven consumer warps only compute and store: per group, one wait, the
 //    vertical fragments, the tiles of the warp (one or two of 16 columns),
 //    one arrive, the stores. Line addresses are ring offsets under a mask,
@@ -46,10 +70,10 @@ constexpr int kWsWarps = warps_per_cta(true);      // consumer warps per CTA
 
 // Nonzero after a pipeline wait ran out: 1 = a group's copies never landed,
 // 2 = a buffer was never released, 3 = ring too small for one group.
-__device__ int g_chain_pipeline_error;
+static __device__ int g_chain_pipeline_error;
 // Wait limit in ns (0: kWaitNs) and the test hook described above (-1: off).
-__device__ unsigned long long g_chain_wait_ns;
-__device__ int g_chain_drop_group = -1;
+static __device__ unsigned long long g_chain_wait_ns;
+static __device__ int g_chain_drop_group = -1;
 
 __host__ __device__ constexpr int tma_threads(bool /*h_first*/)
 {
@@ -326,19 +350,306 @@ __device__ __forceinline__ void pipe_finish(Pipe &p)
 	}
 }
 
+// One block of 16 source lines in a warp's registers: lane k holds the k-th
+// aligned 16-byte chunk of each line's window.
+struct LineBlock {
+	uint4 v[kBlockLines];
+};
+
+// How the producer warp of a kernel without tensor copies sees the source
+// plane and strip of a job.
+struct SoftSource {
+	const char *first;            // sample xlo of line 0
+	ptrdiff_t stride;
+	const char *lo, *hi;          // the plane's bytes
+	int src_h, row_bytes, chunks; // bytes of a line from xlo on; 16-byte chunks of a window
+	uint32_t mask[4];             // samples of this lane's chunk within the line
+};
+
+__device__ __forceinline__ SoftSource soft_source(const FusedJob &J, int strip, int lane)
+{
+	SoftSource s;
+	const int xlo = __ldg(J.win_col + 2 * strip), xhi = __ldg(J.win_col + 2 * strip + 1);
+	const char *src = static_cast<const char *>(J.src);
+	s.first = src + static_cast<ptrdiff_t>(xlo) * 2;
+	s.stride = J.src_stride;
+	const char *last = src + static_cast<ptrdiff_t>(J.src_h - 1) * J.src_stride;
+	s.lo = last < src ? last : src;
+	s.hi = (last < src ? src : last) + static_cast<ptrdiff_t>(J.src_w) * 2;
+	s.src_h = J.src_h;
+	s.row_bytes = (J.src_w - xlo) * 2;
+	s.chunks = ((xhi - xlo) * 2 + 15) / 16;
+#pragma unroll
+	for (int k = 0; k < 4; ++k) {
+		const int x = xlo + lane * 8 + 2 * k;
+		s.mask[k] = (x < J.src_w ? 0xFFFFu : 0u) | (x + 1 < J.src_w ? 0xFFFF0000u : 0u);
+	}
+	return s;
+}
+
+// Block b's window into L2: lane k takes every fourth 128 bytes of two lines.
+__device__ __forceinline__ void prefetch_block(const SoftSource &s, int b, int lane)
+{
+#pragma unroll
+	for (int l = 0; l < kBlockLines; l += 8) {
+		const int y = b * kBlockLines + l + (lane >> 2);
+		const int x = (lane & 3) * 128;
+		if (y < s.src_h && x < s.row_bytes && x < s.chunks * 16)
+			asm volatile("prefetch.global.L2 [%0];\n" ::"l"(s.first + static_cast<ptrdiff_t>(y) * s.stride + x));
+	}
+}
+
+// The chunk at c sample by sample, those outside of the plane zero.
+__device__ __forceinline__ uint4 load_chunk(const SoftSource &s, const char *c)
+{
+	uint32_t w[8];
+#pragma unroll
+	for (int k = 0; k < 8; ++k) {
+		const char *q = c + 2 * k;
+		w[k] = q >= s.lo && q < s.hi ? __ldg(reinterpret_cast<const uint16_t *>(q)) : 0u;
+	}
+	return make_uint4(w[0] | (w[1] << 16), w[2] | (w[3] << 16), w[4] | (w[5] << 16), w[6] | (w[7] << 16));
+}
+
+// Block b's chunks; lines below the plane and chunks beyond a line are zero.
+// In the blocks with the plane's first or last bytes (a test once a block, so
+// that the others' loads issue without a branch between them) a chunk that
+// crosses those is read sample by sample: no access leaves the plane.
+__device__ __forceinline__ void load_block(const SoftSource &s, int b, int lane, LineBlock &blk)
+{
+	const char *row = s.first + static_cast<ptrdiff_t>(b) * kBlockLines * s.stride;
+	const int lines = min(kBlockLines, s.src_h - b * kBlockLines);
+	const char *last = row + static_cast<ptrdiff_t>(lines - 1) * s.stride;
+	const bool inside = (row < last ? row : last) - 15 >= s.lo && (row < last ? last : row) + s.row_bytes + 15 <= s.hi;
+	if (inside) {
+#pragma unroll
+		for (int l = 0; l < kBlockLines; ++l, row += s.stride) {
+			const int at = lane * 16 - (static_cast<int>(reinterpret_cast<uintptr_t>(row)) & 15);
+			blk.v[l] = make_uint4(0, 0, 0, 0);
+			if (l < lines && lane <= s.chunks && at < s.row_bytes)
+				blk.v[l] = __ldg(reinterpret_cast<const uint4 *>(row + at));
+		}
+		return;
+	}
+#pragma unroll
+	for (int l = 0; l < kBlockLines; ++l, row += s.stride) {
+		const char *c = row - (reinterpret_cast<uintptr_t>(row) & 15) + lane * 16;
+		blk.v[l] = make_uint4(0, 0, 0, 0);
+		if (l < lines && lane <= s.chunks && c < row + s.row_bytes)
+			blk.v[l] = load_chunk(s, c);
+	}
+}
+
+// A line's chunks (v, of the line at `row`) moved down to sample xlo by the
+// offset of its start in a chunk, an even number of bytes, the same for the
+// warp; samples beyond the line cleared.
+__device__ __forceinline__ void store_line(const SoftSource &s, const char *row, const uint4 &v, int lane, char *to)
+{
+	const unsigned shift = static_cast<unsigned>(reinterpret_cast<uintptr_t>(row)) & 15u;
+	uint32_t w[8] = { v.x, v.y, v.z, v.w, 0, 0, 0, 0 };
+#pragma unroll
+	for (int k = 0; k < 4; ++k)
+		w[4 + k] = __shfl_down_sync(0xffffffffu, w[k], 1);
+#pragma unroll
+	for (int k = 0; k < 6; ++k)
+		w[k] = shift & 8 ? w[k + 2] : w[k];
+#pragma unroll
+	for (int k = 0; k < 5; ++k)
+		w[k] = shift & 4 ? w[k + 1] : w[k];
+	const unsigned sel = shift & 2 ? 0x5432u : 0x3210u;
+#pragma unroll
+	for (int k = 0; k < 4; ++k)
+		w[k] = __byte_perm(w[k], w[k + 1], sel) & s.mask[k];
+	if (lane < s.chunks)
+		*reinterpret_cast<uint4 *>(to + lane * 16) = make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// The block into its ring slot.
+__device__ __forceinline__ void store_block(const SoftSource &s, int b, int lane, const LineBlock &blk, char *slot, int P)
+{
+	const char *row = s.first + static_cast<ptrdiff_t>(b) * kBlockLines * s.stride;
+#pragma unroll
+	for (int l = 0; l < kBlockLines; ++l, row += s.stride)
+		store_line(s, row, blk.v[l], lane, slot + l * P);
+}
+
+// Blocks of an item that fill_first brings in: what the ring holds, a line of
+// each for every warp and again.
+__device__ __forceinline__ int first_blocks(const Pipe &p, int begin_blk, int end_blk)
+{
+	return min(p.NB, end_blk - begin_blk);
+}
+
+// An item's first blocks without tensor copies: their lines dealt out to every
+// warp of the CTA (all are at the item's start, the ring is free). A CTA of a
+// small plane has no other blocks, so that they come in a latency or two, not
+// in one for each block. A call of its own: inlined, its addresses stay in
+// registers through the producer's loop, and spill there.
+static __device__ __noinline__ void fill_first(const FusedJob &J, int strip, int begin, int end, char *ring, int ring_mask, int P)
+{
+	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+	const SoftSource src = soft_source(J, strip, lane);
+	constexpr int kBatch = 4;
+	for (int y0 = begin + warp; y0 < end; y0 += kBatch * (kWsWarps + 1)) {
+		uint4 v[kBatch];
+#pragma unroll
+		for (int i = 0; i < kBatch; ++i) {
+			const int y = y0 + i * (kWsWarps + 1);
+			const char *row = src.first + static_cast<ptrdiff_t>(y) * src.stride;
+			const char *c = row - (reinterpret_cast<uintptr_t>(row) & 15) + lane * 16;
+			v[i] = make_uint4(0, 0, 0, 0);
+			if (y < min(end, src.src_h) && lane <= src.chunks && c < row + src.row_bytes) {
+				if (c >= src.lo && c + 16 <= src.hi)
+					v[i] = __ldg(reinterpret_cast<const uint4 *>(c));
+				else
+					v[i] = load_chunk(src, c);
+			}
+		}
+#pragma unroll
+		for (int i = 0; i < kBatch; ++i) {
+			const int y = y0 + i * (kWsWarps + 1);
+			if (y < end)
+				store_line(src, src.first + static_cast<ptrdiff_t>(y) * src.stride, v[i], lane,
+				           ring + (y & ring_mask) * P);
+		}
+	}
+}
+
+// The producer warp's part of an item without tensor copies, fill_first done.
+__device__ __forceinline__ void produce_lines(Pipe &p, const FusedJob &J, int strip, int g_begin, int ngroups,
+                                              int slot_bytes)
+{
+	const int window = slot_bytes / 64;  // lines of a group: 16 KV, of KV KB of fragments
+	const char *vtab = reinterpret_cast<const char *>(J.v_dense);
+	const int drop = blockIdx.x == 0 ? g_chain_drop_group : -1;
+	const int *vb = p.vb;
+	const int end_blk = (vb[ngroups - 1] + window - 1) / kBlockLines + 1;
+	int next_blk = vb[0] / kBlockLines, gneed = 0;
+	next_blk += first_blocks(p, next_blk, end_blk);
+	int rel_s = static_cast<int>(p.released % p.NS);
+	unsigned rel_ph = (p.released / p.NS) & 1;
+	auto release_to = [&](unsigned n) -> bool {
+		while (p.released < n) {
+			if (!__all_sync(0xffffffffu, mbar_wait_for(&p.empty[rel_s], rel_ph, p.wait_ns)))
+				return false;
+			++p.released;
+			if (++rel_s == p.NS) {
+				rel_s = 0;
+				rel_ph ^= 1;
+			}
+		}
+		return true;
+	};
+	int s = static_cast<int>(p.base % p.NS);
+	// group k's lines are in the ring: its fragments, and the arrival
+	auto issue = [&](int k) {
+		const unsigned g = p.base + k;
+		__syncwarp();
+		if (p.lane == 0 && static_cast<int>(g) != drop) {
+			mbar_arrive_expect_tx(&p.full[s], static_cast<unsigned>(slot_bytes));
+			bulk_load(p.vslots + s * slot_bytes, vtab + static_cast<size_t>(g_begin + k) * slot_bytes, slot_bytes,
+			          &p.full[s]);
+		}
+		p.issued = g + 1;
+		s = s + 1 == p.NS ? 0 : s + 1;
+	};
+	// the stage's fragment slot was last read by group g - NS
+	auto stage_free = [&](int k) {
+		const unsigned g = p.base + k;
+		if (g >= static_cast<unsigned>(p.NS) && !release_to(g - p.NS + 1))
+			p.error = 2;
+		return !p.error;
+	};
+	// the groups that need no other lines than fill_first's
+	int k = 0;
+	for (; k < ngroups && (vb[k] + window - 1) / kBlockLines < next_blk && stage_free(k); ++k)
+		issue(k);
+	if (k < ngroups && !p.error) {
+		const SoftSource src = soft_source(J, strip, p.lane);
+		constexpr int kAhead = 5;  // blocks asked of L2 ahead: about 20 KB a CTA in flight
+		LineBlock blk;
+		load_block(src, next_blk, p.lane, blk);
+		for (int b = 1; b < kAhead; ++b)
+			if (next_blk + b < end_blk)
+				prefetch_block(src, next_blk + b, p.lane);
+		for (; k < ngroups && stage_free(k); ++k) {
+			const int last_blk = (vb[k] + window - 1) / kBlockLines;
+			for (; next_blk <= last_blk; ++next_blk) {
+				// ring block b mod NB held block b - NB, which groups read up
+				// to the first one whose window starts past it
+				while (gneed < ngroups && vb[gneed] < (next_blk - p.NB + 1) * kBlockLines)
+					++gneed;
+				if (gneed > k) {
+					p.error = 3;  // the ring cannot hold one window
+					break;
+				}
+				if (!release_to(p.base + gneed)) {
+					p.error = 2;
+					break;
+				}
+				store_block(src, next_blk, p.lane, blk, p.ring + (next_blk & (p.NB - 1)) * kBlockLines * p.P, p.P);
+				if (next_blk + 1 < end_blk)
+					load_block(src, next_blk + 1, p.lane, blk);
+				if (next_blk + kAhead < end_blk)
+					prefetch_block(src, next_blk + kAhead, p.lane);
+			}
+			if (p.error)
+				break;
+			issue(k);
+		}
+	}
+	if (p.error && p.lane == 0)
+		*p.abort_item = 1;  // benign race: every writer stores 1
+}
+
+// A warp's staged tiles into rows row0 .. row0 + 15 of a destination that is
+// not 16-byte aligned: consecutive lanes along a row, two samples each where
+// the rows allow 4-byte stores, one otherwise.
+template <int T>
+__device__ __forceinline__ void store_words(char *dst, ptrdiff_t dst_stride, int dst_w, int dst_h, int dst_align, const char *stage,
+                                            int tile0, int row0, int lane)
+{
+	if (dst_align >= 4) {
+#pragma unroll
+		for (int i = 0; i < T * 4; ++i) {
+			const int w = (i * 32 + lane) % (T * 8), row = (i * 32 + lane) / (T * 8);
+			const int col = tile0 * kTileW + 2 * w;
+			if (row0 + row >= dst_h || col >= dst_w)
+				continue;
+			const uint32_t v = lds32(stage + (w >> 3) * kTileStage + row * kStageBytes + (w & 7) * 4);
+			char *d = dst + static_cast<ptrdiff_t>(row0 + row) * dst_stride + static_cast<ptrdiff_t>(col) * 2;
+			if (col + 1 < dst_w)
+				*reinterpret_cast<uint32_t *>(d) = v;
+			else
+				*reinterpret_cast<uint16_t *>(d) = static_cast<uint16_t>(v);
+		}
+		return;
+	}
+#pragma unroll 4
+	for (int i = 0; i < T * 8; ++i) {
+		const int x = (i * 32 + lane) % (T * 16), row = (i * 32 + lane) / (T * 16);
+		const int col = tile0 * kTileW + x;
+		if (row0 + row < dst_h && col < dst_w)
+			reinterpret_cast<uint16_t *>(dst + static_cast<ptrdiff_t>(row0 + row) * dst_stride)[col] =
+				*reinterpret_cast<const uint16_t *>(stage + (x >> 4) * kTileStage + row * kStageBytes + (x & 15) * 2);
+	}
+}
+
 // One item: groups g_begin .. g_begin + ngroups - 1 of strip `strip` of job
-// J, the group bases already in p.vb. The producer warp brings the data in;
+// J (`tmap`: its source plane's tensor map, where FORM takes one), the group
+// bases already in p.vb. The producer warp brings the data in;
 // the consumer warps compute and store. Both sides pass one CTA barrier
 // (group bases visible, the previous item finished).
 // SPECIALISE: compile-time bodies for the common reuse cases (the
 // single-variant kernels; the mixed kernel keeps one body per variant).
-template <bool H_FIRST, int KV, int KH, bool SPECIALISE>
+template <bool H_FIRST, int KV, int KH, bool SPECIALISE, ChainForm FORM>
 __device__ __forceinline__ void chain_item(Pipe &p, const SmemLayout &L, const FusedJob &J, const void *tmap, int strip,
                                            int g_begin, int ngroups)
 {
+	constexpr bool TENSOR = FORM != ChainForm::LINES, ALIGNED = FORM == ChainForm::ALIGNED;
 	constexpr int kSlotBytes = KV * 2 * 32 * 16;
 	constexpr int T = tiles_per_warp(KV, KH);
-	constexpr int kStripTiles = kWsWarps * T;
+	const int strip_tiles = ALIGNED ? kWsWarps * T : J.strip_w / kTileW;  // at most kWsWarps * T
 	const int NS = p.NS, NB = p.NB, P = p.P, warp = p.warp, lane = p.lane;
 	const unsigned line_mask = p.line_mask;
 	const unsigned long long wait_ns = p.wait_ns;
@@ -349,10 +660,19 @@ __device__ __forceinline__ void chain_item(Pipe &p, const SmemLayout &L, const F
 	uint64_t *const full = p.full;
 	uint64_t *const empty = p.empty;
 	const bool producer = p.producer;
+	if constexpr (!TENSOR) {
+		__syncthreads();  // group bases visible; every warp is done with the previous item
+		const int begin_blk = vb[0] / kBlockLines, end_blk = (vb[ngroups - 1] + 16 * KV - 1) / kBlockLines + 1;
+		fill_first(J, strip, begin_blk * kBlockLines, (begin_blk + first_blocks(p, begin_blk, end_blk)) * kBlockLines, ring,
+		           NB * kBlockLines - 1, P);
+	}
 	if (producer) {
 		__syncthreads();  // group bases visible; every warp is done with the previous item
-		if (lane == 0 && !p.error) {
-						const char *vtab = reinterpret_cast<const char *>(J.v_dense);
+		if constexpr (!TENSOR) {
+			if (!p.error)
+				produce_lines(p, J, strip, g_begin, ngroups, kSlotBytes);
+		} else if (lane == 0 && !p.error) {
+			const char *vtab = reinterpret_cast<const char *>(J.v_dense);
 			const int xlo = __ldg(J.win_col + 2 * strip);
 			const int drop = blockIdx.x == 0 ? g_chain_drop_group : -1;
 			// next source block to load; first group of the item whose
@@ -429,8 +749,8 @@ __device__ __forceinline__ void chain_item(Pipe &p, const SmemLayout &L, const F
 		const int xlo = __ldg(J.win_col + 2 * strip);
 		const int gid = lane >> 2, tig = lane & 3;
 		const int ntiles = (J.dst_w + kTileW - 1) / kTileW;
-		const int tile0 = strip * kStripTiles + warp * T;
-		const bool active = tile0 * kTileW < J.dst_w;
+		const int tile0 = strip * strip_tiles + warp * T;
+		const bool active = (ALIGNED || warp * T < strip_tiles) && tile0 * kTileW < J.dst_w;
 		uint4 ah[T][KH][2];
 		uint32_t colb[T];
 		uint32_t blk[T][2 * KV][2];  // H first: the window's 8-line blocks (hfirst_h)
@@ -467,9 +787,10 @@ __device__ __forceinline__ void chain_item(Pipe &p, const SmemLayout &L, const F
 		const int st_tile = store_tile(T, lane);
 		const char *ld_addr = stage + st_tile * kTileStage + st_row * kStageBytes + (lane & 1) * 16;
 		const int st_col = (tile0 + st_tile) * kTileW + (lane & 1) * 8;
-		const bool wide = J.vec_ok && st_col + 8 <= J.dst_w;
+		const bool wide = J.dst_align == 16 && st_col + 8 <= J.dst_w;
 		char *const dst = static_cast<char *>(J.dst);
 		const ptrdiff_t dst_stride = J.dst_stride;
+		const int dst_w = J.dst_w, dst_h = J.dst_h, dst_align = J.dst_align;
 		char *drow = dst + static_cast<ptrdiff_t>(g_begin * 16 + st_row) * dst_stride + static_cast<ptrdiff_t>(st_col) * 2;
 		const ptrdiff_t group_step = 16 * dst_stride;
 		const ptrdiff_t store_step = kStoreRows * dst_stride;
@@ -543,13 +864,13 @@ __device__ __forceinline__ void chain_item(Pipe &p, const SmemLayout &L, const F
 					for (int i = 0; i < kStores; ++i)
 						*reinterpret_cast<uint4 *>(drow + i * store_step) =
 							*reinterpret_cast<const uint4 *>(ld_addr + i * kStoreRows * kStageBytes);
-				} else {
+				} else if (ALIGNED || dst_align == 16) {
 					for (int i = 0; i < kStores; ++i) {
 						const int row = (g_begin + k) * 16 + st_row + i * kStoreRows;
 						if (row < J.dst_h && st_col < J.dst_w) {
 							const uint4 v = *reinterpret_cast<const uint4 *>(ld_addr + i * kStoreRows * kStageBytes);
 							uint16_t *d = reinterpret_cast<uint16_t *>(dst + static_cast<ptrdiff_t>(row) * dst_stride) + st_col;
-							if (J.vec_ok && st_col + 8 <= J.dst_w) {
+							if (J.dst_align == 16 && st_col + 8 <= J.dst_w) {
 								*reinterpret_cast<uint4 *>(d) = v;
 							} else {
 								const uint32_t w[4] = { v.x, v.y, v.z, v.w };
@@ -558,6 +879,8 @@ __device__ __forceinline__ void chain_item(Pipe &p, const SmemLayout &L, const F
 							}
 						}
 					}
+				} else if constexpr (!ALIGNED) {
+					store_words<T>(dst, dst_stride, dst_w, dst_h, dst_align, stage, tile0, (g_begin + k) * 16, lane);
 				}
 				__syncwarp();
 			} else {
@@ -612,7 +935,7 @@ __device__ __forceinline__ void load_bases(Pipe &p, const FusedJob &J, int g_beg
 // order (a whole strip, so that neighbouring CTAs run neighbouring strips in
 // step and read their shared columns once through L2, then an equal share of
 // the strips left over).
-template <bool H_FIRST, int KV, int KH>
+template <bool H_FIRST, int KV, int KH, ChainForm FORM>
 __global__ void __launch_bounds__(tma_threads(H_FIRST), 2)
 chain_tma_kernel(const FusedJob *__restrict__ jobs, int num_jobs, int total_items, const int *__restrict__ ranges,
                  const __grid_constant__ FewJobs few, const __grid_constant__ SmemLayout L,
@@ -645,8 +968,8 @@ chain_tma_kernel(const FusedJob *__restrict__ jobs, int num_jobs, int total_item
 			const int ngroups = min(J.groups - g_begin, t_end - t);
 			t += ngroups;
 			load_bases(p, J, g_begin, ngroups);
-			chain_item<H_FIRST, KV, KH, true>(p, L, J, jobs ? J.tmap : static_cast<const void *>(&few_maps.map[job]), strip,
-			                                  g_begin, ngroups);
+			chain_item<H_FIRST, KV, KH, true, FORM>(p, L, J, jobs ? J.tmap : static_cast<const void *>(&few_maps.map[job]),
+			                                          strip, g_begin, ngroups);
 			p.base += ngroups;
 			__syncthreads();  // the next item rewrites the group bases and the ring
 			if (abort_item)
@@ -654,67 +977,6 @@ chain_tma_kernel(const FusedJob *__restrict__ jobs, int num_jobs, int total_item
 		}
 	}
 	pipe_finish(p);
-}
-
-// Variant codes of mixed launches: the chained kernel's variant - 200
-// (H first, KV, KH), or kCopyVariant for an identity plane.
-constexpr int kCopyVariant = 1000;
-
-// One launch over a batch of mixed jobs: every chained variant and identity
-// copies. CTAs take chunks of units from a counter (guided sizes, cut by the
-// host from estimated costs: large chunks first, small ones last, so that
-// the CTAs end together); an item is dispatched on its job's variant.
-__global__ void __launch_bounds__(tma_threads(true), 2)
-chain_mixed_kernel(const FusedJob *__restrict__ jobs, int num_jobs, const __grid_constant__ WorkChunks C,
-                   const __grid_constant__ SmemLayout L)
-{
-	extern __shared__ float4 smem4[];
-	__shared__ int abort_item;
-	__shared__ int chunk;
-	Pipe p;
-	pipe_init(p, smem4, L, &abort_item);
-	// chunks in the order CTAs ask for them (guided sizes: large first)
-	for (;;) {
-		const int m = next_chunk(C, &chunk);
-		if (m < 0 || abort_item)
-			break;
-		const int t_end = __ldg(C.bounds + m + 1);
-		for (int t = __ldg(C.bounds + m); t < t_end;) {
-			const FusedJob &J = jobs[find_job(jobs, num_jobs, t)];
-			const int local = t - J.item_begin;
-			const int strip = local / J.groups;
-			const int g_begin = local - strip * J.groups;
-			const int ngroups = min(J.groups - g_begin, t_end - t);
-			t += ngroups;
-			const int v = J.variant;
-			if (v == kCopyVariant) {
-				copy_item(J, g_begin, ngroups);
-			} else {
-				load_bases(p, J, g_begin, ngroups);
-				switch (v) {
-#define ZG_CHAIN_CASE(HF, KV, KH)                                                                     \
-	case (HF ? 12 : 0) + (KV - 1) * 4 + (KH - 1):                                                      \
-		chain_item<HF, KV, KH, false>(p, L, J, J.tmap, strip, g_begin, ngroups);                     \
-		break;
-					ZG_CHAIN_CASE(true, 1, 1) ZG_CHAIN_CASE(true, 1, 2) ZG_CHAIN_CASE(true, 1, 3) ZG_CHAIN_CASE(true, 1, 4)
-					ZG_CHAIN_CASE(true, 2, 1) ZG_CHAIN_CASE(true, 2, 2) ZG_CHAIN_CASE(true, 2, 3) ZG_CHAIN_CASE(true, 2, 4)
-					ZG_CHAIN_CASE(true, 3, 1) ZG_CHAIN_CASE(true, 3, 2) ZG_CHAIN_CASE(true, 3, 3) ZG_CHAIN_CASE(true, 3, 4)
-					ZG_CHAIN_CASE(false, 1, 1) ZG_CHAIN_CASE(false, 1, 2) ZG_CHAIN_CASE(false, 1, 3) ZG_CHAIN_CASE(false, 1, 4)
-					ZG_CHAIN_CASE(false, 2, 1) ZG_CHAIN_CASE(false, 2, 2) ZG_CHAIN_CASE(false, 2, 3) ZG_CHAIN_CASE(false, 2, 4)
-					ZG_CHAIN_CASE(false, 3, 1) ZG_CHAIN_CASE(false, 3, 2) ZG_CHAIN_CASE(false, 3, 3) ZG_CHAIN_CASE(false, 3, 4)
-#undef ZG_CHAIN_CASE
-				default:
-					break;
-				}
-			}
-			p.base += J.variant == kCopyVariant ? 0 : ngroups;
-			__syncthreads();  // the next item rewrites the group bases and the ring
-			if (abort_item)
-				break;
-		}
-	}
-	pipe_finish(p);
-	chunks_finish(C);  // the last CTA out leaves the counter zero for the next launch
 }
 
 } // namespace chain_detail

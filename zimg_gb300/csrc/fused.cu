@@ -293,8 +293,6 @@ namespace {
 
 const void *kernel_ptr(int variant)
 {
-	if (variant >= 200)
-		return chain_kernel_ptr(variant);
 	if (variant >= 100)
 		return mma_kernel_ptr(variant);
 	const int vs = variant % 4, hw = variant / 4 % 4;
@@ -310,8 +308,6 @@ const void *kernel_ptr(int variant)
 
 SmemLayout fused_layout(const FusedPlan *const *plans, int n)
 {
-	if (n > 0 && plans[0]->chain)
-		return chain_layout(plans, n);
 	if (n > 0 && plans[0]->mma)
 		return mma_layout(plans, n);
 	int in = 0, ring = 0;
@@ -346,7 +342,7 @@ int fused_grid_size(int variant, size_t smem_bytes)
 	cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
 	const void *k = kernel_ptr(variant);
 	cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemMax));
-	const int threads = variant >= 200 ? chain_threads(variant) : (variant >= 100 ? mma_threads() : kStreamThreads);
+	const int threads = variant >= 100 ? mma_threads() : kStreamThreads;
 	if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, smem_bytes) != cudaSuccess || per_sm < 1)
 		per_sm = 1;
 	return std::max(1, sms) * per_sm;
@@ -360,8 +356,6 @@ bool fused_takes_chunks(int variant)
 cudaError_t launch_fused(int variant, const FusedJob *jobs, int num_jobs, int total_tiles, const SmemLayout &smem_bytes,
                          int grid, const FewJobs &few, cudaStream_t stream, const WorkChunks &chunks)
 {
-	if (variant >= 200)
-		return launch_chain(variant, jobs, num_jobs, total_tiles, smem_bytes, grid, few, stream);
 	if (variant >= 100)
 		return launch_mma(variant, jobs, num_jobs, total_tiles, smem_bytes, grid, few.job[0], stream);
 	grid = std::max(1, std::min(grid, chunks.sched ? chunks.num : total_tiles));
@@ -383,10 +377,13 @@ void fused_set_io(FusedJob &j, const void *src, ptrdiff_t src_stride, void *dst,
 	j.dst_stride = dst_stride;
 	auto al = [](const void *p, ptrdiff_t s) { return reinterpret_cast<uintptr_t>(p) % 16 == 0 && s % 16 == 0; };
 	j.vec_ok = al(src, src_stride) && al(dst, dst_stride) ? 1 : 0;
-	const uintptr_t a = reinterpret_cast<uintptr_t>(src) | static_cast<uintptr_t>(src_stride);
-	j.src_align = a % 16 == 0 ? 16 : (a % 8 == 0 ? 8 : (a % 4 == 0 ? 4 : 2));
-	const uintptr_t d = reinterpret_cast<uintptr_t>(dst) | static_cast<uintptr_t>(dst_stride);
-	j.dst_vec = d % (j.kind == static_cast<int>(FusedKind::F32) ? 16 : 8) == 0;
+	auto divides = [](const void *p, ptrdiff_t s) {
+		const uintptr_t a = reinterpret_cast<uintptr_t>(p) | static_cast<uintptr_t>(s);
+		return a % 16 == 0 ? 16 : (a % 8 == 0 ? 8 : (a % 4 == 0 ? 4 : 2));
+	};
+	j.src_align = divides(src, src_stride);
+	j.dst_align = divides(dst, dst_stride);
+	j.tmap = nullptr;
 }
 
 } // namespace zg

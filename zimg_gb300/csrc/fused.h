@@ -102,8 +102,8 @@ struct FusedJob {
 	float offset;           // 2^(depth-1)
 	int vec_ok;             // planes and strides 16-byte aligned: vector loads and stores
 	int src_align;          // the largest of 16, 8, 4, 2 that divides the source's base and stride
-	int dst_vec;            // destination base and stride: 8-byte (WORD) or 16-byte (FLOAT) aligned
-	const void *tmap;       // TMA-pipelined chained kernel: the source plane's tensor map (device memory)
+	int dst_align;          // as src_align, of the destination
+	const void *tmap;       // chained kernel with tensor copies: the source plane's tensor map (device memory)
 	int variant;            // chained kernel's variant - 200 ((H first, KV, KH)); mixed launches dispatch on it
 };
 
@@ -150,8 +150,8 @@ struct FusedPlan {
 	int max_pxa = 0;         // widest strip patch (elements)
 	int stage_rows = 1;      // u16 raw staging lines (mma kernel)
 	int depth = 1;           // prefetch depth in steps
-	bool mma = false;        // tensor-core variant (mma_kernel.cuh or chain_kernel.cuh)
-	bool chain = false;      // tensor-core variant with the passes chained in registers (chain_kernel.cuh)
+	bool mma = false;        // tensor-core variant (mma_kernel.cuh or chain_tma_kernel.cuh)
+	bool chain = false;      // tensor-core variant with the passes chained in registers (chain_tma_kernel.cuh)
 	float reuse_frac = 0;    // chained H-first plans: share of groups that reuse the previous group's products
 	std::vector<unsigned char> blob;  // host copy of the tables, uploaded by the owner
 	size_t off_h_taps = 0, off_h_left = 0, off_v_dense = 0, off_v_base = 0, off_win_col = 0;
@@ -208,21 +208,25 @@ cudaError_t launch_mma(int variant, const FusedJob *jobs, int num_jobs, int tota
 const void *mma_kernel_ptr(int variant);
 int mma_threads();
 
-// Chained tensor-core u16 kernel (chain_kernel.cuh): variants 200+. Same
+// Chained tensor-core u16 kernel (chain_tma_kernel.cuh): variants 200+. Same
 // exactness certificate as plan_mma; 16-column tiles per warp, windows of up
-// to 3 x 16 lines and 4 x 16 columns.
+// to 3 x 16 lines and 4 x 16 columns. A launch takes the most special of three
+// forms that all its jobs admit (chain_form): the widths of strips and the
+// 16-byte stores built in; any strip and destination; and without tensor
+// copies, for source planes that have no tensor map (which wants a 16-byte
+// aligned base and positive stride).
+enum class ChainForm { ALIGNED, ANY_DST, LINES };
+struct ChainKernels {
+	const void *(*ptr)(int variant);
+	int (*set_fault)(int drop_group, unsigned long long wait_ns);
+	int (*error)(bool reset);
+};
+extern const ChainKernels kChainAligned, kChainAnyDst, kChainLines;
+ChainForm chain_form(const FusedJob *jobs, int n, bool mapped);
+bool chain_mixed_takes(const FusedJob &j);
 bool plan_chain(const FilterTable &first, const FilterTable &second, bool h_first, unsigned depth, unsigned src_w,
                 unsigned src_h, unsigned dst_w, unsigned dst_h, FusedPlan *out);
-SmemLayout chain_layout(const FusedPlan *const *plans, int n);
-const void *chain_kernel_ptr(int variant);
-int chain_threads(int variant);
-cudaError_t launch_chain(int variant, const FusedJob *jobs, int num_jobs, int total_items, const SmemLayout &L, int grid,
-                         const FewJobs &few, cudaStream_t stream);
-// The same kernel with source lines and tap fragments brought in by tensor
-// copies on an mbarrier pipeline (chain_tma_kernel.cuh). Usable when the
-// layout fits (box width <= 256) and the source plane has a tensor map
-// (16-byte aligned base and stride).
-bool chain_tma_enabled();  // false when the environment sets ZG_CHAIN_TMA=0
+bool chain_tma_enabled();  // tensor copies at all: false when the environment sets ZG_CHAIN_TMA=0
 bool chain_tma_layout(const FusedPlan *const *plans, int n, SmemLayout *out);
 bool chain_tma_source_map(CUtensorMap *map, const FusedJob &j, const SmemLayout &L);
 int chain_tma_grid_size(int variant, size_t smem_bytes);
@@ -233,8 +237,8 @@ int chain_tma_grid_size(int variant, size_t smem_bytes);
 struct FewMaps {
 	CUtensorMap map[kFewJobs];
 };
-cudaError_t launch_chain_tma(int variant, const FusedJob *jobs, int num_jobs, int total_items, const int *ranges,
-                             const SmemLayout &L, int grid, const FewJobs &few, const FewMaps *few_maps,
+cudaError_t launch_chain_tma(int variant, ChainForm form, const FusedJob *jobs, int num_jobs, int total_items,
+                             const int *ranges, const SmemLayout &L, int grid, const FewJobs &few, const FewMaps *few_maps,
                              cudaStream_t stream);
 // Per-CTA unit ranges for `grid` CTAs over jobs of `groups` units per strip
 // and `total_items` units: CTA b first the whole strip b, then an equal share

@@ -136,7 +136,7 @@ __device__ __forceinline__ Item make_item(const FusedJob &J, int t, int t_end)
 	it.src_h = J.src_h;
 	it.dst_h = J.dst_h;
 	it.src_align = J.src_align;
-	it.dst_vec = J.dst_vec;
+	it.dst_vec = J.dst_align >= (J.kind == static_cast<int>(FusedKind::F32) ? 16 : 8);
 	it.c0 = strip * J.strip_w;
 	it.cols_valid = min(J.strip_w, J.dst_w - it.c0);
 	it.xlo = __ldg(J.win_col + 2 * strip);
