@@ -10,6 +10,7 @@
 #include "kernels.h"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace zg {
 
@@ -174,6 +175,88 @@ h_f32_kernel(PassTables t, unsigned lines, const uint8_t *__restrict__ src, ptrd
 		for (unsigned k = 0; k < t.width; ++k)
 			acc = __fmaf_rn(__ldg(c + k), __ldg(s + k), acc);
 		reinterpret_cast<float *>(dst + static_cast<ptrdiff_t>(r) * ds)[j] = acc;
+	}
+}
+
+// Up to kRegTaps taps: thread = one output column of kRegRows lines, its taps
+// in registers (the width is built in, so that no sample outside an output's
+// own taps is read), the loads of kRegBatch lines in flight together. The
+// kernels above, left for longer filters, spend two loads and the loop on each
+// multiply-add, one line at a time. Bound: a 2- or 4-byte load per tap.
+// Measured, one plane, horizontal pass alone, before and now:
+//   u16 960x1080 -> 1920x1080, 6 taps    9.0 -> 5.3 us
+//   u16 1920x1080 -> 1279x1080, 10 taps  8.0 -> 5.6 us
+//   f32 960x1080 -> 1920x1080, 6 taps    8.9 -> 4.5 us
+//   f32 3840x2160 -> 1920x2160, 8 taps   40 -> 17 us
+//   f32 1920x1080 -> 960x1080, 16 taps   39 -> 11 us
+constexpr int kRegTaps = 16;
+constexpr unsigned kRegRows = 8;
+constexpr unsigned kRegBatch = 4;
+
+template <bool INT, int W>
+__global__ void __launch_bounds__(kThreads)
+h_reg_kernel(PassTables t, int32_t pixel_max, unsigned lines, const uint8_t *__restrict__ src, ptrdiff_t ss,
+             uint8_t *__restrict__ dst, ptrdiff_t ds)
+{
+	using S = std::conditional_t<INT, uint16_t, float>;
+	using A = std::conditional_t<INT, int32_t, float>;
+	const unsigned j = blockIdx.x * kThreads + threadIdx.x;
+	if (j >= t.rows)
+		return;
+	const unsigned l = __ldg(t.left + j);
+	A c[W];
+#pragma unroll
+	for (int k = 0; k < W; ++k) {
+		if constexpr (INT)
+			c[k] = __ldg(t.i16 + static_cast<size_t>(j) * W + k);
+		else
+			c[k] = __ldg(t.f32 + static_cast<size_t>(j) * W + k);
+	}
+	const uint32_t b = INT ? static_cast<uint32_t>(__ldg(t.bias + j)) : 0u;
+	const unsigned r0 = blockIdx.y * kRegRows, r1 = min(r0 + kRegRows, lines);
+	for (unsigned r = r0; r < r1; r += kRegBatch) {
+		S x[kRegBatch][W];
+#pragma unroll
+		for (unsigned q = 0; q < kRegBatch; ++q) {
+			const S *s = reinterpret_cast<const S *>(src + static_cast<ptrdiff_t>(min(r + q, r1 - 1)) * ss) + l;
+#pragma unroll
+			for (int k = 0; k < W; ++k)
+				x[q][k] = __ldg(s + k);
+		}
+#pragma unroll
+		for (unsigned q = 0; q < kRegBatch; ++q) {
+			if (r + q >= r1)
+				break;
+			S *out = reinterpret_cast<S *>(dst + static_cast<ptrdiff_t>(r + q) * ds) + j;
+			if constexpr (INT) {
+				uint32_t acc = b;
+#pragma unroll
+				for (int k = 0; k < W; ++k)
+					acc += static_cast<uint32_t>(c[k] * static_cast<int32_t>(x[q][k]));
+				*out = pack_u16(acc, pixel_max);
+			} else {
+				float acc = 0.0f;
+#pragma unroll
+				for (int k = 0; k < W; ++k)
+					acc = __fmaf_rn(c[k], x[q][k], acc);
+				*out = acc;
+			}
+		}
+	}
+}
+
+template <bool INT, int W = kRegTaps>
+cudaError_t launch_h_reg(const PassLaunch &l, cudaStream_t stream)
+{
+	if constexpr (W > 0) {
+		if (l.t.width != W)
+			return launch_h_reg<INT, W - 1>(l, stream);
+		dim3 grid((l.t.rows + kThreads - 1) / kThreads, (l.lines + kRegRows - 1) / kRegRows);
+		h_reg_kernel<INT, W><<<grid, kThreads, 0, stream>>>(l.t, l.pixel_max, l.lines, static_cast<const uint8_t *>(l.src),
+		                                                    l.src_stride, static_cast<uint8_t *>(l.dst), l.dst_stride);
+		return cudaGetLastError();
+	} else {
+		return cudaErrorInvalidValue;
 	}
 }
 
@@ -349,6 +432,8 @@ cudaError_t launch_pass(const PassLaunch &l, cudaStream_t stream)
 			return cudaGetLastError();
 		}
 	}
+	if (l.horizontal && l.t.width <= kRegTaps)
+		return l.sample == Sample::U16 ? launch_h_reg<true>(l, stream) : launch_h_reg<false>(l, stream);
 	if (l.horizontal) {
 		const unsigned rpb = 8;
 		dim3 grid((l.t.rows + kThreads - 1) / kThreads, (l.lines + rpb - 1) / rpb);
