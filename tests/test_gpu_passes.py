@@ -1,6 +1,6 @@
-"""Horizontal passes with the taps in registers (pass_kernels.cu): every width
-the kernel is built for and the first that it is not, line counts around its
-batches, against the oracle bit for bit (u16: the C path; f32: one fused
+"""Separate passes with the width built in (pass_kernels.cu): every width the
+kernels are built for and the first that they are not, lines and columns around
+their batches, against the oracle bit for bit (u16: the C path; f32: one fused
 multiply-add per tap in its order)."""
 import numpy as np
 import pytest
@@ -33,3 +33,17 @@ def test_horizontal_taps_in_registers(cuda, oracle, width):
         src = rng.standard_normal((h, sw)).astype(np.float32)
         got, _ = run_conversion(src, dw, h, kind, a, pad=pad, offset=offset)
         np.testing.assert_array_equal(got, oracle.resize_plane(src, dw, h, kind, a, mode="fma"))
+
+
+@pytest.mark.parametrize("width", range(1, 18))
+def test_vertical_window_in_flight(cuda, oracle, width):
+    kind, a, sh, dh = case_of_width(width)
+    rng = np.random.default_rng(100 + width)
+    for w, pad, offset in [(1, 0, 0), (8, 0, 0), (19, 5, 0), (21, 3, 8), (1030, 2, 0), (130, 0, 1)]:
+        for depth in (10, 16):
+            src = rng.integers(0, 1 << depth, size=(sh, w), dtype=np.uint16)
+            got, _ = run_conversion(src, w, dh, kind, a, depth=depth, pad=pad, offset=offset)
+            np.testing.assert_array_equal(got, oracle.resize_plane(src, w, dh, kind, a, depth=depth, mode="c"))
+        src = rng.standard_normal((sh, w)).astype(np.float32)
+        got, _ = run_conversion(src, w, dh, kind, a, pad=pad, offset=offset)
+        np.testing.assert_array_equal(got, oracle.resize_plane(src, w, dh, kind, a, mode="fma"))
