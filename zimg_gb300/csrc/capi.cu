@@ -3,6 +3,7 @@
 #include "depth.h"
 
 #include <algorithm>
+#include <cstring>
 #include <climits>
 
 namespace {
@@ -211,7 +212,7 @@ void check_device(int device)
 		throw Error(kErrLogic, "object used on a different device than the one it was created on");
 }
 
-void run_pass(const DevicePass &p, const void *src, ptrdiff_t ss, void *dst, ptrdiff_t ds, cudaStream_t stream)
+void run_pass(const DevicePass &p, const PassPlane *planes, int n, cudaStream_t stream)
 {
 	PassLaunch l{};
 	l.t = p.tables;
@@ -219,12 +220,20 @@ void run_pass(const DevicePass &p, const void *src, ptrdiff_t ss, void *dst, ptr
 	l.sample = p.sample;
 	l.pixel_max = p.pixel_max;
 	l.lines = p.horizontal ? p.src_h : p.src_w;
-	l.src = src;
-	l.src_stride = ss;
-	l.dst = dst;
-	l.dst_stride = ds;
+	l.src = planes[0].src;
+	l.src_stride = planes[0].src_stride;
+	l.dst = planes[0].dst;
+	l.dst_stride = planes[0].dst_stride;
+	l.planes = planes;
+	l.num_planes = n;
 	l.wide = p.wide;
 	cuda_check(launch_pass(l, stream), "resize pass launch");
+}
+
+void run_pass(const DevicePass &p, const void *src, ptrdiff_t ss, void *dst, ptrdiff_t ds, cudaStream_t stream)
+{
+	const PassPlane plane{ src, ss, dst, ds };
+	run_pass(p, &plane, 1, stream);
 }
 
 void check_plane(const void *p, ptrdiff_t stride, unsigned w, Sample s, const char *what)
@@ -489,10 +498,22 @@ zg_error_code zg_resize_process(const zg_resize *r, const void *src, ptrdiff_t s
 
 namespace zg {
 
+bool same_passes(const zg_resize *a, const zg_resize *b)
+{
+	for (const zg_resize *r : { a, b }) {
+		if (r->fused || r->num_passes == 0)
+			return false;
+		for (int k = 0; k < r->num_passes; ++k)
+			if (r->pass[k]->wide.frag || r->pass[k]->tables.dense)
+				return false;
+	}
+	return a->device == b->device && !std::memcmp(&a->params, &b->params, sizeof(a->params));
+}
+
 void resize_planes(const ResizeIo *io, int n, cudaStream_t st)
 {
-	bool done[kFewJobs] = {};
-	if (n > kFewJobs)
+	bool done[kResizePlanes] = {};
+	if (n > kResizePlanes)
 		throw Error(kErrLogic, "too many planes");
 	for (int k = 0; k < n; ++k) {
 		const zg_resize *r = io[k].r;
@@ -516,13 +537,22 @@ void resize_planes(const ResizeIo *io, int n, cudaStream_t st)
 			           static_cast<size_t>(r->params.dst_width) * bytes_of(r->sample), r->params.dst_height, st);
 			continue;
 		}
-		if (r->num_passes == 1) {
-			run_pass(*r->pass[0], x.src, x.src_stride, x.dst, x.dst_stride, st);
-			continue;
-		}
 		if (!r->fused) {
-			run_pass(*r->pass[0], x.src, x.src_stride, x.tmp, r->tmp_stride, st);
-			run_pass(*r->pass[1], x.tmp, r->tmp_stride, x.dst, x.dst_stride, st);
+			// the planes of the same conversion that follow, in the same launches
+			PassPlane first[kResizePlanes], second[kResizePlanes];
+			int count = 0;
+			for (int b = a; b < n; ++b) {
+				const ResizeIo &y = io[b];
+				if (done[b] || (b > a && !same_passes(r, y.r)))
+					continue;
+				done[b] = true;
+				const bool one = r->num_passes == 1;
+				first[count] = { y.src, y.src_stride, one ? y.dst : y.tmp, one ? y.dst_stride : r->tmp_stride };
+				second[count++] = { y.tmp, r->tmp_stride, y.dst, y.dst_stride };
+			}
+			run_pass(*r->pass[0], first, count, st);
+			if (r->num_passes == 2)
+				run_pass(*r->pass[1], second, count, st);
 			continue;
 		}
 		// the planes of this plan's variant that follow ride in the same
@@ -532,7 +562,7 @@ void resize_planes(const ResizeIo *io, int n, cudaStream_t st)
 		int count = 0, items = 0, grid = r->fgrid;
 		for (int b = a; b < n; ++b) {
 			const zg_resize *q = io[b].r;
-			if (done[b] || !q->fused || q->fplan.variant != r->fplan.variant ||
+			if (done[b] || count == kFewJobs || !q->fused || q->fplan.variant != r->fplan.variant ||
 			    (b > a && r->fplan.mma && !r->fplan.chain))
 				continue;
 			done[b] = true;

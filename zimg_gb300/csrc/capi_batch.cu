@@ -46,6 +46,8 @@ struct zg_batch {
 	std::vector<int> chunks_host;
 	DeviceBuffer chunks_dev;
 	DeviceBuffer sched_dev;  // two words per group (zero between launches)
+	// unfused jobs, those of one conversion together (up to kResizePlanes)
+	std::vector<std::vector<unsigned>> unfused;
 	std::vector<FusedJob> table_host;
 	DeviceBuffer table_dev;
 	std::vector<CUtensorMap> maps_host;  // per table entry (chained groups' source planes that admit one)
@@ -161,18 +163,16 @@ void batch_launch(const zg_batch *b, void *tmp, cudaStream_t st)
 			           "batch plane copies");
 		});
 	}
-	for (size_t i = 0; i < b->jobs.size(); ++i) {
-		if (b->table_index[i] >= 0 || b->jobs[i]->num_passes == 0)
-			continue;
-		work.push_back([b, i, tmp](cudaStream_t s) {
-			const zg_batch_io &io = b->io[i];
-			void *t = b->tmp_size ? static_cast<char *>(tmp) + b->tmp_offset[i] : nullptr;
-			zg_error_code rc = zg_resize_process(b->jobs[i], io.src, io.src_stride, io.dst, io.dst_stride, t,
-			                                     reinterpret_cast<zg_stream>(s));
-			if (rc != ZG_ERROR_SUCCESS)
-				rethrow_last(rc);
+	for (const auto &u : b->unfused)
+		work.push_back([b, &u, tmp](cudaStream_t s) {
+			ResizeIo io[kResizePlanes];
+			for (size_t k = 0; k < u.size(); ++k) {
+				const zg_batch_io &x = b->io[u[k]];
+				io[k] = { b->jobs[u[k]], x.src, x.src_stride, x.dst, x.dst_stride,
+				          b->tmp_size ? static_cast<char *>(tmp) + b->tmp_offset[u[k]] : nullptr };
+			}
+			resize_planes(io, static_cast<int>(u.size()), s);
 		});
-	}
 	if (work.size() <= 1) {
 		for (auto &w : work)
 			w(st);
@@ -348,6 +348,19 @@ void regroup(zg_batch *b)
 		b->tmp_offset.push_back(b->tmp_size);
 		if (!b->jobs[i]->fused)
 			b->tmp_size += (b->jobs[i]->tmp_size + 255) & ~static_cast<size_t>(255);
+	}
+	b->unfused.clear();
+	for (unsigned i = 0; i < num_jobs; ++i) {
+		const zg_resize *r = b->jobs[i];
+		if (r->fused || r->num_passes == 0)
+			continue;
+		auto g = std::find_if(b->unfused.begin(), b->unfused.end(), [&](const std::vector<unsigned> &u) {
+			return u.size() < static_cast<size_t>(kResizePlanes) && same_passes(b->jobs[u[0]], r);
+		});
+		if (g == b->unfused.end())
+			b->unfused.push_back({ i });
+		else
+			g->push_back(i);
 	}
 	b->groups.clear();
 	b->ranges_host.clear();
@@ -828,11 +841,8 @@ zg_error_code zg_batch_get_launch_count(const zg_batch *b, unsigned *out)
 		} else {
 			n = static_cast<unsigned>(b->groups.size()) + (b->copy_jobs.empty() ? 0u : 1u);
 		}
-		for (size_t i = 0; i < b->jobs.size(); ++i) {
-			if (b->table_index[i] >= 0)
-				continue;
-			n += static_cast<unsigned>(b->jobs[i]->num_passes);
-		}
+		for (const auto &u : b->unfused)
+			n += static_cast<unsigned>(b->jobs[u[0]]->num_passes);
 		*out = n;
 	});
 }

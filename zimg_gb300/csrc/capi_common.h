@@ -189,6 +189,11 @@ struct ResizeIo {
 
 // Independent planes (each with its own tmp), in as few launches as their
 // plans allow. Throws on bad arguments and failed launches.
+constexpr int kResizePlanes = kPassPlanes;
 void resize_planes(const ResizeIo *io, int n, cudaStream_t stream);
+// Whether two unfused conversions are one, so that resize_planes runs their
+// planes in the same launches: equal parameters give equal tables. (Wide
+// filters' kernels take a plane each.)
+bool same_passes(const ::zg_resize *a, const ::zg_resize *b);
 
 } // namespace zg

@@ -71,7 +71,19 @@ struct WideTables {
 	int umax_taps;            // widest band of one output (taps)
 };
 
-// One pass over a whole plane. For a horizontal pass the plane has
+// The planes of one launch of a pass.
+struct PassPlane {
+	const void *src;
+	ptrdiff_t src_stride;  // bytes
+	void *dst;
+	ptrdiff_t dst_stride;  // bytes
+};
+constexpr int kPassPlanes = 16;
+struct PassPlanes {
+	PassPlane p[kPassPlanes];
+};
+
+// One pass over whole planes of one size. For a horizontal pass the plane has
 // `lines` rows of input_width samples -> rows outputs each; for a vertical
 // pass it has `lines` columns, input_width rows -> rows rows.
 struct PassLaunch {
@@ -80,10 +92,12 @@ struct PassLaunch {
 	Sample sample;
 	int32_t pixel_max;     // (1 << depth) - 1 for U16
 	unsigned lines;        // height (H) or width (V) of the plane
-	const void *src;
+	const void *src;       // the first plane
 	ptrdiff_t src_stride;  // bytes
 	void *dst;
 	ptrdiff_t dst_stride;  // bytes
+	const PassPlane *planes = nullptr;  // num_planes of them (the first one too), where pass_takes_planes()
+	int num_planes = 1;
 	WideTables wide;       // FP32 passes on the tensor cores when wide.frag is set
 };
 

@@ -25,14 +25,26 @@ __device__ __forceinline__ uint16_t pack_u16(uint32_t acc, int32_t pixel_max)
 	return static_cast<uint16_t>(x);
 }
 
+// The block's plane: planes of one size and filter run in one launch, one to
+// a grid layer. A batch's planes, small ones above all, were bound by a launch
+// for each of their passes: a call of 9 4:2:0 frames 496x210 -> 216x92, 17
+// taps, 187 -> 19 us, of 32 f32 planes 1920x1080 -> 480x270, Lanczos-3, 426 ->
+// 142 us (with the kernels for up to kRegTaps taps below).
+#define ZG_PASS_PLANE                                                          \
+	const uint8_t *const src = static_cast<const uint8_t *>(P.p[blockIdx.z].src); \
+	const ptrdiff_t ss = P.p[blockIdx.z].src_stride;                             \
+	uint8_t *const dst = static_cast<uint8_t *>(P.p[blockIdx.z].dst);            \
+	const ptrdiff_t ds = P.p[blockIdx.z].dst_stride;
+
 // ---------------------------------------------------------------- vertical --
 // Thread = VEC adjacent columns; block = kThreads * VEC columns x `rows_per_block`
 // output rows. Every load of a row segment is coalesced across the warp.
 template <int VEC>
 __global__ void __launch_bounds__(kThreads)
-v_u16_kernel(PassTables t, int32_t pixel_max, unsigned plane_w, const uint8_t *__restrict__ src, ptrdiff_t ss,
-             uint8_t *__restrict__ dst, ptrdiff_t ds, unsigned rows_per_block)
+v_u16_kernel(PassTables t, int32_t pixel_max, unsigned plane_w, const __grid_constant__ PassPlanes P,
+             unsigned rows_per_block)
 {
+	ZG_PASS_PLANE
 	const unsigned j0 = (blockIdx.x * kThreads + threadIdx.x) * VEC;
 	if (j0 >= plane_w)
 		return;
@@ -87,9 +99,10 @@ v_u16_kernel(PassTables t, int32_t pixel_max, unsigned plane_w, const uint8_t *_
 
 template <int VEC>
 __global__ void __launch_bounds__(kThreads)
-v_f32_kernel(PassTables t, unsigned plane_w, const uint8_t *__restrict__ src, ptrdiff_t ss,
-             uint8_t *__restrict__ dst, ptrdiff_t ds, unsigned rows_per_block)
+v_f32_kernel(PassTables t, unsigned plane_w, const __grid_constant__ PassPlanes P,
+             unsigned rows_per_block)
 {
+	ZG_PASS_PLANE
 	const unsigned j0 = (blockIdx.x * kThreads + threadIdx.x) * VEC;
 	if (j0 >= plane_w)
 		return;
@@ -138,9 +151,10 @@ v_f32_kernel(PassTables t, unsigned plane_w, const uint8_t *__restrict__ src, pt
 // -------------------------------------------------------------- horizontal --
 // Thread = one output column for `rows_per_block` lines; its taps stay in L1.
 __global__ void __launch_bounds__(kThreads)
-h_u16_kernel(PassTables t, int32_t pixel_max, unsigned lines, const uint8_t *__restrict__ src, ptrdiff_t ss,
-             uint8_t *__restrict__ dst, ptrdiff_t ds, unsigned rows_per_block)
+h_u16_kernel(PassTables t, int32_t pixel_max, unsigned lines, const __grid_constant__ PassPlanes P,
+             unsigned rows_per_block)
 {
+	ZG_PASS_PLANE
 	const unsigned j = blockIdx.x * kThreads + threadIdx.x;
 	if (j >= t.rows)
 		return;
@@ -159,9 +173,10 @@ h_u16_kernel(PassTables t, int32_t pixel_max, unsigned lines, const uint8_t *__r
 }
 
 __global__ void __launch_bounds__(kThreads)
-h_f32_kernel(PassTables t, unsigned lines, const uint8_t *__restrict__ src, ptrdiff_t ss,
-             uint8_t *__restrict__ dst, ptrdiff_t ds, unsigned rows_per_block)
+h_f32_kernel(PassTables t, unsigned lines, const __grid_constant__ PassPlanes P,
+             unsigned rows_per_block)
 {
+	ZG_PASS_PLANE
 	const unsigned j = blockIdx.x * kThreads + threadIdx.x;
 	if (j >= t.rows)
 		return;
@@ -189,15 +204,15 @@ h_f32_kernel(PassTables t, unsigned lines, const uint8_t *__restrict__ src, ptrd
 //   f32 960x1080 -> 1920x1080, 6 taps    8.9 -> 4.5 us
 //   f32 3840x2160 -> 1920x2160, 8 taps   40 -> 17 us
 //   f32 1920x1080 -> 960x1080, 16 taps   39 -> 11 us
-constexpr int kRegTaps = 16;
+constexpr int kRegTaps = 32;
 constexpr unsigned kRegRows = 8;
 constexpr unsigned kRegBatch = 4;
 
 template <bool INT, int W>
 __global__ void __launch_bounds__(kThreads)
-h_reg_kernel(PassTables t, int32_t pixel_max, unsigned lines, const uint8_t *__restrict__ src, ptrdiff_t ss,
-             uint8_t *__restrict__ dst, ptrdiff_t ds)
+h_reg_kernel(PassTables t, int32_t pixel_max, unsigned lines, const __grid_constant__ PassPlanes P)
 {
+	ZG_PASS_PLANE
 	using S = std::conditional_t<INT, uint16_t, float>;
 	using A = std::conditional_t<INT, int32_t, float>;
 	const unsigned j = blockIdx.x * kThreads + threadIdx.x;
@@ -246,14 +261,13 @@ h_reg_kernel(PassTables t, int32_t pixel_max, unsigned lines, const uint8_t *__r
 }
 
 template <bool INT, int W = kRegTaps>
-cudaError_t launch_h_reg(const PassLaunch &l, cudaStream_t stream)
+cudaError_t launch_h_reg(const PassLaunch &l, const PassPlanes &P, cudaStream_t stream)
 {
 	if constexpr (W > 0) {
 		if (l.t.width != W)
-			return launch_h_reg<INT, W - 1>(l, stream);
-		dim3 grid((l.t.rows + kThreads - 1) / kThreads, (l.lines + kRegRows - 1) / kRegRows);
-		h_reg_kernel<INT, W><<<grid, kThreads, 0, stream>>>(l.t, l.pixel_max, l.lines, static_cast<const uint8_t *>(l.src),
-		                                                    l.src_stride, static_cast<uint8_t *>(l.dst), l.dst_stride);
+			return launch_h_reg<INT, W - 1>(l, P, stream);
+		dim3 grid((l.t.rows + kThreads - 1) / kThreads, (l.lines + kRegRows - 1) / kRegRows, l.num_planes);
+		h_reg_kernel<INT, W><<<grid, kThreads, 0, stream>>>(l.t, l.pixel_max, l.lines, P);
 		return cudaGetLastError();
 	} else {
 		return cudaErrorInvalidValue;
@@ -274,9 +288,9 @@ constexpr unsigned kRegColRows = 4;
 
 template <bool INT, int VEC, int W>
 __global__ void __launch_bounds__(kThreads)
-v_reg_kernel(PassTables t, int32_t pixel_max, unsigned plane_w, const uint8_t *__restrict__ src, ptrdiff_t ss,
-             uint8_t *__restrict__ dst, ptrdiff_t ds)
+v_reg_kernel(PassTables t, int32_t pixel_max, unsigned plane_w, const __grid_constant__ PassPlanes P)
 {
+	ZG_PASS_PLANE
 	using S = std::conditional_t<INT, uint16_t, float>;
 	using A = std::conditional_t<INT, uint32_t, float>;
 	const unsigned j0 = (blockIdx.x * kThreads + threadIdx.x) * VEC;
@@ -354,14 +368,13 @@ v_reg_kernel(PassTables t, int32_t pixel_max, unsigned plane_w, const uint8_t *_
 }
 
 template <bool INT, int VEC, int W = kRegTaps>
-cudaError_t launch_v_reg(const PassLaunch &l, cudaStream_t stream)
+cudaError_t launch_v_reg(const PassLaunch &l, const PassPlanes &P, cudaStream_t stream)
 {
 	if constexpr (W > 0) {
 		if (l.t.width != W)
-			return launch_v_reg<INT, VEC, W - 1>(l, stream);
-		dim3 grid((l.lines + kThreads * VEC - 1) / (kThreads * VEC), (l.t.rows + kRegColRows - 1) / kRegColRows);
-		v_reg_kernel<INT, VEC, W><<<grid, kThreads, 0, stream>>>(l.t, l.pixel_max, l.lines, static_cast<const uint8_t *>(l.src),
-		                                                         l.src_stride, static_cast<uint8_t *>(l.dst), l.dst_stride);
+			return launch_v_reg<INT, VEC, W - 1>(l, P, stream);
+		dim3 grid((l.lines + kThreads * VEC - 1) / (kThreads * VEC), (l.t.rows + kRegColRows - 1) / kRegColRows, l.num_planes);
+		v_reg_kernel<INT, VEC, W><<<grid, kThreads, 0, stream>>>(l.t, l.pixel_max, l.lines, P);
 		return cudaGetLastError();
 	} else {
 		return cudaErrorInvalidValue;
@@ -540,37 +553,46 @@ cudaError_t launch_pass(const PassLaunch &l, cudaStream_t stream)
 			return cudaGetLastError();
 		}
 	}
+	if (l.num_planes < 1 || l.num_planes > kPassPlanes)
+		return cudaErrorInvalidValue;
+	PassPlanes P{};
+	P.p[0] = { l.src, l.src_stride, l.dst, l.dst_stride };
+	bool vec = true;
+	for (int k = 0; k < l.num_planes; ++k) {
+		if (l.planes)
+			P.p[k] = l.planes[k];
+		vec = vec && aligned16(P.p[k].src, P.p[k].src_stride) && aligned16(P.p[k].dst, P.p[k].dst_stride);
+	}
 	if (l.horizontal && l.t.width <= kRegTaps)
-		return l.sample == Sample::U16 ? launch_h_reg<true>(l, stream) : launch_h_reg<false>(l, stream);
+		return l.sample == Sample::U16 ? launch_h_reg<true>(l, P, stream) : launch_h_reg<false>(l, P, stream);
 	if (l.horizontal) {
 		const unsigned rpb = 8;
-		dim3 grid((l.t.rows + kThreads - 1) / kThreads, (l.lines + rpb - 1) / rpb);
+		dim3 grid((l.t.rows + kThreads - 1) / kThreads, (l.lines + rpb - 1) / rpb, l.num_planes);
 		if (l.sample == Sample::U16)
-			h_u16_kernel<<<grid, kThreads, 0, stream>>>(l.t, l.pixel_max, l.lines, src, l.src_stride, dst, l.dst_stride, rpb);
+			h_u16_kernel<<<grid, kThreads, 0, stream>>>(l.t, l.pixel_max, l.lines, P, rpb);
 		else
-			h_f32_kernel<<<grid, kThreads, 0, stream>>>(l.t, l.lines, src, l.src_stride, dst, l.dst_stride, rpb);
+			h_f32_kernel<<<grid, kThreads, 0, stream>>>(l.t, l.lines, P, rpb);
 	} else {
 		const unsigned rpb = 4;
-		const bool vec = aligned16(l.src, l.src_stride) && aligned16(l.dst, l.dst_stride);
 		if (l.t.width <= kRegTaps && (l.sample == Sample::U16 || vec)) {
 			if (l.sample == Sample::F32)
-				return launch_v_reg<false, 4>(l, stream);
-			return vec ? launch_v_reg<true, 8>(l, stream) : launch_v_reg<true, 1>(l, stream);
+				return launch_v_reg<false, 4>(l, P, stream);
+			return vec ? launch_v_reg<true, 8>(l, P, stream) : launch_v_reg<true, 1>(l, P, stream);
 		}
 		if (l.sample == Sample::U16) {
 			const int V = vec ? 8 : 1;
-			dim3 grid((l.lines + kThreads * V - 1) / (kThreads * V), (l.t.rows + rpb - 1) / rpb);
+			dim3 grid((l.lines + kThreads * V - 1) / (kThreads * V), (l.t.rows + rpb - 1) / rpb, l.num_planes);
 			if (vec)
-				v_u16_kernel<8><<<grid, kThreads, 0, stream>>>(l.t, l.pixel_max, l.lines, src, l.src_stride, dst, l.dst_stride, rpb);
+				v_u16_kernel<8><<<grid, kThreads, 0, stream>>>(l.t, l.pixel_max, l.lines, P, rpb);
 			else
-				v_u16_kernel<1><<<grid, kThreads, 0, stream>>>(l.t, l.pixel_max, l.lines, src, l.src_stride, dst, l.dst_stride, rpb);
+				v_u16_kernel<1><<<grid, kThreads, 0, stream>>>(l.t, l.pixel_max, l.lines, P, rpb);
 		} else {
 			const int V = vec ? 4 : 1;
-			dim3 grid((l.lines + kThreads * V - 1) / (kThreads * V), (l.t.rows + rpb - 1) / rpb);
+			dim3 grid((l.lines + kThreads * V - 1) / (kThreads * V), (l.t.rows + rpb - 1) / rpb, l.num_planes);
 			if (vec)
-				v_f32_kernel<4><<<grid, kThreads, 0, stream>>>(l.t, l.lines, src, l.src_stride, dst, l.dst_stride, rpb);
+				v_f32_kernel<4><<<grid, kThreads, 0, stream>>>(l.t, l.lines, P, rpb);
 			else
-				v_f32_kernel<1><<<grid, kThreads, 0, stream>>>(l.t, l.lines, src, l.src_stride, dst, l.dst_stride, rpb);
+				v_f32_kernel<1><<<grid, kThreads, 0, stream>>>(l.t, l.lines, P, rpb);
 		}
 	}
 	return cudaGetLastError();
