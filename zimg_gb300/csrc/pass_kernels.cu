@@ -1,6 +1,6 @@
-// Single-pass resize kernels: one horizontal or vertical banded pass over a
-// whole plane, for any tap count. These are the general path (and the
-// building block of two-pass conversions whose intermediate lives in HBM).
+// Single-pass resize kernels: one horizontal or vertical banded pass over whole
+// planes, for any tap count. These are the general path (and the building
+// block of two-pass conversions whose intermediate lives in HBM).
 //
 // Arithmetic, per output sample, is exactly zimg's C path
 // (src/zimg/resize/resize_impl.cpp:31-114):
@@ -97,59 +97,31 @@ v_u16_kernel(PassTables t, int32_t pixel_max, unsigned plane_w, const __grid_con
 	}
 }
 
-template <int VEC>
+// Planes that are not 16-byte aligned, a column a thread (see v_reg_kernel and
+// v_f32_dense_kernel for the others).
 __global__ void __launch_bounds__(kThreads)
-v_f32_kernel(PassTables t, unsigned plane_w, const __grid_constant__ PassPlanes P,
-             unsigned rows_per_block)
+v_f32_kernel(PassTables t, unsigned plane_w, const __grid_constant__ PassPlanes P, unsigned rows_per_block)
 {
 	ZG_PASS_PLANE
-	const unsigned j0 = (blockIdx.x * kThreads + threadIdx.x) * VEC;
-	if (j0 >= plane_w)
+	const unsigned j = blockIdx.x * kThreads + threadIdx.x;
+	if (j >= plane_w)
 		return;
-	const bool full = j0 + VEC <= plane_w;
 	const unsigned i0 = blockIdx.y * rows_per_block;
 	const unsigned i1 = min(i0 + rows_per_block, t.rows);
 
 	for (unsigned i = i0; i < i1; ++i) {
-		const unsigned top = __ldg(t.left + i);
 		const float *c = t.f32 + static_cast<size_t>(i) * t.width;
-		float acc[VEC];
-#pragma unroll
-		for (int v = 0; v < VEC; ++v)
-			acc[v] = 0.0f;
-
-		const uint8_t *row = src + static_cast<ptrdiff_t>(top) * ss + static_cast<size_t>(j0) * 4;
-		for (unsigned k = 0; k < t.width; ++k, row += ss) {
-			const float ck = __ldg(c + k);
-			if (VEC == 4 && full) {
-				float4 q = __ldg(reinterpret_cast<const float4 *>(row));
-				acc[0] = __fmaf_rn(ck, q.x, acc[0]);
-				acc[1] = __fmaf_rn(ck, q.y, acc[1]);
-				acc[2] = __fmaf_rn(ck, q.z, acc[2]);
-				acc[3] = __fmaf_rn(ck, q.w, acc[3]);
-			} else {
-				const float *rf = reinterpret_cast<const float *>(row);
-#pragma unroll
-				for (int v = 0; v < VEC; ++v)
-					if (full || j0 + v < plane_w)
-						acc[v] = __fmaf_rn(ck, __ldg(rf + v), acc[v]);
-			}
-		}
-
-		float *out = reinterpret_cast<float *>(dst + static_cast<ptrdiff_t>(i) * ds) + j0;
-		if (VEC == 4 && full) {
-			*reinterpret_cast<float4 *>(out) = make_float4(acc[0], acc[1], acc[2], acc[3]);
-		} else {
-#pragma unroll
-			for (int v = 0; v < VEC; ++v)
-				if (full || j0 + v < plane_w)
-					out[v] = acc[v];
-		}
+		const uint8_t *row = src + static_cast<ptrdiff_t>(__ldg(t.left + i)) * ss + static_cast<size_t>(j) * 4;
+		float acc = 0.0f;
+		for (unsigned k = 0; k < t.width; ++k, row += ss)
+			acc = __fmaf_rn(__ldg(c + k), __ldg(reinterpret_cast<const float *>(row)), acc);
+		reinterpret_cast<float *>(dst + static_cast<ptrdiff_t>(i) * ds)[j] = acc;
 	}
 }
 
 // -------------------------------------------------------------- horizontal --
-// Thread = one output column for `rows_per_block` lines; its taps stay in L1.
+// Filters longer than kRegTaps: thread = one output column for
+// `rows_per_block` lines; its taps stay in L1.
 __global__ void __launch_bounds__(kThreads)
 h_u16_kernel(PassTables t, int32_t pixel_max, unsigned lines, const __grid_constant__ PassPlanes P,
              unsigned rows_per_block)
@@ -281,8 +253,8 @@ cudaError_t launch_h_reg(const PassLaunch &l, const PassPlanes &P, cudaStream_t 
 //   u16 1920x1080 -> 1920x721, 10 taps          7.4 -> 4.5 us
 //   u16 1919x1080 -> 1919x721 (2-byte loads)    8.5 -> 6.8 us
 //   f32 1920x1080 -> 1920x540, 16 taps          9.8 -> 5.4 us
-//   f32 3840x2160 -> 3840x1080, 8 taps         15.7 -> 12.4 us
-// f32 planes that are not 16-byte aligned stay with v_f32_kernel<1>, whose
+//   f32 3840x2160 -> 3840x1080, 8 taps         15.7 -> 13.0 us
+// f32 planes that are not 16-byte aligned stay with v_f32_kernel, whose
 // 4-byte loads came to 18.3 us at 3839x2160 -> 3839x1080, 18.6 us here.
 constexpr unsigned kRegColRows = 4;
 
@@ -587,12 +559,8 @@ cudaError_t launch_pass(const PassLaunch &l, cudaStream_t stream)
 			else
 				v_u16_kernel<1><<<grid, kThreads, 0, stream>>>(l.t, l.pixel_max, l.lines, P, rpb);
 		} else {
-			const int V = vec ? 4 : 1;
-			dim3 grid((l.lines + kThreads * V - 1) / (kThreads * V), (l.t.rows + rpb - 1) / rpb, l.num_planes);
-			if (vec)
-				v_f32_kernel<4><<<grid, kThreads, 0, stream>>>(l.t, l.lines, P, rpb);
-			else
-				v_f32_kernel<1><<<grid, kThreads, 0, stream>>>(l.t, l.lines, P, rpb);
+			dim3 grid((l.lines + kThreads - 1) / kThreads, (l.t.rows + rpb - 1) / rpb, l.num_planes);
+			v_f32_kernel<<<grid, kThreads, 0, stream>>>(l.t, l.lines, P, rpb);
 		}
 	}
 	return cudaGetLastError();
