@@ -625,10 +625,10 @@ fused_kernel(const FusedJob *__restrict__ jobs, int num_jobs, int total_items, c
 			const Item it = make_item(J, t, c_end);
 			t += it.steps;
 
-			// lines and records of a step, one cp.async group; `next`, `slot`:
-			// the first line not yet in the ring and its slot
+			// lines of a step, and its records; `next`, `slot`: the first line
+			// not yet in the ring and its slot
 			int next, slot;
-			auto load_step = [&](int k) {
+			auto load_step_lines = [&](int k) {
 				const int hi = __ldg(it.ranges + it.step0 + k).y;
 				if (hi > next) {
 					load_lines<E>(it, next, hi, in, it.in_rows, slot);
@@ -637,8 +637,14 @@ fused_kernel(const FusedJob *__restrict__ jobs, int num_jobs, int total_items, c
 						slot -= it.in_rows;
 					next = hi;
 				}
+			};
+			auto load_step_records = [&](int k) {
 				load_records(it.records + static_cast<size_t>(it.step0 + k) * kRecordBytes,
 				             records + (k & 1) * kRecordBytes, kRecordBytes);
+			};
+			auto load_step = [&](int k) {  // both, one cp.async group
+				load_step_lines(k);
+				load_step_records(k);
 				cp_async_commit();
 			};
 			next = __ldg(it.ranges + it.step0).x;
@@ -669,15 +675,25 @@ fused_kernel(const FusedJob *__restrict__ jobs, int num_jobs, int total_items, c
 			for (int k = 0; k < it.steps; ++k) {
 				// early: the next step's lines go into slots that no line of
 				// this one's windows holds; late: only after its vertical
-				// pass (H first: horizontal pass)
+				// pass (H first: horizontal pass). The next step's records
+				// replace those of the step before this one, whose readers
+				// have left them at the step's last barrier (V first) or at
+				// the next one (H first: the vertical pass comes last).
 				const bool more = k + 1 < it.steps;
 				if (more && !it.late) {
-					load_step(k + 1);
+					load_step_lines(k + 1);
+					if constexpr (!H_FIRST)
+						load_step_records(k + 1);
+					cp_async_commit();
 					cp_async_wait<1>();
 				} else {
 					cp_async_wait<0>();
 				}
 				__syncthreads();
+				if (H_FIRST && more && !it.late) {
+					load_step_records(k + 1);
+					cp_async_commit();
+				}
 				const int row0 = (it.step0 + k) * kStepRows;
 				const uint32_t rec = records_a + (k & 1) * kRecordBytes;
 				if constexpr (H_FIRST) {
