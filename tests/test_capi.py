@@ -169,3 +169,19 @@ def test_wide_forms_used_starts_empty(lib):
     t.start()
     t.join()
     assert out == [0, 0]
+
+
+@pytest.mark.parametrize("mask", [0, 7, 0x7FFFFFFF, 0xFFFFFFFF, -1, -8, (1 << 32) | 3, True])
+def test_image_buffer_takes_the_masks_that_ctypes_takes(mask):
+    """BUFFER_MAX is also -1; a mask is the low 32 bits of any int."""
+    from zimg_gb300 import capi
+    want = capi.ImageBuffer()
+    want.version = capi.API_VERSION_2_4
+    fields = []
+    for i in range(4):
+        want.plane[i] = capi._PlaneC(0x7F0012340000 + i, -(1 << 40) - 64 * i, mask)
+        fields += [0x7F0012340000 + i, -(1 << 40) - 64 * i, mask]
+    got = capi.image_buffer(fields)
+    assert got.version == want.version
+    for g, w in zip(got.plane, want.plane):
+        assert (g.data, g.stride, g.mask) == (w.data, w.stride, w.mask)

@@ -115,7 +115,10 @@ _IMAGE_BUFFER = struct.Struct("@I" + "PqI" * 4 + "0P")  # ImageBuffer's layout
 
 
 def image_buffer(fields) -> ImageBuffer:
-    """An ImageBuffer of four planes' (data, stride, mask), in one list."""
+    """An ImageBuffer of four planes' (data, stride, mask), in one list; masks
+    are taken to 32 bits, as ctypes takes them (BUFFER_MAX is also -1)."""
+    for i in range(2, len(fields), 3):
+        fields[i] &= BUFFER_MAX
     return ImageBuffer.from_buffer_copy(_IMAGE_BUFFER.pack(API_VERSION_2_4, *fields))
 
 # zg_graph_callback: int (*)(void *user, unsigned i, unsigned left, unsigned right)
