@@ -115,8 +115,13 @@ ZG_API void zg_clear_last_error(void);
  * variant chosen by `plane` mod 4, dither.cpp:137-210), RANDOM (zimg's 64x64
  * blue-noise matrix at the offsets chosen by `plane` mod 4,
  * dither.cpp:219-234) and ERROR_DIFFUSION (Floyd-Steinberg over the whole
- * plane, dither.cpp:59-85 and 291-345; one thread block per plane runs the
- * lines as a wavefront) are built. ERROR_DIFFUSION on a plane of more than
+ * plane, dither.cpp:59-85 and 291-345; the lines run as a wavefront, on a
+ * cluster of up to 8 thread blocks per plane, on one block where a line has
+ * more than about 21,000 samples) are built. The cluster's blocks wait for
+ * each other's errors. Such a wait ends after 0.25 s of the clock and another
+ * 32 ms or more of the kernel's own running time, so that a launch always
+ * ends; the plane is then wrong although the call has succeeded, and bit 16
+ * of zg_pipeline_status tells once the stream is idle. ERROR_DIFFUSION on a plane of more than
  * 32 x 32 lines whose width leaves no launch shape within a block's shared
  * memory (from about 18,000 to 32,000 columns, by height) returns
  * ZG_ERROR_UNSUPPORTED_OPERATION. A limited-range format below 8 bits returns
@@ -236,13 +241,15 @@ ZG_API zg_error_code zg_unresize_process(const zg_unresize *u, const void *src, 
  * cleared. No zimg counterpart (zimg has no asynchronous device work). */
 ZG_API int zg_pipeline_status(int reset);
 
-/* Test hook for the bounded waits of the chained u16 kernel's TMA form
- * (current device): from the next launch on, CTA 0's producer skips group
- * drop_group of its pipeline without arming that group's stage (-1: none),
- * and every wait of that kernel gives up after wait_ns nanoseconds (0: the
- * default 0.25 s). A consumer wait then runs out, the kernel returns and
- * zg_pipeline_status reports cause 1. Returns 0, or -1 when the device
- * words cannot be written. Not for production use; no zimg counterpart. */
+/* Test hook for the bounded waits of the chained u16 kernel's TMA form and
+ * of the error diffusion (current device): from the next launch on, CTA 0's
+ * producer skips group drop_group of its pipeline without arming that
+ * group's stage (-1: none), a diffused plane's first 32 lines do not hand on
+ * the errors of their drop_group-th 16 steps, and every wait of those kernels
+ * gives up after wait_ns nanoseconds (0: the default 0.25 s). A wait then
+ * runs out, the kernel returns and zg_pipeline_status reports cause 1, or bit
+ * 16. Returns 0, or -1 when the device words cannot be written. Not for
+ * production use; no zimg counterpart. */
 ZG_API int zg_debug_pipeline_fault(int drop_group, unsigned long long wait_ns);
 
 /* The forms that ran the FP32 wide-filter passes enqueued by this host

@@ -109,6 +109,34 @@ def test_error_diffusion_hand_off_edges(cuda, oracle, h, w):
         np.testing.assert_array_equal(got, oracle.depth_convert(src, fin, fout, "error_diffusion", 0))
 
 
+@pytest.mark.parametrize("h,w,chunk", [(1080, 1920, 0), (1080, 1920, 57), (270, 480, 35), (40, 100, 2), (640, 9000, 300)])
+def test_error_diffusion_wait_runs_out(cuda, lib, oracle, h, w, chunk):
+    """A hand-off that never comes (the first band's of one chunk, left out by
+    the test hook): the launch ends, bit 16 of the pipelines' status says so
+    until it is reset, and the next conversion is right again."""
+    import time
+    import torch
+    from oracle.oracle import PixelFormat as PF
+    fin, fout = PF("word", 10), PF("byte", 8)
+    src = make_src(np.random.default_rng(h + w + chunk), fin, h, w, special=False)
+    want = oracle.depth_convert(src, fin, fout, "error_diffusion", 0)
+    got, _ = convert(src, fin, fout, "error_diffusion", 0)
+    np.testing.assert_array_equal(got, want)
+    assert lib.zg_debug_pipeline_fault(chunk, 1000000) == 0
+    try:
+        t0 = time.time()
+        convert(src, fin, fout, "error_diffusion", 0)
+        torch.cuda.synchronize()
+        seconds = time.time() - t0
+        status = [int(lib.zg_pipeline_status(r)) for r in (0, 1, 0)]
+    finally:
+        assert lib.zg_debug_pipeline_fault(-1, 0) == 0
+    assert status == [1 << 16, 1 << 16, 0]
+    assert seconds < 5.0
+    got, _ = convert(src, fin, fout, "error_diffusion", 0)
+    np.testing.assert_array_equal(got, want)
+
+
 def test_error_diffusion_non_finite(cuda, oracle):
     """zimg's C path keeps a NaN through the clamp, stores 0 for it and
     carries its NaN error to the samples after and below it; infinities clamp

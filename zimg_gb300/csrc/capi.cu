@@ -268,7 +268,7 @@ int zg_pipeline_status(int reset)
 
 int zg_debug_pipeline_fault(int drop_group, unsigned long long wait_ns)
 {
-	return chain_tma_set_fault(drop_group, wait_ns);
+	return chain_tma_set_fault(drop_group, wait_ns) || ed_set_fault(drop_group, wait_ns) ? -1 : 0;
 }
 
 zg_error_code zg_get_last_error(char *err_msg, size_t n)

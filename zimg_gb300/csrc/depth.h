@@ -76,6 +76,9 @@ size_t ed_smem_bytes(int warps, int ring);
 cudaError_t launch_error_diffusion(const EdLaunch &L, cudaStream_t stream);
 // Nonzero when a hand-off wait of the clustered form ran out (optionally reset); -1 when unreadable.
 int ed_wait_error(bool reset);
+// Test hook of that form: a plane's first band leaves out the hand-off of chunk
+// drop_chunk (-1: none); waits give up after wait_ns (0: the default).
+int ed_set_fault(int drop_chunk, unsigned long long wait_ns);
 
 } // namespace zg
 

@@ -229,9 +229,10 @@ __global__ void __launch_bounds__(kMaxWarps * 32) ed_kernel(const __grid_constan
 // band). Plain stores and a flag with release order instead cost the writer
 // 900 cycles a chunk. A buffer holds a whole line, so the writer never waits:
 // a warp's next band is written only by a band that depends on every sample
-// the warp's current band has read. Waits are bounded (kWaitNs): one that runs
-// out is recorded in g_ed_wait_error and the warp goes on without waiting, so
-// that the launch ends.
+// the warp's current band has read. Waits are bounded (hand_off_wait): one that
+// runs out is recorded in g_ed_wait_error and the warp goes on without waiting,
+// so that the launch ends, its outputs wrong from there on; the cluster's blocks
+// then stay until every hand-off on its way must have landed (leave_cluster).
 //
 // Measured, a 1920x1080 4:2:0 frame, WORD 10 bits -> BYTE, its planes side by
 // side: 1,185 us in ed_kernel, 224 us here (about 1,250 cycles a chunk; the
@@ -248,6 +249,10 @@ constexpr int kAheadChunks = kReadAhead / kEdChunk + 1;  // so chunk k needs the
 static_assert(kReadAhead % kEdChunk == 0, "receive reads start on chunk boundaries");
 
 __device__ int g_ed_wait_error;
+// Wait limit in ns (0: kWaitNs), and a test hook: the chunk whose hand-off a
+// plane's first band leaves out (-1: none).
+__device__ unsigned long long g_ed_wait_ns;
+__device__ int g_ed_drop_chunk = -1;
 
 // floats of one warp's receive buffer for lines of `width` samples: a slot
 // per band step, and the zeros that the last chunks read past them
@@ -284,6 +289,47 @@ __device__ __forceinline__ uint32_t cluster_addr(const void *p, unsigned rank)
 __device__ __forceinline__ void cluster_barrier()
 {
 	asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+
+// Wait for a hand-off. Gives up (false) after the limit in ns of the clock and
+// then kOwnPolls polls of the warp's own, a microsecond apart: while the GPU
+// runs another process's work the clock goes on, but neither side of a hand-off
+// does. (A call of its own: inlined, it costs the loading warp spills.)
+constexpr int kOwnPolls = 1 << 15;
+
+__device__ __noinline__ bool hand_off_pending(uint64_t *bar, unsigned parity)
+{
+	if (mbar_wait(bar, parity, g_ed_wait_ns ? g_ed_wait_ns : kWaitNs))
+		return true;
+	for (int i = 0; i < kOwnPolls; ++i) {
+		if (mbar_test(bar, parity))
+			return true;
+		__nanosleep(1000);
+	}
+	return false;
+}
+
+__device__ __forceinline__ bool hand_off_wait(uint64_t *bar, unsigned parity)
+{
+	return mbar_test(bar, parity) || hand_off_pending(bar, parity);
+}
+
+// A word of a block's shared memory that is 0 until a warp of the cluster has
+// given up a wait: the last float of its first warp's receive buffer, beyond
+// what a line reads.
+__device__ __forceinline__ float *lost_word(float *smem, int chunks)
+{
+	return smem + kWarpFloats + receive_floats(chunks) - 1;
+}
+
+// The end of a block: none leaves while another may write to its shared memory.
+// All hand-offs were sent by then, and waited for unless a warp has given up;
+// then they get a millisecond, thousands of times what they take.
+__device__ __forceinline__ void leave_cluster(float *smem, int chunks)
+{
+	cluster_barrier();
+	for (int i = 0; i < 1000 && *static_cast<volatile float *>(lost_word(smem, chunks)) != 0.0f; ++i)
+		__nanosleep(1000);
 }
 
 // Clamps that keep a NaN (PTX max.NaN / min.NaN), as zimg's std::clamp does.
@@ -360,7 +406,8 @@ __device__ __forceinline__ bool whole_chunk(const EdPlane &p, int band, int k)
 // The loading warp: inputs into tile_in, and the wait for the errors that the
 // computing warp reads next.
 template <class T>
-__device__ __forceinline__ void ed_load(const EdPlane &p, int first_band, int nw, int warp, const EdShared &m)
+__device__ __forceinline__ void ed_load(const EdPlane &p, int first_band, int nw, int warp, const EdShared &m, float *lost,
+                                        int cluster)
 {
 	const EdLane l;
 	const int lane = threadIdx.x & 31;
@@ -419,9 +466,11 @@ __device__ __forceinline__ void ed_load(const EdPlane &p, int first_band, int nw
 			if (band == 0)
 				return;
 			for (const int need = min(k + kAheadChunks, chunks); arrived < need && !gave_up; ++arrived) {
-				if (!__all_sync(0xffffffffu, mbar_wait(m.bars + arrived, phase))) {
+				if (!__all_sync(0xffffffffu, hand_off_wait(m.bars + arrived, phase))) {
 					gave_up = true;
 					atomicExch(&g_ed_wait_error, 1);
+					if (lane < cluster)
+						asm volatile("st.shared::cluster.f32 [%0], %1;\n" ::"r"(cluster_addr(lost, lane)), "f"(1.0f) : "memory");
 				} else if (lane == 0) {
 					mbar_arrive_expect_tx(m.bars + arrived, kEdChunk * 4);
 				}
@@ -460,6 +509,7 @@ __device__ __forceinline__ void ed_store(const EdPlane &p, int first_band, int n
 	const int lane = threadIdx.x & 31;
 	const int W = p.width, H = p.height, chunks = band_chunks(W);
 	const ptrdiff_t step = 2 * p.dst_stride - 2 * kEdLag * static_cast<ptrdiff_t>(sizeof(U));
+	const int drop = first_band == 0 ? g_ed_drop_chunk : -1;
 	for (int band = first_band; band < p.bands; band += nw) {
 		const int rows_left = H - band * kBandLines - l.half;  // line 2j + half exists iff 2j < rows_left
 		char *out0 = static_cast<char *>(p.dst) + static_cast<ptrdiff_t>(band * kBandLines + l.half) * p.dst_stride +
@@ -467,7 +517,7 @@ __device__ __forceinline__ void ed_store(const EdPlane &p, int first_band, int n
 		chunk_barrier(warp);
 		for (int k = 0; k < chunks; ++k) {
 			chunk_barrier(warp);  // chunk k is done
-			if (lane < kEdChunk / 4 && band + 1 < p.bands) {
+			if (lane < kEdChunk / 4 && band + 1 < p.bands && (band > 0 || k != drop)) {
 				const float4 v = *reinterpret_cast<const float4 *>(m.last + (k & 1) * kEdChunk + 4 * lane);
 				asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];\n" ::"r"(
 					             next_recv + static_cast<uint32_t>(k * kEdChunk + 4 * lane) * 4),
@@ -533,8 +583,8 @@ __global__ void __launch_bounds__(kClusterThreads, 1) ed_cluster_kernel(const __
 	cluster_barrier();
 
 	if (role == 1) {
-		ed_load<T>(p, g, nw, warp, m);
-		cluster_barrier();
+		ed_load<T>(p, g, nw, warp, m, lost_word(ed_smem, chunks), cluster);
+		leave_cluster(ed_smem, chunks);
 		return;
 	}
 	if (role >= 2) {
@@ -542,7 +592,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) ed_cluster_kernel(const __
 		if (role == 2)
 			ed_store<U>(p, g, nw, warp, m, cluster_addr(next_recv, next / C),
 			            cluster_addr(next_recv + receive_floats(chunks), next / C));
-		cluster_barrier();
+		leave_cluster(ed_smem, chunks);
 		return;
 	}
 	const float vmax = p.vmax;
@@ -617,7 +667,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) ed_cluster_kernel(const __
 			chunk_barrier(warp);
 		}
 	}
-	cluster_barrier();  // no block leaves while another may write to its shared memory
+	leave_cluster(ed_smem, chunks);
 }
 
 // Chunk times until a plane's last band ends, with nw warps: a band starts
@@ -713,6 +763,14 @@ int round_up(int v, int m)
 }
 
 } // namespace
+
+int ed_set_fault(int drop_chunk, unsigned long long wait_ns)
+{
+	if (cudaMemcpyToSymbol(g_ed_drop_chunk, &drop_chunk, sizeof(drop_chunk)) != cudaSuccess ||
+	    cudaMemcpyToSymbol(g_ed_wait_ns, &wait_ns, sizeof(wait_ns)) != cudaSuccess)
+		return -1;
+	return 0;
+}
 
 int ed_wait_error(bool reset)
 {

@@ -37,8 +37,8 @@ __device__ __forceinline__ unsigned long long global_ns()
 }
 
 // Wait until the phase of the given parity has completed; false when the
-// wait has lasted kWaitNs.
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, unsigned parity)
+// wait has lasted `limit` ns.
+__device__ __forceinline__ bool mbar_wait(uint64_t *bar, unsigned parity, unsigned long long limit = kWaitNs)
 {
 	const unsigned a = smem_addr(bar);
 	unsigned long long t0 = 0;
@@ -58,10 +58,25 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, unsigned parity)
 			const unsigned long long t = global_ns();
 			if (i == 0)
 				t0 = t;
-			else if (t - t0 > kWaitNs)
+			else if (t - t0 > limit)
 				return false;
 		}
 	}
+}
+
+// Whether the phase of the given parity has completed.
+__device__ __forceinline__ bool mbar_test(uint64_t *bar, unsigned parity)
+{
+	unsigned done;
+	asm volatile("{\n"
+	             "  .reg .pred p;\n"
+	             "  mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+	             "  selp.u32 %0, 1, 0, p;\n"
+	             "}\n"
+	             : "=r"(done)
+	             : "r"(smem_addr(bar)), "r"(parity)
+	             : "memory");
+	return done != 0;
 }
 
 // One box of the tensor map at (x, y) into shared memory, completing on bar.
