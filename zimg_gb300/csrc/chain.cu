@@ -14,6 +14,7 @@ namespace {
 constexpr int kChainKVMax = 3;
 constexpr int kChainKHMax = 4;
 constexpr int kChainWindow = 248;  // samples of a strip's lines
+constexpr size_t kChainSmem = 110 * 1024;  // two CTAs per SM
 
 size_t align_up(size_t x, size_t a)
 {
@@ -189,51 +190,55 @@ bool plan_chain(const FilterTable &first, const FilterTable &second, bool h_firs
 		return false;
 	const int strip_w = strip_tiles * chain_detail::kTileW;
 
-	// prefetch depth: about 32 KB of source lines in flight per CTA
+	// prefetch depth: about 32 KB of source lines in flight per CTA, and no more
+	// than the shared memory holds as they are (lines, stages, staged tiles,
+	// bases): the layout, whose ring is a power of two blocks, makes do with
+	// fewer lines and stages than a deeper pipeline asks for
 	auto hi_of = [&](int g) { return gbase[std::min(g, groups - 1)] + 16 * KV; };
 	int new_lines = 1;
 	for (int g = 1; g < groups; ++g)
 		new_lines = std::max(new_lines, hi_of(g) - hi_of(g - 1));
 	const int group_bytes = std::max(1, new_lines * max_pxa * 2);
+	const int pitch = (max_pxa + 15) / 16 * 16 + 8;
+	int ahead = std::max(1, std::min(8, (32 * 1024 + group_bytes - 1) / group_bytes)), ring = 0;
+	for (;; --ahead) {
+		// a warp may read group g while loads of group g + 1 + ahead land
+		ring = 16 * KV;
+		for (int g = 0; g < groups; ++g)
+			ring = std::max(ring, hi_of(g + 1 + ahead) - gbase[g]);
+		const size_t bytes = static_cast<size_t>(ring) * pitch * 2 + static_cast<size_t>(ahead + 2) * KV * 1024 +
+		                     static_cast<size_t>(chain_detail::kMaxWarps) * per_warp * chain_detail::kTileStage +
+		                     static_cast<size_t>(groups) * 4;
+		if (ahead == 1 || bytes <= kChainSmem)
+			break;
+	}
 	FusedPlan &p = *out;
 	p = FusedPlan{};
 	FusedJob &J = p.job;
-	bool fits = false;
-	for (int ahead = std::max(1, std::min(8, (32 * 1024 + group_bytes - 1) / group_bytes)); ahead >= 1; --ahead) {
-		// a warp may read group g while loads of group g + 1 + ahead land
-		int ring = 16 * KV;
-		for (int g = 0; g < groups; ++g)
-			ring = std::max(ring, hi_of(g + 1 + ahead) - gbase[g]);
-		J = FusedJob{};
-		J.h_first = h_first ? 1 : 0;
-		J.kind = static_cast<int>(FusedKind::U16_EXACT);
-		J.src_w = static_cast<int>(src_w);
-		J.src_h = static_cast<int>(src_h);
-		J.dst_w = static_cast<int>(dst_w);
-		J.dst_h = static_cast<int>(dst_h);
-		J.strips = strips;
-		J.strip_w = strip_w;
-		J.groups = groups;
-		J.seg_groups = 1;  // work units: (strip, group) pairs, split evenly over the CTAs
-		J.segments = groups;
-		J.step_groups = 1;
-		J.in_rows = ring;
-		J.ring_rows = 1;
-		J.hw = KH;
-		J.vs = KV;
-		J.depth = ahead;
-		p.max_pxa = max_pxa;
-		p.depth = ahead;
-		p.mma = true;
-		p.chain = true;
-		const FusedPlan *pp = &p;
-		SmemLayout layout;
-		if (chain_tma_layout(&pp, 1, &layout)) {
-			fits = true;
-			break;
-		}
-	}
-	if (!fits)
+	J.h_first = h_first ? 1 : 0;
+	J.kind = static_cast<int>(FusedKind::U16_EXACT);
+	J.src_w = static_cast<int>(src_w);
+	J.src_h = static_cast<int>(src_h);
+	J.dst_w = static_cast<int>(dst_w);
+	J.dst_h = static_cast<int>(dst_h);
+	J.strips = strips;
+	J.strip_w = strip_w;
+	J.groups = groups;
+	J.seg_groups = 1;  // work units: (strip, group) pairs, split evenly over the CTAs
+	J.segments = groups;
+	J.step_groups = 1;
+	J.in_rows = ring;
+	J.ring_rows = 1;
+	J.hw = KH;
+	J.vs = KV;
+	J.depth = ahead;
+	p.max_pxa = max_pxa;
+	p.depth = ahead;
+	p.mma = true;
+	p.chain = true;
+	const FusedPlan *pp = &p;
+	SmemLayout layout;
+	if (!chain_tma_layout(&pp, 1, &layout))
 		return false;
 
 	// tables: h fragments | hstart | v fragments | gbase | win_col
