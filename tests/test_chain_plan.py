@@ -93,3 +93,16 @@ def test_prefetch_depth_fits_unshrunk(plan):
         held = p["lines"] * pitch * 2 + (p["depth"] + 2) * p["kv"] * 1024 + tiles * 800 + p["groups"] * 4
         assert held <= 110 * 1024, (job, p, held)
     assert n > 100
+
+
+def test_small_windows_keep_seven_warps_busy(plan):
+    """Windows of 16 lines and 16 columns: strips of seven warps' tiles, four a
+    warp where the strip's lines fit one copy, else two."""
+    n = {2: 0, 4: 0}
+    for job, p in zip(jobs_of_ratios(), plan(jobs_of_ratios())):
+        if not p["variant"] or (p["kv"], p["kh"]) != (1, 1):
+            continue
+        tiles = p["strip_w"] / (7 * 16)
+        assert tiles in (2, 4), (job, p)
+        n[int(tiles)] += 1
+    assert min(n.values()) > 20

@@ -162,6 +162,44 @@ def test_chained_kernel_any_alignment(cuda, oracle, sw, sh, dw, dh, kind, pad, o
             np.testing.assert_array_equal(q.cpu().numpy().view(np.uint16), want)
 
 
+@pytest.mark.parametrize("sw,sh,dw,dh,kind", [
+    (640, 48, 800, 60, "bilinear"),    # H first, strips of 224 columns: four, the last one partial
+    (256, 33, 448, 58, "bicubic"),     # two strips, whole
+    (257, 33, 449, 58, "bicubic"),     # one column past them
+    (300, 95, 330, 104, "bilinear"),   # nearly 1x
+    (900, 40, 1283, 57, "spline16")])  # six strips
+@pytest.mark.parametrize("pad,offset,flip", [(0, 0, False), (1, 1, False), (2, 4, True), (8, 8, False)])
+def test_chained_kernel_narrow_strips(cuda, oracle, sw, sh, dw, dh, kind, pad, offset, flip):
+    """Windows of 16 lines and columns in strips of two tiles a warp."""
+    test_chained_kernel_any_alignment(cuda, oracle, sw, sh, dw, dh, kind, pad, offset, flip)
+
+
+def test_narrow_strips_in_a_mixed_batch(cuda, oracle):
+    """Jobs of two and of four tiles a warp, downscales and copies in one launch."""
+    import torch
+    import zimg_gb300 as zg
+    rng = np.random.default_rng(0x7C)
+    jobs = [(640, 48, 800, 60), (320, 64, 640, 128), (640, 96, 400, 64), (208, 160, 384, 176), (320, 64, 320, 64)] * 3
+    convs, srcs, dsts, want = [], [], [], []
+    for sw, sh, dw, dh in jobs:
+        src = rng.integers(0, 1024, size=(sh, sw), dtype=np.uint16)
+        want.append(oracle.resize_plane(src, dw, dh, "bilinear", depth=10, mode="c", nthreads=16))
+        convs.append(zg.ResizeConversion(sw, sh, "word").set_depth(10).set_filter("bilinear").set_dst_width(dw)
+                     .set_dst_height(dh))
+        srcs.append(torch.from_numpy(src.view(np.int16)).cuda())
+        dsts.append(torch.empty(dh, dw, dtype=torch.int16, device="cuda"))
+    b = zg.Batch(convs)
+    b.set_io(srcs, dsts)
+    assert b.launch_count == 1
+    for run in (b.process, b.process_graph):
+        for d in dsts:
+            d.zero_()
+        run()
+        torch.cuda.synchronize()
+        for k, (d, w) in enumerate(zip(dsts, want)):
+            np.testing.assert_array_equal(d.cpu().numpy().view(np.uint16), w, err_msg=str(jobs[k]))
+
+
 FAULT_CHILD = r"""
 import json, os, sys, time
 import numpy as np

@@ -240,7 +240,7 @@ double unit_cost(const zg_resize *r, const FusedJob &j, bool copy)
 	const double units = std::max(1, fused_items(j));
 	double eff = 0.9;
 	if (!copy) {
-		const bool hf = j.variant >= 12;
+		const bool hf = j.h_first != 0;
 		const double reuse = r->fplan.reuse_frac;
 		eff = hf ? 1.0 / (reuse / 0.70 + (1.0 - reuse) / 0.38) : 0.47;
 	}

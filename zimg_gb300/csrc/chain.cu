@@ -11,8 +11,8 @@ namespace zg {
 
 namespace {
 
-constexpr int kChainKVMax = 3;
-constexpr int kChainKHMax = 4;
+using chain_detail::kChainKHMax;
+using chain_detail::kChainKVMax;
 constexpr int kChainWindow = 248;  // samples of a strip's lines
 constexpr size_t kChainSmem = 110 * 1024;  // two CTAs per SM
 
@@ -89,11 +89,6 @@ void a_fragments(const std::vector<float> (&dense)[2], int K, uint32_t *out)
 
 } // namespace
 
-int chain_variant(bool h_first, int kv, int kh)
-{
-	return 200 + (h_first ? kChainKVMax * kChainKHMax : 0) + (kv - 1) * kChainKHMax + (kh - 1);
-}
-
 bool plan_chain(const FilterTable &first, const FilterTable &second, bool h_first, unsigned depth, unsigned src_w,
                 unsigned src_h, unsigned dst_w, unsigned dst_h, FusedPlan *out)
 {
@@ -164,8 +159,9 @@ bool plan_chain(const FilterTable &first, const FilterTable &second, bool h_firs
 	// strips of up to 7 warps' tiles whose source columns [lo, hi), lo a
 	// multiple of 8, fit the widest window that both ways of copying lines
 	// take (31 chunks of 16 bytes for a warp; a tensor copy's 256 samples)
-	const int per_warp = chain_detail::tiles_per_warp(KV, KH);
-	int strip_tiles = chain_detail::warps_per_cta(h_first) * per_warp, strips = 0, max_pxa = 0;
+	int code = (h_first ? chain_detail::kChainShapes : 0) + (KV - 1) * kChainKHMax + (KH - 1);
+	int per_warp = chain_detail::tiles_per_warp(KV, KH);
+	int strip_tiles = chain_detail::kWsWarps * per_warp, strips = 0, max_pxa = 0;
 	std::vector<int> win_col;
 	for (; strip_tiles >= per_warp; strip_tiles -= per_warp) {
 		strips = (tiles + strip_tiles - 1) / strip_tiles;
@@ -185,6 +181,11 @@ bool plan_chain(const FilterTable &first, const FilterTable &second, bool h_firs
 		}
 		if (max_pxa <= kChainWindow)
 			break;
+		if (h_first && KV == 1 && KH == 1 && per_warp > 2) {
+			code = chain_detail::kNarrowVariant;
+			per_warp = chain_detail::chain_variant_of(code).tiles;
+			strip_tiles = (chain_detail::kWsWarps + 1) * per_warp;  // next: seven warps' tiles
+		}
 	}
 	if (strip_tiles < per_warp)
 		return false;
@@ -207,7 +208,7 @@ bool plan_chain(const FilterTable &first, const FilterTable &second, bool h_firs
 		for (int g = 0; g < groups; ++g)
 			ring = std::max(ring, hi_of(g + 1 + ahead) - gbase[g]);
 		const size_t bytes = static_cast<size_t>(ring) * pitch * 2 + static_cast<size_t>(ahead + 2) * KV * 1024 +
-		                     static_cast<size_t>(chain_detail::kMaxWarps) * per_warp * chain_detail::kTileStage +
+		                     static_cast<size_t>(chain_detail::kWsWarps) * per_warp * chain_detail::kTileStage +
 		                     static_cast<size_t>(groups) * 4;
 		if (ahead == 1 || bytes <= kChainSmem)
 			break;
@@ -232,6 +233,8 @@ bool plan_chain(const FilterTable &first, const FilterTable &second, bool h_firs
 	J.hw = KH;
 	J.vs = KV;
 	J.depth = ahead;
+	J.variant = code;
+	p.variant = 200 + code;
 	p.max_pxa = max_pxa;
 	p.depth = ahead;
 	p.mma = true;
@@ -297,8 +300,6 @@ bool plan_chain(const FilterTable &first, const FilterTable &second, bool h_firs
 	J.offset = offset;
 	J.magic = 12582912.0f + offset;
 	J.pixel_max = static_cast<float>((1UL << depth) - 1);
-	p.variant = chain_variant(h_first, KV, KH);
-	J.variant = p.variant - 200;
 	// H first: the share of a window's 8-line blocks that a group can take
 	// over from the previous one (its window moved by a multiple of 8 lines)
 	double kept = 0;

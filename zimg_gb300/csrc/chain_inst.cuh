@@ -8,35 +8,24 @@
 
 namespace zg {
 
-constexpr int kKVMax = 3;
-constexpr int kKHMax = 4;
-
 namespace {
 
-template <ChainForm F, bool HF, int KV>
-const void *form_ptr_kh(int kh)
+// The instances from code CODE on.
+template <ChainForm F, int CODE = 0>
+const void *form_ptr_from(int code)
 {
-	switch (kh) {
-	case 1: return reinterpret_cast<const void *>(&chain_detail::chain_tma_kernel<HF, KV, 1, F>);
-	case 2: return reinterpret_cast<const void *>(&chain_detail::chain_tma_kernel<HF, KV, 2, F>);
-	case 3: return reinterpret_cast<const void *>(&chain_detail::chain_tma_kernel<HF, KV, 3, F>);
-	default: return reinterpret_cast<const void *>(&chain_detail::chain_tma_kernel<HF, KV, 4, F>);
+	constexpr chain_detail::ChainVariant V = chain_detail::chain_variant_of(CODE);
+	if constexpr (CODE < chain_detail::kNarrowVariant) {
+		if (code != CODE)
+			return form_ptr_from<F, CODE + 1>(code);
 	}
-}
-
-template <ChainForm F, bool HF>
-const void *form_ptr_kv(int kv, int kh)
-{
-	return kv == 1 ? form_ptr_kh<F, HF, 1>(kh) : (kv == 2 ? form_ptr_kh<F, HF, 2>(kh) : form_ptr_kh<F, HF, 3>(kh));
+	return reinterpret_cast<const void *>(&chain_detail::chain_tma_kernel<V.h_first, V.kv, V.kh, V.tiles, F>);
 }
 
 template <ChainForm F>
 const void *form_ptr(int variant)
 {
-	const int v = variant - 200;
-	const int per = kKVMax * kKHMax;
-	const int kv = (v % per) / kKHMax + 1, kh = v % kKHMax + 1;
-	return v >= per ? form_ptr_kv<F, true>(kv, kh) : form_ptr_kv<F, false>(kv, kh);
+	return form_ptr_from<F>(variant - 200);
 }
 
 int form_set_fault(int drop_group, unsigned long long wait_ns)

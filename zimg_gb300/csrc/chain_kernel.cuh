@@ -33,11 +33,7 @@ using mma_detail::u16x2_to_centred_h2;
 
 // CTA shape: 7 computing warps and one producer warp at up to 128 registers
 // each, two CTAs per SM. A strip is up to 7 warps' tiles.
-__host__ __device__ constexpr int warps_per_cta(bool /*h_first*/)
-{
-	return 7;
-}
-constexpr int kMaxWarps = 7;
+constexpr int kWsWarps = 7;                // computing warps per CTA
 constexpr int kTileW = 16;                 // output columns of one tile (one m16 block)
 
 // Tiles per warp: several share the loop, the loads and the barriers, as far
@@ -47,10 +43,31 @@ __host__ __device__ constexpr int tiles_per_warp(int kv, int kh)
 {
 	return (kv == 1 && kh == 1) ? 4 : ((kv + kh <= 3 || kh == 1) ? 2 : 1);
 }
+
+// A kernel instance by its code (FusedJob::variant): the pass order, windows of
+// 16 kv lines and 16 kh columns, tiles per warp. The last has H first, windows
+// of 16 by 16 and two tiles a warp: where four make strips too wide for one copy
+// of their lines (above about 0.53 source samples an output), seven warps of
+// two tiles are busy instead of four to six of four. 10-bit planes, bilinear:
+// 40 of 640x360 -> 800x450 30.2 -> 24.1 us, 40 of 1280x720 -> 1760x990 74.2 ->
+// 60.1 us. (V first, windows of 16 columns from a multiple of 8 have at most
+// about half a source sample an output.)
+struct ChainVariant {
+	bool h_first;
+	int kv, kh, tiles;
+};
+constexpr int kChainKVMax = 3, kChainKHMax = 4;
+constexpr int kChainShapes = kChainKVMax * kChainKHMax;
+constexpr int kNarrowVariant = 2 * kChainShapes;
+__host__ __device__ constexpr ChainVariant chain_variant_of(int code)
+{
+	if (code == kNarrowVariant)
+		return { true, 1, 1, 2 };
+	const int kv = code % kChainShapes / kChainKHMax + 1, kh = code % kChainKHMax + 1;
+	return { code >= kChainShapes, kv, kh, tiles_per_warp(kv, kh) };
+}
 constexpr int kStageBytes = 48;            // staged row: 16 u16 + pad (stmatrix rows without bank conflicts)
-constexpr int kMaxTilesPerWarp = 4;
 constexpr int kTileStage = 16 * kStageBytes + 32;       // a warp's staged tiles lie 32 mod 128 bytes apart
-constexpr int kWarpStage = kMaxTilesPerWarp * kTileStage;
 
 __device__ __forceinline__ void stsm_x4(void *p, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3)
 {

@@ -50,7 +50,7 @@ chain_mixed_kernel(const FusedJob *__restrict__ jobs, int num_jobs, const __grid
 				switch (v) {
 #define ZG_CHAIN_CASE(HF, KV, KH)                                                                     \
 	case (HF ? 12 : 0) + (KV - 1) * 4 + (KH - 1):                                                      \
-		chain_item<HF, KV, KH, false, ChainForm::ALIGNED>(p, L, J, J.tmap, strip, g_begin, ngroups);  \
+		chain_item<HF, KV, KH, tiles_per_warp(KV, KH), false, ChainForm::ALIGNED>(p, L, J, J.tmap, strip, g_begin, ngroups);  \
 		break;
 					ZG_CHAIN_CASE(true, 1, 1) ZG_CHAIN_CASE(true, 1, 2) ZG_CHAIN_CASE(true, 1, 3) ZG_CHAIN_CASE(true, 1, 4)
 					ZG_CHAIN_CASE(true, 2, 1) ZG_CHAIN_CASE(true, 2, 2) ZG_CHAIN_CASE(true, 2, 3) ZG_CHAIN_CASE(true, 2, 4)
@@ -59,6 +59,9 @@ chain_mixed_kernel(const FusedJob *__restrict__ jobs, int num_jobs, const __grid
 					ZG_CHAIN_CASE(false, 2, 1) ZG_CHAIN_CASE(false, 2, 2) ZG_CHAIN_CASE(false, 2, 3) ZG_CHAIN_CASE(false, 2, 4)
 					ZG_CHAIN_CASE(false, 3, 1) ZG_CHAIN_CASE(false, 3, 2) ZG_CHAIN_CASE(false, 3, 3) ZG_CHAIN_CASE(false, 3, 4)
 #undef ZG_CHAIN_CASE
+				case kNarrowVariant:
+					chain_item<true, 1, 1, 2, false, ChainForm::ALIGNED>(p, L, J, J.tmap, strip, g_begin, ngroups);
+					break;
 				default:
 					break;
 				}
@@ -102,7 +105,7 @@ EncodeTiled encoder()
 
 int tma_threads(int variant)
 {
-	return chain_detail::tma_threads(variant - 200 >= kKVMax * kKHMax);
+	return chain_detail::tma_threads(chain_detail::chain_variant_of(variant - 200).h_first);
 }
 
 } // namespace
@@ -116,8 +119,7 @@ const ChainKernels *const kForms[] = { &kChainAligned, &kChainAnyDst, &kChainLin
 // A strip of the full width of its variant.
 bool full_strip(const FusedJob &j)
 {
-	const int tiles = chain_detail::tiles_per_warp(j.variant % (kKVMax * kKHMax) / kKHMax + 1, j.variant % kKHMax + 1);
-	return j.strip_w == chain_detail::kWsWarps * tiles * chain_detail::kTileW;
+	return j.strip_w == chain_detail::kWsWarps * chain_detail::chain_variant_of(j.variant).tiles * chain_detail::kTileW;
 }
 
 } // namespace
@@ -145,7 +147,7 @@ bool chain_tma_layout(const FusedPlan *const *plans, int n, SmemLayout *out)
 		groups = std::max(groups, p.job.groups);
 		depth = std::max(depth, p.depth);
 		kv = std::max(kv, p.job.vs);
-		tiles = std::max(tiles, chain_detail::tiles_per_warp(p.job.vs, p.job.hw));
+		tiles = std::max(tiles, chain_detail::chain_variant_of(p.job.variant).tiles);
 	}
 	auto a16 = [](size_t x) { return static_cast<int>((x + 15) / 16 * 16); };
 	auto pow2 = [](int x) {

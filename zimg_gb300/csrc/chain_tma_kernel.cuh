@@ -66,7 +66,6 @@ namespace zg {
 namespace chain_detail {
 
 constexpr int kBlockLines = 16;                     // source lines per tensor copy
-constexpr int kWsWarps = warps_per_cta(true);      // consumer warps per CTA
 
 // Nonzero after a pipeline wait ran out: 1 = a group's copies never landed,
 // 2 = a buffer was never released, 3 = ring too small for one group.
@@ -642,13 +641,12 @@ __device__ __forceinline__ void store_words(char *dst, ptrdiff_t dst_stride, int
 // (group bases visible, the previous item finished).
 // SPECIALISE: compile-time bodies for the common reuse cases (the
 // single-variant kernels; the mixed kernel keeps one body per variant).
-template <bool H_FIRST, int KV, int KH, bool SPECIALISE, ChainForm FORM>
+template <bool H_FIRST, int KV, int KH, int T, bool SPECIALISE, ChainForm FORM>
 __device__ __forceinline__ void chain_item(Pipe &p, const SmemLayout &L, const FusedJob &J, const void *tmap, int strip,
                                            int g_begin, int ngroups)
 {
 	constexpr bool TENSOR = FORM != ChainForm::LINES, ALIGNED = FORM == ChainForm::ALIGNED;
 	constexpr int kSlotBytes = KV * 2 * 32 * 16;
-	constexpr int T = tiles_per_warp(KV, KH);
 	const int strip_tiles = ALIGNED ? kWsWarps * T : J.strip_w / kTileW;  // at most kWsWarps * T
 	const int NS = p.NS, NB = p.NB, P = p.P, warp = p.warp, lane = p.lane;
 	const unsigned line_mask = p.line_mask;
@@ -935,7 +933,7 @@ __device__ __forceinline__ void load_bases(Pipe &p, const FusedJob &J, int g_beg
 // order (a whole strip, so that neighbouring CTAs run neighbouring strips in
 // step and read their shared columns once through L2, then an equal share of
 // the strips left over).
-template <bool H_FIRST, int KV, int KH, ChainForm FORM>
+template <bool H_FIRST, int KV, int KH, int T, ChainForm FORM>
 __global__ void __launch_bounds__(tma_threads(H_FIRST), 2)
 chain_tma_kernel(const FusedJob *__restrict__ jobs, int num_jobs, int total_items, const int *__restrict__ ranges,
                  const __grid_constant__ FewJobs few, const __grid_constant__ SmemLayout L,
@@ -968,8 +966,8 @@ chain_tma_kernel(const FusedJob *__restrict__ jobs, int num_jobs, int total_item
 			const int ngroups = min(J.groups - g_begin, t_end - t);
 			t += ngroups;
 			load_bases(p, J, g_begin, ngroups);
-			chain_item<H_FIRST, KV, KH, true, FORM>(p, L, J, jobs ? J.tmap : static_cast<const void *>(&few_maps.map[job]),
-			                                          strip, g_begin, ngroups);
+			chain_item<H_FIRST, KV, KH, T, true, FORM>(p, L, J, jobs ? J.tmap : static_cast<const void *>(&few_maps.map[job]),
+			                                           strip, g_begin, ngroups);
 			p.base += ngroups;
 			__syncthreads();  // the next item rewrites the group bases and the ring
 			if (abort_item)
