@@ -200,6 +200,36 @@ def test_narrow_strips_in_a_mixed_batch(cuda, oracle):
             np.testing.assert_array_equal(d.cpu().numpy().view(np.uint16), w, err_msg=str(jobs[k]))
 
 
+@pytest.mark.parametrize("pad,offset", [(0, 0), (8, 8), (1, 3), (2, 0)])
+def test_strips_of_two_and_four_tiles_in_one_launch(cuda, oracle, pad, offset):
+    """Upscales of small windows, some in strips of four tiles a warp and some
+    of two: one launch, whatever the planes' alignment."""
+    import torch
+    import zimg_gb300 as zg
+    from test_gpu_resize import empty
+    rng = np.random.default_rng(0x7E + pad)
+    jobs = [(640, 48, 800, 60), (320, 64, 640, 128), (512, 33, 901, 58), (240, 40, 481, 80)] * 3
+    convs, srcs, dsts, want = [], [], [], []
+    for sw, sh, dw, dh in jobs:
+        src = rng.integers(0, 1024, size=(sh, sw), dtype=np.uint16)
+        want.append(oracle.resize_plane(src, dw, dh, "bilinear", depth=10, mode="c", nthreads=16))
+        convs.append(zg.ResizeConversion(sw, sh, "word").set_depth(10).set_filter("bilinear").set_dst_width(dw)
+                     .set_dst_height(dh))
+        srcs.append(empty(sh, sw, np.uint16, pad=pad, offset=offset))
+        srcs[-1].copy_(torch.from_numpy(src.view(np.int16)))
+        dsts.append(empty(dh, dw, np.uint16, pad=pad, offset=offset))
+    b = zg.Batch(convs)
+    b.set_io(srcs, dsts)
+    assert b.launch_count == 1
+    for run in (b.process, b.process_graph):
+        for d in dsts:
+            d.zero_()
+        run()
+        torch.cuda.synchronize()
+        for k, (d, w) in enumerate(zip(dsts, want)):
+            np.testing.assert_array_equal(d.cpu().numpy().view(np.uint16), w, err_msg=str(jobs[k]))
+
+
 FAULT_CHILD = r"""
 import json, os, sys, time
 import numpy as np

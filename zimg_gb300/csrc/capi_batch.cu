@@ -382,8 +382,18 @@ void regroup(zg_batch *b)
 	for (unsigned i = 0; i < num_jobs; ++i)
 		if (b->jobs[i]->fused)
 			by_variant[b->jobs[i]->fplan.variant].push_back(i);
+	for (auto a = by_variant.begin(); a != by_variant.end(); ++a)
+		for (auto c = std::next(a); c != by_variant.end(); ++c)
+			if (const int joint = chain_joint_variant(a->first, c->first); joint >= 0) {
+				std::vector<unsigned> &both = by_variant[joint];
+				std::merge(a->second.begin(), a->second.end(), c->second.begin(), c->second.end(), std::back_inserter(both));
+				a->second.clear();
+				c->second.clear();
+			}
 	b->table_index.assign(num_jobs, -1);
 	for (auto &kv : by_variant) {
+		if (kv.second.empty())
+			continue;
 		zg_batch::Group g{ kv.first, SmemLayout{}, 0, static_cast<int>(b->table_host.size()), 0, 0 };
 		std::vector<const FusedPlan *> plans;
 		for (unsigned i : kv.second) {

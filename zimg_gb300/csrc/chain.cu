@@ -89,6 +89,14 @@ void a_fragments(const std::vector<float> (&dense)[2], int K, uint32_t *out)
 
 } // namespace
 
+int chain_joint_variant(int a, int b)
+{
+	const int wide = 200 + chain_detail::kChainShapes, narrow = 200 + chain_detail::kNarrowVariant;
+	if (a == b)
+		return a;
+	return (a == wide && b == narrow) || (a == narrow && b == wide) ? 200 + chain_detail::kEitherVariant : -1;
+}
+
 bool plan_chain(const FilterTable &first, const FilterTable &second, bool h_first, unsigned depth, unsigned src_w,
                 unsigned src_h, unsigned dst_w, unsigned dst_h, FusedPlan *out)
 {

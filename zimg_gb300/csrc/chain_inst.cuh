@@ -15,7 +15,7 @@ template <ChainForm F, int CODE = 0>
 const void *form_ptr_from(int code)
 {
 	constexpr chain_detail::ChainVariant V = chain_detail::chain_variant_of(CODE);
-	if constexpr (CODE < chain_detail::kNarrowVariant) {
+	if constexpr (CODE < chain_detail::kEitherVariant) {
 		if (code != CODE)
 			return form_ptr_from<F, CODE + 1>(code);
 	}

@@ -45,24 +45,29 @@ __host__ __device__ constexpr int tiles_per_warp(int kv, int kh)
 }
 
 // A kernel instance by its code (FusedJob::variant): the pass order, windows of
-// 16 kv lines and 16 kh columns, tiles per warp. The last has H first, windows
-// of 16 by 16 and two tiles a warp: where four make strips too wide for one copy
+// 16 kv lines and 16 kh columns, tiles per warp. kNarrowVariant has H first,
+// windows of 16 by 16 and two tiles a warp: where four make strips too wide for one copy
 // of their lines (above about 0.53 source samples an output), seven warps of
 // two tiles are busy instead of four to six of four. 10-bit planes, bilinear:
 // 40 of 640x360 -> 800x450 30.2 -> 24.1 us, 40 of 1280x720 -> 1760x990 74.2 ->
 // 60.1 us. (V first, windows of 16 columns from a multiple of 8 have at most
-// about half a source sample an output.)
+// about half a source sample an output.) kEitherVariant, no job's own, runs such
+// jobs and those of four tiles in one launch, where a batch has both: the body
+// of four alone is 4 % faster (16 planes 1920x1080 -> 3840x2160 78.5 us, 81.5
+// with both in it), two launches, or the mixed one, cost small batches more
+// (1280x720 -> 1920x1080 and 1920x1080 -> 3840x2160, a plane each: 14.5 us,
+// 20.5 in the mixed launch).
 struct ChainVariant {
 	bool h_first;
 	int kv, kh, tiles;
 };
 constexpr int kChainKVMax = 3, kChainKHMax = 4;
 constexpr int kChainShapes = kChainKVMax * kChainKHMax;
-constexpr int kNarrowVariant = 2 * kChainShapes;
+constexpr int kNarrowVariant = 2 * kChainShapes, kEitherVariant = kNarrowVariant + 1;
 __host__ __device__ constexpr ChainVariant chain_variant_of(int code)
 {
-	if (code == kNarrowVariant)
-		return { true, 1, 1, 2 };
+	if (code >= kNarrowVariant)
+		return { true, 1, 1, code == kNarrowVariant ? 2 : 0 };
 	const int kv = code % kChainShapes / kChainKHMax + 1, kh = code % kChainKHMax + 1;
 	return { code >= kChainShapes, kv, kh, tiles_per_warp(kv, kh) };
 }

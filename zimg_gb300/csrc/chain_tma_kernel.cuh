@@ -933,6 +933,7 @@ __device__ __forceinline__ void load_bases(Pipe &p, const FusedJob &J, int g_beg
 // order (a whole strip, so that neighbouring CTAs run neighbouring strips in
 // step and read their shared columns once through L2, then an equal share of
 // the strips left over).
+// T: tiles per warp; 0: each job's by its variant (kEitherVariant).
 template <bool H_FIRST, int KV, int KH, int T, ChainForm FORM>
 __global__ void __launch_bounds__(tma_threads(H_FIRST), 2)
 chain_tma_kernel(const FusedJob *__restrict__ jobs, int num_jobs, int total_items, const int *__restrict__ ranges,
@@ -979,8 +980,16 @@ chain_tma_kernel(const FusedJob *__restrict__ jobs, int num_jobs, int total_item
 			const int ngroups = min(J.groups - g_begin, t_end - t);
 			t += ngroups;
 			load_bases(p, J, g_begin, ngroups);
-			chain_item<H_FIRST, KV, KH, T, true, FORM>(p, L, J, jobs ? J.tmap : static_cast<const void *>(&few_maps.map[job]),
-			                                           strip, g_begin, ngroups);
+			const void *tmap = jobs ? J.tmap : static_cast<const void *>(&few_maps.map[job]);
+			if constexpr (T != 0) {
+				chain_item<H_FIRST, KV, KH, T, true, FORM>(p, L, J, tmap, strip, g_begin, ngroups);
+			} else {
+				constexpr int kNarrow = chain_variant_of(kNarrowVariant).tiles, kWide = tiles_per_warp(KV, KH);
+				if (J.variant == kNarrowVariant)
+					chain_item<H_FIRST, KV, KH, kNarrow, true, FORM>(p, L, J, tmap, strip, g_begin, ngroups);
+				else
+					chain_item<H_FIRST, KV, KH, kWide, true, FORM>(p, L, J, tmap, strip, g_begin, ngroups);
+			}
 			p.base += ngroups;
 			__syncthreads();  // the next item rewrites the group bases and the ring
 			if (abort_item)

@@ -233,6 +233,8 @@ struct ChainKernels {
 extern const ChainKernels kChainAligned, kChainAnyDst, kChainLines;
 ChainForm chain_form(const FusedJob *jobs, int n, bool mapped);
 bool chain_mixed_takes(const FusedJob &j);
+// The variant whose launch takes jobs of both variants, or -1.
+int chain_joint_variant(int a, int b);
 bool plan_chain(const FilterTable &first, const FilterTable &second, bool h_first, unsigned depth, unsigned src_w,
                 unsigned src_h, unsigned dst_w, unsigned dst_h, FusedPlan *out);
 bool chain_tma_enabled();  // tensor copies at all: false when the environment sets ZG_CHAIN_TMA=0
