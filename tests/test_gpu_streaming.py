@@ -67,9 +67,9 @@ def test_streaming_many_steps(cuda, oracle, sw, sh, dw, dh, kind, a, sample):
     (1920, 1080, 320, 180),   # 6x
     (1927, 1267, 275, 181),   # 7x, odd sizes
     (700, 3001, 129, 251),    # 12x, steps' windows far apart
-    (900, 1500, 450, 115),    # 13x down the columns: the tallest steps that fit
+    (900, 1500, 450, 125),    # 12x down the columns, 2x along the lines
     (300, 1400, 43, 800)])    # 7x along the lines only
 def test_point_filter_gaps(cuda, oracle, sw, sh, dw, dh, sample):
     """One tap an output: where rows lie far apart, so do the steps' windows,
-    and the lines between them are in no ring."""
+    and a step brings in more lines than its windows hold."""
     check_batch(oracle, sw, sh, dw, dh, "point", math.nan, sample, planes=12)

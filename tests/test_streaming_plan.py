@@ -37,7 +37,7 @@ const char *walk(const FusedPlan &p, const std::vector<int> &gbase, int start)
 	std::vector<int> in(J.in_rows, -1), mid(std::max(1, J.ring_rows), -1);
 	int next = ranges[2 * start], h_line = next;
 	auto load = [&](int k) -> const char * {  // the lines of step k; early: step k - 1 is being read
-		const int hi = ranges[2 * k + 1], a = stream_first_line(next, ranges[2 * k]);
+		const int hi = ranges[2 * k + 1], a = next;
 		if (hi - a > J.in_rows)
 			return "a step brings in more lines than the ring holds";
 		for (int y = a; y < hi; ++y) {
@@ -57,8 +57,8 @@ const char *walk(const FusedPlan &p, const std::vector<int> &gbase, int start)
 			if (const char *e = load(k + 1))
 				return e;
 		if (h_first) {
-			for (int y = stream_first_line(h_line, ranges[2 * k]); y < ranges[2 * k + 1]; ++y) {
-				if (y >= ranges[2 * k] && in[y % J.in_rows] != y)
+			for (int y = h_line; y < ranges[2 * k + 1]; ++y) {
+				if (in[y % J.in_rows] != y)
 					return "a source line is not in its slot";
 				mid[y % J.ring_rows] = y;
 			}

@@ -162,11 +162,13 @@ bool plan_fused(const FilterTable &first, const FilterTable &second, bool h_firs
 		ranges[2 * k] = h_first ? lo / 4 * 4 : lo;
 		ranges[2 * k + 1] = h_first ? (hi + 3) / 4 * 4 : hi;
 	}
-	// any step may start an item, when its new lines are its whole range;
+	// any step may start an item, when its new lines are its whole range, and
+	// brings in every line from the end of the step before: more than its range
+	// where that starts beyond (a point filter 5.5x and more down the columns);
 	// early: the next step's lines arrive beside this one's
 	int rows_late = 4, rows_early = 4;
 	for (int k = 0; k < steps; ++k) {
-		rows_late = std::max(rows_late, ranges[2 * k + 1] - ranges[2 * k]);
+		rows_late = std::max(rows_late, ranges[2 * k + 1] - (k ? std::min(ranges[2 * k], ranges[2 * k - 1]) : ranges[0]));
 		rows_early = std::max(rows_early, ranges[2 * std::min(k + 1, steps - 1) + 1] - ranges[2 * k]);
 	}
 

@@ -57,15 +57,6 @@ __host__ __device__ constexpr int stream_record_bytes(bool h_first, int vs)
 	return vs * (4 * group_rows(h_first) + 4);
 }
 
-// CUDA-core kernel: the first source line that a step brings in whose windows
-// start at line lo, `next` being the end of the lines brought in before it.
-// Lines between two steps' windows (a point filter far down) stay out: a ring
-// holds a step's windows, not the way to them.
-__host__ __device__ constexpr int stream_first_line(int next, int lo)
-{
-	return next > lo ? next : lo;
-}
-
 // One fused job as the kernel sees it (device-resident table entry).
 struct FusedJob {
 	// planes (filled from the caller's io)

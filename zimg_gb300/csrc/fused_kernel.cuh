@@ -629,17 +629,14 @@ fused_kernel(const FusedJob *__restrict__ jobs, int num_jobs, int total_items, c
 			// not yet in the ring and its slot
 			int next, slot;
 			auto load_step_lines = [&](int k) {
-				const int2 window = __ldg(it.ranges + it.step0 + k);
-				const int first = stream_first_line(next, window.x);
-				if (first > next)
-					slot = (slot + first - next) % it.in_rows;
-				if (window.y > first) {
-					load_lines<E>(it, first, window.y, in, it.in_rows, slot);
-					slot += window.y - first;
+				const int hi = __ldg(it.ranges + it.step0 + k).y;
+				if (hi > next) {
+					load_lines<E>(it, next, hi, in, it.in_rows, slot);
+					slot += hi - next;
 					while (slot >= it.in_rows)
 						slot -= it.in_rows;
+					next = hi;
 				}
-				next = max(first, window.y);
 			};
 			auto load_step_records = [&](int k) {
 				load_records(it.records + static_cast<size_t>(it.step0 + k) * kRecordBytes,
@@ -700,18 +697,12 @@ fused_kernel(const FusedJob *__restrict__ jobs, int num_jobs, int total_items, c
 				const int row0 = (it.step0 + k) * kStepRows;
 				const uint32_t rec = records_a + (k & 1) * kRecordBytes;
 				if constexpr (H_FIRST) {
-					const int2 window = __ldg(it.ranges + it.step0 + k);
-					const int first = stream_first_line(h_line, window.x);
-					if (first > h_line) {
-						h_in = (h_in + (first - h_line)) % it.in_rows;
-						h_mid = (h_mid + (first - h_line)) % it.ring_rows;
-						h_line = first;
-					}
-					if (window.y > h_line) {
-						hfirst_h<INT, HW>(it, in_a, taps, left, h_line, window.y, h_in, mid, h_mid);
-						h_in = (h_in + (window.y - h_line)) % it.in_rows;
-						h_mid = (h_mid + (window.y - h_line)) % it.ring_rows;
-						h_line = window.y;
+					const int hi = __ldg(it.ranges + it.step0 + k).y;
+					if (hi > h_line) {
+						hfirst_h<INT, HW>(it, in_a, taps, left, h_line, hi, h_in, mid, h_mid);
+						h_in = (h_in + (hi - h_line)) % it.in_rows;
+						h_mid = (h_mid + (hi - h_line)) % it.ring_rows;
+						h_line = hi;
 					}
 				} else {
 					vfirst_v<INT, VS>(it, in_a, rec, mid_a, q, half);
