@@ -67,3 +67,13 @@ def test_unresize_chunks(cuda, oracle, uw, uh, ow, oh, sw, sh, content):
     nan = np.isnan(want)
     np.testing.assert_array_equal(np.isnan(got), nan)
     np.testing.assert_array_equal(got[~nan].view(np.uint32), want[~nan].view(np.uint32))
+
+
+@pytest.mark.parametrize("ratio", [14.0, 15.0, 15.5, 16.0, 16.5, 17.0, 30.0])
+def test_unresize_long_rows(cuda, oracle, ratio):
+    """Rows around the number of taps from which the chunks give way."""
+    rng = np.random.default_rng(int(ratio * 2))
+    for ow, oh in ((37, 21), (130, 3), (5, 70)):
+        uw, uh = int(ow * ratio), int(oh * ratio)
+        src = make_src(rng, uh, uw)
+        np.testing.assert_array_equal(run(src, ow, oh).view(np.uint32), oracle.unresize_plane(src, ow, oh).view(np.uint32))

@@ -17,8 +17,9 @@
 // shared memory, so the dot products, both substitutions and the comparison
 // need no pass over memory in between.
 //
-// Lines too long for shared memory, and contexts whose factors do not shrink
-// (bilinear weights of a half: no reach), take two launches: the dot products,
+// Lines too long for shared memory, contexts whose factors do not shrink
+// (bilinear weights of a half: no reach) and long rows of taps (chunk_shape) take
+// two launches: the dot products,
 // one thread per output sample (k in zimg's order), into the pass's output
 // plane, then the substitutions, one thread per line or column, rewriting the
 // plane in place, with the next inputs loaded before the dependent steps so
@@ -429,12 +430,18 @@ unresize_lines(UnresizeTables t, const __grid_constant__ ChunkShape L, unsigned 
 // Shape of a block, or series = 0 where the chunked form does not apply.
 // Chunks about as long as the reach (their work doubles then), within one
 // block; columns 16 to a block (64-byte segments), lines 8, or as many as
-// fit the shared memory.
+// fit the shared memory. Rows of more than kMaxRow taps (about 16x) take the two
+// launches: a block has its few outputs' dot products for whole lines then, and
+// the two launches spread them out. Two launches against chunks, us: 1920x1080
+// -> 192x108 (20 taps) 39 and 23, 8000x4000 -> 400x200 (40) 110 and 116,
+// 1920x1080 -> 64x36 (60) 26 and 31, 20000x64 -> 200x64 (200) 35 and 121.
+constexpr unsigned kMaxRow = 32;
+
 ChunkShape chunk_shape(const UnresizeTables &t, bool horizontal, size_t *smem)
 {
 	constexpr size_t kMaxSmem = 227 * 1024;
 	ChunkShape L{};
-	if (!t.reach)
+	if (!t.reach || t.row_size > kMaxRow)
 		return L;
 	const int n = static_cast<int>(t.orig);
 	L.pitch = n | 1;
