@@ -154,3 +154,22 @@ def test_no_step_overruns_its_rings(walk):
     assert {"h-early", "h-late", "v-early", "v-late"} <= set(modes)
     bad = [(j, m, e) for j, (m, e) in zip(jobs, got) if e not in ("ok", "none", "refused")]
     assert not bad, (len(bad), bad[:5])
+
+
+@pytest.mark.parametrize("kind", [0, 1, 2, 4, 5])
+def test_planes_of_mostly_unused_lines_stay_separate(walk, kind):
+    """A point filter far down large planes leaves most lines without a tap;
+    no other filter does."""
+    a = {2: 0.0, 5: 3.0}.get(kind, math.nan)
+    b = 0.5 if kind == 2 else math.nan
+    jobs, want = [], []
+    for sw, sh, large in ((7680, 4320, True), (3840, 2160, False), (1920, 1080, False)):
+        for ratio in (2, 3, 7, 9, 12):
+            for u16 in (0, 1):
+                jobs.append((kind, a, b, sw, sh, sw // ratio, sh // ratio, 0.0, u16))
+                want.append(kind == 0 and large and ratio >= 7)
+    for job, (mode, e), separate in zip(jobs, walk(jobs), want):
+        if kind == 0 and (separate or job[3] < 7680 or job[5] > 3000):
+            assert (e == "refused") == separate, (job, mode, e)
+        elif kind:
+            assert e == "ok" or job[3] // job[5] >= 3, (job, mode, e)  # refused for their taps, if at all

@@ -21,6 +21,7 @@ constexpr int kVsBuckets[] = { 8, 12, 16, 24 };
 constexpr size_t kSmemBudget = 56 * 1024;   // preferred: four CTAs of 128 threads per SM
 constexpr size_t kSmemMax = 110 * 1024;     // hard limit: two CTAs per SM
 constexpr int kBlockColumns = 4 * 66;       // columns of the intermediate block (fused_kernel.cuh)
+constexpr size_t kUnusedBytes = 24 << 20;   // see plan_fused
 
 int bucket_index(const int *b, int n, int v)
 {
@@ -106,6 +107,23 @@ bool plan_fused(const FilterTable &first, const FilterTable &second, bool h_firs
 	if (vs_i < 0)
 		return false;
 	const int VS = kVsBuckets[vs_i];
+
+	// V first, the streaming kernel reads every line, a vertical pass alone the
+	// lines that have a tap (and its output comes and goes once more): far down
+	// with a point filter, and planes so large that the lines between cost more
+	// than the second launch, the separate passes are faster. One plane, 9x down,
+	// streaming and separate: u16 3840x2160 8.2 and 11.0 us (10 MB), 7680x4320
+	// 18.5 and 12.3 (39 MB), f32 3840x2160 10.3 and 11.2 (19 MB), 7680x4320 30.6
+	// and 12.4 (77 MB).
+	if (!h_first) {
+		std::vector<bool> tapped(src_h, false);
+		for (unsigned i = 0; i < dst_h; ++i)
+			for (unsigned k = 0; k < V.width; ++k)
+				tapped[V.left[i] + k] = true;
+		const size_t lines = static_cast<size_t>(std::count(tapped.begin(), tapped.end(), true)) + 2 * static_cast<size_t>(dst_h);
+		if (lines < src_h && (src_h - lines) * src_w * (u16 ? 2 : 4) > kUnusedBytes)
+			return false;
+	}
 
 	// strips: output columns (a multiple of 8, at most kStripW) whose inputs
 	// stay within the kernel's window; of those the width that needs the
