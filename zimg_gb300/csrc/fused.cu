@@ -345,7 +345,7 @@ SmemLayout fused_layout(const FusedPlan *const *plans, int n)
 	L.ring_off = off;
 	off += h_first ? ring * kStripW * 4 : 2 * kBlockColumns * 16;
 	L.vcoef_off = off;
-	off += 2 * 4 * stream_record_bytes(h_first, J.vs);
+	off += stream_record_buffers(h_first) * 4 * stream_record_bytes(h_first, J.vs);
 	L.total_bytes = off;
 	return L;
 }

@@ -56,6 +56,13 @@ __host__ __device__ constexpr int stream_record_bytes(bool h_first, int vs)
 {
 	return vs * (4 * group_rows(h_first) + 4);
 }
+// ... and the steps whose records are in shared memory at once: the next one's
+// are copied while this one's are read and, H first, where the vertical pass
+// ends a step, while warps may still read the last one's.
+__host__ __device__ constexpr int stream_record_buffers(bool h_first)
+{
+	return h_first ? 3 : 2;
+}
 
 // One fused job as the kernel sees it (device-resident table entry).
 struct FusedJob {

@@ -597,6 +597,7 @@ fused_kernel(const FusedJob *__restrict__ jobs, int num_jobs, int total_items, c
 	constexpr int E = INT ? 2 : 4;
 	constexpr int kStepRows = stream_step_rows(H_FIRST);
 	constexpr int kRecordBytes = 4 * stream_record_bytes(H_FIRST, VS);  // a step's four groups
+	constexpr int kRecordBuffers = stream_record_buffers(H_FIRST);
 	extern __shared__ float4 smem4[];
 	char *smem = reinterpret_cast<char *>(smem4);
 	char *in = smem + L.in_off;      // source lines
@@ -625,10 +626,10 @@ fused_kernel(const FusedJob *__restrict__ jobs, int num_jobs, int total_items, c
 			const Item it = make_item(J, t, c_end);
 			t += it.steps;
 
-			// lines of a step, and its records; `next`, `slot`: the first line
-			// not yet in the ring and its slot
+			// lines and records of a step, one cp.async group; `next`, `slot`:
+			// the first line not yet in the ring and its slot
 			int next, slot;
-			auto load_step_lines = [&](int k) {
+			auto load_step = [&](int k, int rec) {
 				const int hi = __ldg(it.ranges + it.step0 + k).y;
 				if (hi > next) {
 					load_lines<E>(it, next, hi, in, it.in_rows, slot);
@@ -637,20 +638,13 @@ fused_kernel(const FusedJob *__restrict__ jobs, int num_jobs, int total_items, c
 						slot -= it.in_rows;
 					next = hi;
 				}
-			};
-			auto load_step_records = [&](int k) {
-				load_records(it.records + static_cast<size_t>(it.step0 + k) * kRecordBytes,
-				             records + (k & 1) * kRecordBytes, kRecordBytes);
-			};
-			auto load_step = [&](int k) {  // both, one cp.async group
-				load_step_lines(k);
-				load_step_records(k);
+				load_records(it.records + static_cast<size_t>(it.step0 + k) * kRecordBytes, records + rec, kRecordBytes);
 				cp_async_commit();
 			};
 			next = __ldg(it.ranges + it.step0).x;
 			slot = next % it.in_rows;
 			int h_line = next, h_in = slot, h_mid = H_FIRST ? next % it.ring_rows : 0;
-			load_step(0);
+			load_step(0, 0);
 
 			// this thread's output column: taps, and where its inputs are
 			const int c = min(static_cast<int>(threadIdx.x), it.cols_valid - 1);
@@ -672,30 +666,25 @@ fused_kernel(const FusedJob *__restrict__ jobs, int num_jobs, int total_items, c
 					at[k] = mid_a + (((left + k) & 3) * kPlane + ((left + k) >> 2)) * 16;
 			}
 
+			int rec_at = 0;
 			for (int k = 0; k < it.steps; ++k) {
 				// early: the next step's lines go into slots that no line of
 				// this one's windows holds; late: only after its vertical
-				// pass (H first: horizontal pass). The next step's records
-				// replace those of the step before this one, whose readers
-				// have left them at the step's last barrier (V first) or at
-				// the next one (H first: the vertical pass comes last).
+				// pass (H first: horizontal pass). Records: H first, a warp may
+				// still read those of the step before this one.
 				const bool more = k + 1 < it.steps;
+				int rec_next = ((k + 1) & 1) * kRecordBytes;
+				if constexpr (H_FIRST)
+					rec_next = rec_at == (kRecordBuffers - 1) * kRecordBytes ? 0 : rec_at + kRecordBytes;
 				if (more && !it.late) {
-					load_step_lines(k + 1);
-					if constexpr (!H_FIRST)
-						load_step_records(k + 1);
-					cp_async_commit();
+					load_step(k + 1, rec_next);
 					cp_async_wait<1>();
 				} else {
 					cp_async_wait<0>();
 				}
 				__syncthreads();
-				if (H_FIRST && more && !it.late) {
-					load_step_records(k + 1);
-					cp_async_commit();
-				}
 				const int row0 = (it.step0 + k) * kStepRows;
-				const uint32_t rec = records_a + (k & 1) * kRecordBytes;
+				const uint32_t rec = records_a + (H_FIRST ? rec_at : (k & 1) * kRecordBytes);
 				if constexpr (H_FIRST) {
 					const int hi = __ldg(it.ranges + it.step0 + k).y;
 					if (hi > h_line) {
@@ -709,11 +698,12 @@ fused_kernel(const FusedJob *__restrict__ jobs, int num_jobs, int total_items, c
 				}
 				__syncthreads();
 				if (more && it.late)
-					load_step(k + 1);
+					load_step(k + 1, rec_next);
 				if constexpr (H_FIRST)
 					hfirst_v<INT, VS>(it, mid_a, rec, row0);
 				else
 					vfirst_h<INT, HW>(it, taps, at, row0);
+				rec_at = rec_next;
 			}
 			__syncthreads();  // the next item reuses every buffer
 		}
