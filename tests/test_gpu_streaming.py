@@ -73,3 +73,11 @@ def test_point_filter_gaps(cuda, oracle, sw, sh, dw, dh, sample):
     """One tap an output: where rows lie far apart, so do the steps' windows,
     and a step brings in more lines than its windows hold."""
     check_batch(oracle, sw, sh, dw, dh, "point", math.nan, sample, planes=12)
+
+
+@pytest.mark.parametrize("sample", ["word16", "float"])
+@pytest.mark.parametrize("planes", [1, 2, 5, 9, 20])
+@pytest.mark.parametrize("sw,sh,dw,dh", [(257, 420, 101, 169), (515, 1300, 257, 650), (65, 600, 263, 1401)])
+def test_small_batches_in_short_chunks(cuda, oracle, sw, sh, dw, dh, planes, sample):
+    """Chunks of one step to eight, some of them across strips and planes."""
+    check_batch(oracle, sw, sh, dw, dh, "bicubic", math.nan, sample, planes=planes)
