@@ -90,3 +90,35 @@ def test_batch_of_separate_passes(cuda, oracle, planes):
         for d, w in zip(dsts, want):
             got = d.cpu().numpy()
             np.testing.assert_array_equal(got.view(np.uint16) if w.dtype == np.uint16 else got, w)
+
+
+@pytest.mark.parametrize("sample", ["word", "float"])
+@pytest.mark.parametrize("odd", [(0,), (2,), (0, 2, 3), (0, 1, 2, 3)])
+def test_large_planes_of_mixed_alignment(cuda, oracle, odd, sample):
+    """Vertical passes of planes in 16-byte accesses beside those that cannot
+    go so, in the order of the batch."""
+    import torch
+    import zimg_gb300 as zg
+    from test_gpu_resize import empty, to_dev
+    w, sh, dh = 3848, 1500, 771
+    depth = 16 if sample == "word" else None
+    rng = np.random.default_rng(len(odd))
+    jobs, srcs, dsts, want = [], [], [], []
+    for k in range(4):
+        conv = zg.ResizeConversion(w, sh, sample).set_filter("bicubic").set_dst_height(dh)
+        jobs.append(conv.set_depth(depth) if depth else conv)
+        src = rng.integers(0, 1 << 16, size=(sh, w), dtype=np.uint16) if depth else \
+            rng.standard_normal((sh, w)).astype(np.float32)
+        off = k in odd
+        srcs.append(empty(sh, w, src.dtype, pad=off, offset=off))
+        srcs[-1].copy_(to_dev(src))
+        dsts.append(empty(dh, w, src.dtype, pad=8 * (k % 2), offset=0))
+        want.append(oracle.resize_plane(src, w, dh, "bicubic", depth=depth, mode="c", nthreads=16) if depth else
+                    oracle.resize_plane(src, w, dh, "bicubic", mode="fma", nthreads=16))
+    b = zg.Batch(jobs)
+    b.set_io(srcs, dsts)
+    b.process()
+    torch.cuda.synchronize()
+    for d, x in zip(dsts, want):
+        got = d.cpu().numpy()
+        np.testing.assert_array_equal(got.view(np.uint16) if depth else got, x)

@@ -96,7 +96,7 @@ struct PassLaunch {
 	ptrdiff_t src_stride;  // bytes
 	void *dst;
 	ptrdiff_t dst_stride;  // bytes
-	const PassPlane *planes = nullptr;  // num_planes of them (the first one too), where pass_takes_planes()
+	const PassPlane *planes = nullptr;  // num_planes of them (the first one too); wide and dense passes take one
 	int num_planes = 1;
 	WideTables wide;       // FP32 passes on the tensor cores when wide.frag is set
 };
