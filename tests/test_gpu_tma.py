@@ -163,6 +163,20 @@ def test_chained_kernel_any_alignment(cuda, oracle, sw, sh, dw, dh, kind, pad, o
 
 
 @pytest.mark.parametrize("sw,sh,dw,dh,kind", [
+    (640, 16, 272, 7, "bicubic"),    # a window of one block, the plane
+    (640, 17, 272, 8, "bilinear"),   # the second of two in part
+    (640, 79, 272, 33, "bicubic"),   # three blocks below the last group's row
+    (640, 80, 272, 34, "bilinear"),  # ... and the plane ends with a block
+    (640, 96, 320, 48, "bicubic"),   # whole groups
+    (160, 16, 320, 33, "bicubic"),   # H first
+    (160, 17, 320, 33, "lanczos")])
+@pytest.mark.parametrize("pad,offset", [(0, 0), (1, 0), (8, 8)])
+def test_windows_below_the_plane(cuda, oracle, sw, sh, dw, dh, kind, pad, offset):
+    """Windows of whole 16-line blocks that end below the plane."""
+    test_chained_kernel_any_alignment(cuda, oracle, sw, sh, dw, dh, kind, pad, offset, False)
+
+
+@pytest.mark.parametrize("sw,sh,dw,dh,kind", [
     (640, 48, 800, 60, "bilinear"),    # H first, strips of 224 columns: four, the last one partial
     (256, 33, 448, 58, "bicubic"),     # two strips, whole
     (257, 33, 449, 58, "bicubic"),     # one column past them
