@@ -416,7 +416,9 @@ ZG_API zg_error_code zg_batch_autotune(zg_batch *b, zg_stream stream, unsigned *
  * stride, set by zg_batch_set_io), the chained jobs of all kernel variants and
  * the identity planes run as one persistent launch whose CTAs take chunks of
  * work units from a counter (large chunks first, by estimated cost, small
- * ones last). */
+ * ones last), unless a downscale's strips are narrower than its kernel's full
+ * ones. A separate pass over planes of one conversion counts as one; where
+ * large aligned planes have unaligned ones beside them it issues two. */
 ZG_API zg_error_code zg_batch_get_launch_count(const zg_batch *b, unsigned *out);
 
 /* ---------------------------------------------------------------- graph --

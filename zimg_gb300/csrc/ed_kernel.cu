@@ -12,10 +12,11 @@
 // a sample). The last line of a band hands its errors to the first line of
 // the next.
 //
-// ed_cluster_kernel runs a plane on a cluster of up to 8 SMs, four warps
-// each, one to a scheduler, so that nothing but the chain sets a step's time;
-// the warps run free of one another and hand errors on through distributed
-// shared memory. ed_kernel (one block a plane, a block barrier every 16 steps)
+// ed_cluster_kernel runs a plane on a cluster of up to 8 SMs, two or four
+// computing warps each (cluster_warps), one to a scheduler; two more warps for
+// each of them move its data, with two on schedulers of their own, with four
+// beside them. The warps run free of one another and hand errors on through
+// distributed shared memory. ed_kernel (one block a plane, a block barrier every 16 steps)
 // stays for planes whose lines do not fit the cluster's hand-off buffers.
 #include <cuda_runtime.h>
 

@@ -1,5 +1,5 @@
-// Fused two-pass resize: both passes of a conversion in one kernel. Each CTA
-// owns a strip of 128 output columns and streams the source rows of a row
+// Fused two-pass resize: both passes of a conversion in one kernel. An item is
+// a strip of output columns (up to 128 in the CUDA-core kernel), whose CTA streams the source rows of a row
 // segment through a ring of lines in shared memory, so every source line is
 // read from HBM and filtered once and the intermediate never reaches HBM.
 #pragma once
@@ -170,8 +170,8 @@ void fused_set_io(FusedJob &j, const void *src, ptrdiff_t src_stride, void *dst,
 // Try to build a fused plan for a two-pass conversion. Returns false (and
 // leaves the conversion to the two-pass kernels) when the job is not fusable:
 // taps too wide for the buckets, window tables that are not monotonic, rings
-// larger than the shared-memory budget, or u16 sums that cannot be proved
-// exact in float.
+// larger than the shared-memory budget, u16 sums that may pass int32, or large
+// planes most of whose lines have no tap.
 bool plan_fused(const FilterTable &first, const FilterTable &second, bool h_first, bool u16, unsigned depth,
                 unsigned src_w, unsigned src_h, unsigned dst_w, unsigned dst_h, FusedPlan *out);
 

@@ -176,6 +176,9 @@ h_f32_kernel(PassTables t, unsigned lines, const __grid_constant__ PassPlanes P,
 //   f32 960x1080 -> 1920x1080, 6 taps    8.9 -> 4.5 us
 //   f32 3840x2160 -> 1920x2160, 8 taps   40 -> 17 us
 //   f32 1920x1080 -> 960x1080, 16 taps   39 -> 11 us
+//   u16 1920x1080 -> 640x1080, 17 taps   8.3 -> 5.3 us
+//   u16 1920x1080 -> 384x1080, 29 taps   10.5 -> 6.1 us
+//   f32 1920x1080 -> 479x1080, 26 taps   18.0 -> 10.8 us
 constexpr int kRegTaps = 32;
 constexpr unsigned kRegRows = 8;
 constexpr unsigned kRegBatch = 4;
@@ -254,6 +257,9 @@ cudaError_t launch_h_reg(const PassLaunch &l, const PassPlanes &P, cudaStream_t 
 //   u16 1919x1080 -> 1919x721 (2-byte loads)    8.5 -> 6.8 us
 //   f32 1920x1080 -> 1920x540, 16 taps          9.8 -> 5.4 us
 //   f32 3840x2160 -> 3840x1080, 8 taps         15.7 -> 13.0 us
+//   u16 1920x1080 -> 1920x360, 17 taps         10.0 -> 4.9 us
+//   u16 1920x1080 -> 1920x216, 29 taps         14.8 -> 5.3 us
+//   f32 1920x1080 -> 1920x269, 26 taps         12.9 -> 5.8 us
 // f32 planes that are not 16-byte aligned stay with v_f32_kernel, whose
 // 4-byte loads came to 18.3 us at 3839x2160 -> 3839x1080, 18.6 us here.
 constexpr unsigned kRegColRows = 4;
