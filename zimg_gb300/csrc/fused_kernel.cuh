@@ -638,7 +638,8 @@ fused_kernel(const FusedJob *__restrict__ jobs, int num_jobs, int total_items, c
 						slot -= it.in_rows;
 					next = hi;
 				}
-				load_records(it.records + static_cast<size_t>(it.step0 + k) * kRecordBytes, records + rec, kRecordBytes);
+				load_records(it.records + static_cast<size_t>(it.step0 + k) * kRecordBytes,
+				             records + (H_FIRST ? rec : (k & 1) * kRecordBytes), kRecordBytes);
 				cp_async_commit();
 			};
 			next = __ldg(it.ranges + it.step0).x;
@@ -673,7 +674,7 @@ fused_kernel(const FusedJob *__restrict__ jobs, int num_jobs, int total_items, c
 				// pass (H first: horizontal pass). Records: H first, a warp may
 				// still read those of the step before this one.
 				const bool more = k + 1 < it.steps;
-				int rec_next = ((k + 1) & 1) * kRecordBytes;
+				int rec_next = 0;
 				if constexpr (H_FIRST)
 					rec_next = rec_at == (kRecordBuffers - 1) * kRecordBytes ? 0 : rec_at + kRecordBytes;
 				if (more && !it.late) {
