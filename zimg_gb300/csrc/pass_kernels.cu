@@ -544,23 +544,24 @@ cudaError_t launch_pass(const PassLaunch &l, cudaStream_t stream)
 	constexpr size_t kSplitBytes = 32 << 20;
 	PassPlanes P{};
 	P.p[0] = { l.src, l.src_stride, l.dst, l.dst_stride };
-	if (l.planes)
-		std::copy(l.planes, l.planes + l.num_planes, P.p);
-	const auto unaligned = std::stable_partition(P.p, P.p + l.num_planes, [](const PassPlane &p) {
-		return aligned16(p.src, p.src_stride) && aligned16(p.dst, p.dst_stride);
-	});
-	const bool vec = unaligned == P.p + l.num_planes;
-	const size_t aligned_bytes = static_cast<size_t>(unaligned - P.p) * l.lines * (l.t.input_width + l.t.rows) *
+	int aligned = 0;
+	for (int k = 0, other = l.num_planes; k < l.num_planes; ++k) {
+		const PassPlane &p = l.planes ? l.planes[k] : P.p[0];
+		const bool a = aligned16(p.src, p.src_stride) && aligned16(p.dst, p.dst_stride);
+		P.p[a ? aligned++ : --other] = p;
+	}
+	const bool vec = aligned == l.num_planes;
+	const size_t aligned_bytes = static_cast<size_t>(aligned) * l.lines * (l.t.input_width + l.t.rows) *
 	                             (l.sample == Sample::U16 ? 2 : 4);
 	if (!l.horizontal && !vec && aligned_bytes > kSplitBytes) {
 		PassLaunch part = l;
 		part.planes = P.p;
-		part.num_planes = static_cast<int>(unaligned - P.p);
+		part.num_planes = aligned;
 		const cudaError_t e = launch_pass(part, stream);
 		if (e != cudaSuccess)
 			return e;
-		part.planes = unaligned;
-		part.num_planes = l.num_planes - part.num_planes;
+		part.planes = P.p + aligned;
+		part.num_planes = l.num_planes - aligned;
 		return launch_pass(part, stream);
 	}
 	if (l.horizontal && l.t.width <= kRegTaps)
