@@ -46,12 +46,13 @@
 //    is a warp-uniform branch between two unrolled bodies.
 //  - Rounding is one paired fp32 multiply-add per two samples and one
 //    s16x2 minimum with relu (pack_u16x2).
-//  - Source blocks wholly below the plane are copies like any other, filled
-//    with zeros: written by the producer's one lane instead, 7 KB each, they
-//    held up a plane's last group. One of 1920x1080 -> 800x450, bilinear,
-//    12.3 -> 8.2 us, 16 of 3840x2160 -> 1920x1080 98.4 -> 94.2 us; 16 of
-//    3840x2160 -> 1506x847, bilinear, 97.1 -> 100.5 us by the compiler's
-//    schedule.
+//  - Source blocks wholly below the plane are zeros: V first, copies like any
+//    other, whose fill they are. The producer's one lane writing them, 7 KB
+//    each, held up a plane's last group: one of 1920x1080 -> 800x450, bilinear,
+//    12.3 -> 8.2 us, 16 of 3840x2160 -> 1600x900 86.1 -> 81.4 us (16 of 3840x2160
+//    -> 1506x847 97.1 -> 100.5 us by the compiler's schedule). H first, it does
+//    write them: upscales seldom have such blocks, and with copies alone the
+//    schedule of their loop costs 64 planes 1920x1080 -> 3840x2160 271 -> 283 us.
 //  - Every mbarrier wait is bounded (g_chain_wait_ns, default 0.25 s). A wait
 //    that runs out records its cause in g_chain_pipeline_error, the CTA
 //    stops, and the producer first waits (again bounded) for the copies it
@@ -697,6 +698,7 @@ __device__ __forceinline__ void chain_item(Pipe &p, const SmemLayout &L, const F
 				return true;
 			};
 			int s = static_cast<int>(p.base % NS);
+			const int in_blks = (J.src_h + kBlockLines - 1) / kBlockLines;
 			asm volatile("prefetch.tensormap [%0];\n" ::"l"(tmap) : "memory");
 			for (int k = 0; k < ngroups; ++k, s = s + 1 == NS ? 0 : s + 1) {
 				const unsigned g = p.base + k;
@@ -725,12 +727,29 @@ __device__ __forceinline__ void chain_item(Pipe &p, const SmemLayout &L, const F
 				}
 				// windows are padded to 16 KV lines: blocks below the plane come
 				// as zeros too, which their zero taps want finite
-				mbar_arrive_expect_tx(&full[s], static_cast<unsigned>(kSlotBytes + (last_blk + 1 - next_blk) * kBlockLines * P));
+				if constexpr (H_FIRST) {
+					const int copy_end = min(last_blk + 1, in_blks);
+					const int ncopy = max(0, copy_end - next_blk);
+					for (int b = max(next_blk, in_blks); b <= last_blk; ++b) {
+						float4 *z = reinterpret_cast<float4 *>(ring + (b & (NB - 1)) * kBlockLines * P);
+						for (int i = 0; i < kBlockLines * P / 16; ++i)
+							z[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+						// later tensor copies into this block come after these stores
+						asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+					}
+					mbar_arrive_expect_tx(&full[s], static_cast<unsigned>(kSlotBytes + ncopy * kBlockLines * P));
+					for (int b = next_blk; b < copy_end; ++b)
+						tma_load_2d(ring + (b & (NB - 1)) * kBlockLines * P, tmap, xlo, b * kBlockLines, &full[s]);
+				} else {
+					mbar_arrive_expect_tx(&full[s],
+					                      static_cast<unsigned>(kSlotBytes + (last_blk + 1 - next_blk) * kBlockLines * P));
 #pragma unroll 1
-				for (; next_blk <= last_blk; ++next_blk)
-					tma_load_2d(ring + (next_blk & (NB - 1)) * kBlockLines * P, tmap, xlo, next_blk * kBlockLines, &full[s]);
+					for (int b = next_blk; b <= last_blk; ++b)
+						tma_load_2d(ring + (b & (NB - 1)) * kBlockLines * P, tmap, xlo, b * kBlockLines, &full[s]);
+				}
 				bulk_load(vslots + s * kSlotBytes, vtab + static_cast<size_t>(g_begin + k) * kSlotBytes,
 				          kSlotBytes, &full[s]);
+				next_blk = max(next_blk, last_blk + 1);
 				p.issued = g + 1;
 			}
 			if (p.error)
